@@ -1285,48 +1285,6 @@ inline int sm_count(int device) {
   return n;
 }
 
-// Projection: ceil(n / K) passes of up to K sweeps; each pass reads one copy of
-// (u, v) and writes the other. `cur_u`/`cur_v` track which copy holds the
-// live field (0: u/v, 1: ub/vb) and are updated for the caller.
-// `zero_first`: the first pass also performs zero_pressure (inside a step).
-template <class S>
-inline int enqueue_blocked_projection(os_handle* h, cudaStream_t st, int* cur_u, int* cur_v,
-                                      bool zero_first) {
-  const int K = h->block_k;
-  const bool pressure = h->cfg.enable_pressure != 0;
-  const TileGeom g = make_geom(h->W, h->H, 2 * K, true, pressure, sm_count(h->cfg.device));
-  S* U[2] = {static_cast<S*>(h->u), static_cast<S*>(h->ub)};
-  S* V[2] = {static_cast<S*>(h->v), static_cast<S*>(h->vb)};
-  const int tiles = g.tiles_x * g.tiles_y;
-  int launches = 0;
-  for (int done = 0, pass = 0; done < h->c.n; pass++) {
-    const int sweeps = std::min(K, h->c.n - done);
-    const S* uin = U[*cur_u];
-    const S* vin = V[*cur_v];
-    S* uout = U[1 - *cur_u];
-    S* vout = V[1 - *cur_v];
-    if (pressure) {
-      cudaFuncSetAttribute(k_project_blocked<true, S>,
-                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g.smem);
-      launch_pdl(h->pdl, k_project_blocked<true, S>, tiles, kBlockThreads, g.smem, st,
-                 uin, vin, uout, vout, h->p, (const uint8_t*)h->flags, h->c,
-                 (const StepParams*)h->d_params, sweeps, g.halo, g.TX, g.TY, g.tiles_x,
-                 (zero_first && pass == 0) ? 1 : 0);
-    } else {
-      cudaFuncSetAttribute(k_project_blocked<false, S>,
-                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g.smem);
-      launch_pdl(h->pdl, k_project_blocked<false, S>, tiles, kBlockThreads, g.smem, st,
-                 uin, vin, uout, vout, h->p, (const uint8_t*)h->flags, h->c,
-                 (const StepParams*)h->d_params, sweeps, g.halo, g.TX, g.TY, g.tiles_x, 0);
-    }
-    launches++;
-    *cur_u = 1 - *cur_u;
-    *cur_v = 1 - *cur_v;
-    done += sweeps;
-  }
-  return launches;
-}
-
 // Dynamic shared memory of k_diffuse_blocked_tma: two 128-byte aligned
 // buffers of RH x 256 floats and the alignment slack.
 inline size_t tma_diffusion_smem(int RH) {
@@ -1378,38 +1336,21 @@ inline bool prepare_tma_diffusion(os_handle* h) {
   return true;
 }
 
-template <class S>
-inline int enqueue_blocked_diffusion(os_handle* h, cudaStream_t st, int* cur_u) {
+// ceil(n / K) diffusion passes staged by tensor copies.
+inline int enqueue_tma_diffusion(os_handle* h, cudaStream_t st, int* cur_u) {
   const int K = diffusion_depth(h);
   const TileGeom g = make_geom(h->W, h->H, K, false, false, sm_count(h->cfg.device));
-  S* U[2] = {static_cast<S*>(h->u), static_cast<S*>(h->ub)};
+  float* U[2] = {static_cast<float*>(h->u), static_cast<float*>(h->ub)};
   const int tiles = g.tiles_x * g.tiles_y;
-  if constexpr (std::is_same<S, float>::value) {
-    if (h->tma_diffusion) {
-      const size_t smem = tma_diffusion_smem(g.RH);
-      cudaFuncSetAttribute(k_diffuse_blocked_tma, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)smem);
-      int launches = 0;
-      for (int done = 0; done < h->c.n;) {
-        const int sweeps = std::min(K, h->c.n - done);
-        launch_pdl(h->pdl, k_diffuse_blocked_tma, tiles, kBlockThreads, smem, st,
-                   h->diff_maps[*cur_u], U[1 - *cur_u], h->c, (const StepParams*)h->d_params,
-                   sweeps, g.halo, g.TX, g.TY, g.tiles_x, h->rerr, h->d_host_rerr);
-        launches++;
-        *cur_u = 1 - *cur_u;
-        done += sweeps;
-      }
-      return launches;
-    }
-  }
-  cudaFuncSetAttribute(k_diffuse_blocked<S>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)g.smem);
+  const size_t smem = tma_diffusion_smem(g.RH);
+  cudaFuncSetAttribute(k_diffuse_blocked_tma, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                       (int)smem);
   int launches = 0;
   for (int done = 0; done < h->c.n;) {
     const int sweeps = std::min(K, h->c.n - done);
-    launch_pdl(h->pdl, k_diffuse_blocked<S>, tiles, kBlockThreads, g.smem, st,
-               (const S*)U[*cur_u], U[1 - *cur_u], h->c, (const StepParams*)h->d_params, sweeps,
-               g.halo, g.TX, g.TY, g.tiles_x);
+    launch_pdl(h->pdl, k_diffuse_blocked_tma, tiles, kBlockThreads, smem, st,
+               h->diff_maps[*cur_u], U[1 - *cur_u], h->c, (const StepParams*)h->d_params,
+               sweeps, g.halo, g.TX, g.TY, g.tiles_x, h->rerr, h->d_host_rerr);
     launches++;
     *cur_u = 1 - *cur_u;
     done += sweeps;

@@ -18,6 +18,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <iterator>
 #include <map>
 #include <mutex>
 #include <new>
@@ -170,8 +171,10 @@ struct os_handle {
   bool pdl = true;
   int resident = 0;       // projection
   int resident_diff = 0;  // diffusion
-  unsigned* rflags = nullptr;
+  unsigned* rflags = nullptr;  // exchange numbers per tile: projection, diffusion
   unsigned* dflags = nullptr;
+  uint4* rpackets = nullptr;   // exchanged cells
+  uint4* dpackets = nullptr;
   int* rerr = nullptr;
   int* host_rerr = nullptr;
   int* d_host_rerr = nullptr;
@@ -227,8 +230,9 @@ void dev_free(os_handle* h, void* p) {
 
 // The temporally blocked projection/diffusion engine works on the handle.
 #include "os_blocked.cuh"
-// The projection phase with tiles resident in shared memory across passes.
-#include "os_resident.cuh"
+// Projection and diffusion with tiles in registers, pass by pass or across
+// passes.
+#include "os_tile.cuh"
 // FP64 divergence-residual and conservation sums.
 #include "os_diag.cuh"
 // Pixel colours, velocity arrows and path lines as device buffers.
@@ -284,17 +288,12 @@ constexpr bool kBlockedTypes = std::is_same<A, float>::value &&
 template <class S, class A>
 void enqueue_diffusion(os_handle* h, Vel<S>& w, Enq& q) {
   if constexpr (kBlockedTypes<S, A>) {
-    if (use_blocked<S, A>(h) && h->resident_diff) {
-      const int n = enqueue_resident_diffusion<S>(h, q.st, &w.cu);
-      if (n > 0) {
-        q.count += n;
-        return;
-      }
-      q.failed = true;
-      return;
-    }
     if (use_blocked<S, A>(h)) {
-      q.count += enqueue_blocked_diffusion<S>(h, q.st, &w.cu);
+      const int n = h->tma_diffusion && !h->resident_diff
+                        ? enqueue_tma_diffusion(h, q.st, &w.cu)
+                        : enqueue_tiled_diffusion(h, q.st, &w.cu);
+      q.count += std::max(n, 0);
+      q.failed = q.failed || n < 0;
       return;
     }
   }
@@ -306,26 +305,19 @@ void enqueue_diffusion(os_handle* h, Vel<S>& w, Enq& q) {
   }
 }
 
-// With `extrapolated` non-null, the resident form may apply the extrapolation
-// that follows in a step to its last pass's regions; *extrapolated says
-// whether it did.
+// With `extrapolated` non-null, the tiled form applies the extrapolation that
+// follows in a step in its last pass; *extrapolated says whether it did.
 template <class S, class A>
 void enqueue_projection(os_handle* h, Vel<S>& w, Enq& q, bool zero_pressure_first,
                         bool* extrapolated = nullptr) {
   if (extrapolated) *extrapolated = false;
   if constexpr (kBlockedTypes<S, A>) {
-    if (use_blocked<S, A>(h) && h->resident) {
-      const int n = enqueue_resident_projection<S>(h, q.st, &w.cu, &w.cv, zero_pressure_first,
-                                                   extrapolated);
-      if (n > 0) {
-        q.count += n;
-        return;
-      }
-      q.failed = true;
-      return;
-    }
     if (use_blocked<S, A>(h)) {
-      q.count += enqueue_blocked_projection<S>(h, q.st, &w.cu, &w.cv, zero_pressure_first);
+      const int n = enqueue_tiled_projection(h, q.st, &w.cu, &w.cv, zero_pressure_first,
+                                             extrapolated != nullptr);
+      q.count += std::max(n, 0);
+      q.failed = q.failed || n < 0;
+      if (extrapolated) *extrapolated = n > 0;
       return;
     }
   }
@@ -450,7 +442,7 @@ int enqueue_phase(os_handle* h, int phase, Enq& q) {
   }
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return set_err(OS_ERR_CUDA, "launch failed: %s", cudaGetErrorString(e));
-  if (q.failed) return set_err(OS_ERR_CUDA, "resident projection launch refused");
+  if (q.failed) return set_err(OS_ERR_CUDA, "a projection or diffusion launch was refused");
   return OS_OK;
 }
 
@@ -498,7 +490,7 @@ int enqueue_step(os_handle* h, Enq& q) {
   }
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return set_err(OS_ERR_CUDA, "launch failed: %s", cudaGetErrorString(e));
-  if (q.failed) return set_err(OS_ERR_CUDA, "resident projection launch refused");
+  if (q.failed) return set_err(OS_ERR_CUDA, "a projection or diffusion launch was refused");
   return OS_OK;
 }
 
@@ -616,33 +608,29 @@ int enable_resident(os_handle* h, int mask) {
   if (h->block_k <= 0 || h->storage == OS_STORAGE_F64 || h->arena) return OS_OK;
   const bool pressure = h->cfg.enable_pressure != 0;
   const int sms = sm_count(h->cfg.device);
-  TileGeom g, gd;
-  bool proj = (mask & 1) && resident_geom(h->W, h->H, h->block_k, pressure, sms, &g);
-  bool diff = (mask & 2) && resident_diffusion_geom(h->W, h->H, h->block_k, sms, &gd);
-  switch (h->storage) {
-    case OS_STORAGE_F32:
-      proj = proj && (pressure ? resident_launchable<true, float>(g, sms)
-                               : resident_launchable<false, float>(g, sms));
-      diff = diff && resident_diffusion_launchable<float>(gd, sms);
-      break;
-    case OS_STORAGE_F16:
-      proj = proj && (pressure ? resident_launchable<true, __half>(g, sms)
-                               : resident_launchable<false, __half>(g, sms));
-      diff = diff && resident_diffusion_launchable<__half>(gd, sms);
-      break;
-    case OS_STORAGE_BF16:
-      proj = proj && (pressure ? resident_launchable<true, __nv_bfloat16>(g, sms)
-                               : resident_launchable<false, __nv_bfloat16>(g, sms));
-      diff = diff && resident_diffusion_launchable<__nv_bfloat16>(gd, sms);
-      break;
-  }
+  RegTile g, gd;
+  const bool proj = (mask & 1) && resident_tile(h, true, &g) &&
+                    tiles_launchable(pressure ? project_kernel<true>(g.R)
+                                              : project_kernel<false>(g.R), g, sms);
+  const bool diff = (mask & 2) && resident_tile(h, false, &gd) &&
+                    tiles_launchable(diffuse_kernel(gd.R), gd, sms);
   cudaGetLastError();
   if (!proj && !diff) return OS_OK;
-  const size_t fb = (size_t)sms * sizeof(unsigned);
-  CUDA_OR_RETURN(cudaMalloc(&h->rflags, fb));
-  CUDA_OR_RETURN(cudaMemset(h->rflags, 0, fb));
-  CUDA_OR_RETURN(cudaMalloc(&h->dflags, fb));
-  CUDA_OR_RETURN(cudaMemset(h->dflags, 0, fb));
+  if (proj) {
+    const size_t pb = resident_packet_bytes(h->W, h->H, kPacketsPerQuad<2>);
+    CUDA_OR_RETURN(cudaMalloc(&h->rflags, resident_epoch_bytes(sms)));
+    CUDA_OR_RETURN(cudaMalloc(&h->rpackets, pb));
+    CUDA_OR_RETURN(cudaMemsetAsync(h->rflags, 0, resident_epoch_bytes(sms), h->stream));
+    CUDA_OR_RETURN(cudaMemsetAsync(h->rpackets, 0, pb, h->stream));
+  }
+  if (diff) {
+    const size_t pb = resident_packet_bytes(h->W, h->H, kPacketsPerQuad<1>);
+    CUDA_OR_RETURN(cudaMalloc(&h->dflags, resident_epoch_bytes(sms)));
+    CUDA_OR_RETURN(cudaMalloc(&h->dpackets, pb));
+    CUDA_OR_RETURN(cudaMemsetAsync(h->dflags, 0, resident_epoch_bytes(sms), h->stream));
+    CUDA_OR_RETURN(cudaMemsetAsync(h->dpackets, 0, pb, h->stream));
+  }
+  CUDA_OR_RETURN(cudaStreamSynchronize(h->stream));
   int rc = ensure_error_words(h);
   if (rc) return rc;
   h->resident = proj;
@@ -669,8 +657,14 @@ int check_resident(os_handle* h) {
   if (!h->host_rerr || *(volatile int*)h->host_rerr == 0) return OS_OK;
   *(volatile int*)h->host_rerr = 0;
   const int sms = sm_count(h->cfg.device);
-  if (h->rflags) cudaMemsetAsync(h->rflags, 0, (size_t)sms * sizeof(unsigned), h->stream);
-  if (h->dflags) cudaMemsetAsync(h->dflags, 0, (size_t)sms * sizeof(unsigned), h->stream);
+  if (h->rflags) {
+    cudaMemsetAsync(h->rflags, 0, resident_epoch_bytes(sms), h->stream);
+    cudaMemsetAsync(h->rpackets, 0, resident_packet_bytes(h->W, h->H, kPacketsPerQuad<2>), h->stream);
+  }
+  if (h->dflags) {
+    cudaMemsetAsync(h->dflags, 0, resident_epoch_bytes(sms), h->stream);
+    cudaMemsetAsync(h->dpackets, 0, resident_packet_bytes(h->W, h->H, kPacketsPerQuad<1>), h->stream);
+  }
   cudaMemsetAsync(h->rerr, 0, sizeof(int), h->stream);
   cudaStreamSynchronize(h->stream);
   return set_err(OS_ERR_TIMEOUT,
@@ -689,6 +683,8 @@ void free_handle(os_handle* h) {
   if (h->h_params) cudaFreeHost(h->h_params);
   if (h->rflags) cudaFree(h->rflags);
   if (h->dflags) cudaFree(h->dflags);
+  if (h->rpackets) cudaFree(h->rpackets);
+  if (h->dpackets) cudaFree(h->dpackets);
   if (h->rerr) cudaFree(h->rerr);
   if (h->host_rerr) cudaFreeHost(h->host_rerr);
   if (h->params_event) cudaEventDestroy(h->params_event);
@@ -1295,12 +1291,12 @@ int os_selftest_bounded_wait(int32_t device, int32_t* status) {
   if (!status) return set_err(OS_ERR_INVALID, "null argument");
   *status = OS_OK;
   CUDA_OR_RETURN(cudaSetDevice(device));
-  unsigned* flags = nullptr;
+  uint4* packets = nullptr;
   int* dev_err = nullptr;
   int* host_err = nullptr;
   int* d_host_err = nullptr;
-  cudaError_t e = cudaMalloc(&flags, 2 * sizeof(unsigned));
-  if (e == cudaSuccess) e = cudaMemset(flags, 0, 2 * sizeof(unsigned));
+  cudaError_t e = cudaMalloc(&packets, sizeof(uint4));
+  if (e == cudaSuccess) e = cudaMemset(packets, 0, sizeof(uint4));
   if (e == cudaSuccess) e = cudaMalloc(&dev_err, sizeof(int));
   if (e == cudaSuccess) e = cudaMemset(dev_err, 0, sizeof(int));
   if (e == cudaSuccess) e = cudaHostAlloc(&host_err, sizeof(int), cudaHostAllocMapped);
@@ -1309,12 +1305,12 @@ int os_selftest_bounded_wait(int32_t device, int32_t* status) {
     e = cudaHostGetDevicePointer((void**)&d_host_err, host_err, 0);
   }
   if (e == cudaSuccess) {
-    k_wait_selftest<<<1, 32>>>(ResidentSync{flags, dev_err, d_host_err});
+    k_wait_selftest<<<1, 32>>>(ResidentSync{nullptr, packets, dev_err, d_host_err});
     e = cudaGetLastError();
   }
   if (e == cudaSuccess) e = cudaDeviceSynchronize();
   if (e == cudaSuccess) *status = *(volatile int*)host_err ? OS_ERR_TIMEOUT : OS_OK;
-  if (flags) cudaFree(flags);
+  if (packets) cudaFree(packets);
   if (dev_err) cudaFree(dev_err);
   if (host_err) cudaFreeHost(host_err);
   if (e != cudaSuccess) return set_err(OS_ERR_CUDA, "self-test: %s", cudaGetErrorString(e));

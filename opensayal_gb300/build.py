@@ -11,6 +11,8 @@ from __future__ import annotations
 import os
 import shutil
 import subprocess
+import tempfile
+from concurrent.futures import ThreadPoolExecutor
 from pathlib import Path
 
 PKG = Path(__file__).resolve().parent
@@ -23,8 +25,15 @@ HEADER = ROOT / "include" / "opensayal_gb300.h"
 ARCH_FLAGS = ["-gencode", "arch=compute_103a,code=sm_103a"]
 NVCC_FLAGS = [
     "-std=c++17", "-O3", "--use_fast_math", "-lineinfo",
-    "-Xcompiler", "-fPIC", "-shared", "-diag-suppress", "177",
+    "-Xcompiler", "-fPIC", "-diag-suppress", "177",
 ]
+
+# Translation units, compiled side by side: (source, defines). The tile kernels
+# take one unit per strip height.
+TILE_ROWS = {"project": (10, 8, 6, 4, 2), "diffuse": (12, 8, 6, 4, 2)}
+UNITS = [("os_fluid.cu", ())]
+UNITS += [(f"os_tile_{phase}.cu", (f"OS_TILE_ROWS={rows}",))
+          for phase, heights in TILE_ROWS.items() for rows in heights]
 
 
 def _nvcc() -> str:
@@ -49,20 +58,32 @@ def _stale(target: Path, deps: list[Path]) -> bool:
     return any(d.stat().st_mtime > t for d in deps)
 
 
+def _run(cmd: list[str], verbose: bool) -> None:
+    res = subprocess.run(cmd, capture_output=True, text=True)
+    if res.returncode != 0:
+        raise RuntimeError(f"nvcc failed ({' '.join(cmd)}):\n{res.stdout}\n{res.stderr}")
+    if verbose:
+        print(res.stderr)
+
+
 def build_library(force: bool = False, verbose: bool = False) -> Path:
     """Compile the library if any source is newer than the built .so."""
     if not force and not _stale(LIB_PATH, _sources()):
         return LIB_PATH
     LIB_DIR.mkdir(parents=True, exist_ok=True)
     tmp = LIB_PATH.with_suffix(".so.tmp")
-    cmd = [_nvcc(), *NVCC_FLAGS, *ARCH_FLAGS, "-o", str(tmp), str(CSRC / "os_fluid.cu")]
-    if verbose:
-        cmd.insert(1, "-Xptxas=-v")
-    res = subprocess.run(cmd, capture_output=True, text=True)
-    if res.returncode != 0:
-        raise RuntimeError(f"nvcc failed ({' '.join(cmd)}):\n{res.stdout}\n{res.stderr}")
-    if verbose:
-        print(res.stderr)
+    with tempfile.TemporaryDirectory(dir=LIB_DIR) as work:
+        def compile_unit(index: int) -> str:
+            source, defines = UNITS[index]
+            obj = str(Path(work) / f"{index}.o")
+            cmd = [_nvcc(), *NVCC_FLAGS, *ARCH_FLAGS, *(f"-D{d}" for d in defines),
+                   *(["-Xptxas=-v"] if verbose else []), "-c", "-o", obj, str(CSRC / source)]
+            _run(cmd, verbose)
+            return obj
+
+        with ThreadPoolExecutor(max_workers=os.cpu_count() or 1) as pool:
+            objects = list(pool.map(compile_unit, range(len(UNITS))))
+        _run([_nvcc(), *ARCH_FLAGS, "-shared", "-o", str(tmp), *objects], verbose)
     os.replace(tmp, LIB_PATH)
     return LIB_PATH
 

@@ -84,4 +84,31 @@ __host__ __device__ __forceinline__ int cell_index32(int W, int H, int i, int j)
   return (H - 1 - j) * W + i;
 }
 
+// Programmatic dependent launch: a kernel of the step graph first waits until
+// the kernel before it has completed and its writes are visible, then lets
+// the next kernel launch, so launch latency and tails overlap. For a kernel
+// launched without the attribute both are no-ops.
+__device__ __forceinline__ void pdl_entry() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+// A product that is never fused into a later add (the reference stores it to
+// memory and reloads it, which also blocks contraction).
+__device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
+
+// a * b + c with one rounding: the reference's `x += a * b` as nvcc fuses it
+// per thread. Written out so that the fusion does not depend on the calling
+// context (a loop-invariant a * b hoisted out of a loop would otherwise be
+// rounded on its own).
+__device__ __forceinline__ float fma_rn(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ double fma_rn(double a, double b, double c) { return __fma_rn(a, b, c); }
+
+// a = viscosity * dt / h^2 (src/fluid.cu:177).
+template <class A>
+__device__ __forceinline__ A diffusion_coeff(const Consts& c, A d_t) {
+  return (A)c.viscosity * d_t / (A)(c.h * c.h);
+}
+
 }  // namespace osg

@@ -29,6 +29,7 @@
 #include "../../include/opensayal_gb300.h"
 #include "../../include/opensayal_gb300/config_parser.hpp"
 #include "os_kernels.cuh"
+#include "os_tile.cuh"
 
 using namespace osg;
 
@@ -134,6 +135,14 @@ class Arena {
 
 }  // namespace
 
+// The tile a phase runs on, for blocking depth K and form (os_tile_host.cuh).
+struct TileChoice {
+  int K = 0;
+  bool resident = false;
+  int depth = 0;
+  osg::RegTile tile;
+};
+
 struct os_handle {
   os_config cfg;
   Consts c;
@@ -160,18 +169,23 @@ struct os_handle {
   bool params_valid = false;
   int* d_pkeys = nullptr;   // pressure extrema as ordered integer keys
   int* h_pkeys = nullptr;   // pinned copy
+  char* pinned = nullptr;   // one pinned block: h_params, h_pkeys, host_rerr
   float* conv = nullptr;    // FP32 staging for non-FP32 storage transfers
   double* diag = nullptr;   // diagnostics partials and result (first use)
-  // Resident projection (one cooperative launch per phase): tile flags, the
-  // device error word, and a mapped host word the kernel sets on a failed wait.
+  // The device error word and the mapped host word that a kernel sets when a
+  // bounded wait gives up (the host word: handles outside a batch), and the
+  // resident forms' exchange state.
   // Diffusion passes staged by the tensor memory accelerator: maps of u, ub.
   CUtensorMap diff_maps[2];
   bool tma_diffusion = false;
   // Step kernels launched with programmatic dependent launch.
   bool pdl = true;
+  TileChoice tile_choice[2];  // projection, diffusion
   int resident = 0;       // projection
   int resident_diff = 0;  // diffusion
-  unsigned* rflags = nullptr;  // exchange numbers per tile: projection, diffusion
+  char* resident_block = nullptr;  // the four arrays that follow
+  size_t resident_bytes = 0;
+  unsigned* rflags = nullptr;  // exchange numbers per CTA: projection, diffusion
   unsigned* dflags = nullptr;
   uint4* rpackets = nullptr;   // exchanged cells
   uint4* dpackets = nullptr;
@@ -191,6 +205,9 @@ struct os_handle {
 
 namespace {
 
+// The pressure extrema's keys and the error word of bounded waits.
+constexpr size_t kKeyBytes = 3 * sizeof(int);
+
 // Diagnostics scratch: 256 block partials and the result, 7 doubles each.
 constexpr size_t kDiagBytes = (256 + 1) * 7 * sizeof(double);
 
@@ -201,7 +218,7 @@ size_t handle_footprint(const os_config& c) {
   const size_t N = (size_t)c.width * c.height;
   const size_t e = storage_bytes(c.storage);
   auto r = [](size_t b) { return (b + 255) / 256 * 256; };
-  size_t bytes = 6 * r(N * e) + 3 * r(N * 4) + r(N) + r(sizeof(StepParams)) + r(2 * sizeof(int));
+  size_t bytes = 6 * r(N * e) + 3 * r(N * 4) + r(N) + r(sizeof(StepParams)) + r(kKeyBytes);
   bytes += r((size_t)(c.width + 2) * (c.height + 2) * sizeof(uint16_t));
   if (c.storage != OS_STORAGE_F32) bytes += r(N * 4);
   bytes += r(kDiagBytes);
@@ -232,7 +249,7 @@ void dev_free(os_handle* h, void* p) {
 #include "os_blocked.cuh"
 // Projection and diffusion with tiles in registers, pass by pass or across
 // passes.
-#include "os_tile.cuh"
+#include "os_tile_host.cuh"
 // FP64 divergence-residual and conservation sums.
 #include "os_diag.cuh"
 // Pixel colours, velocity arrows and path lines as device buffers.
@@ -600,53 +617,31 @@ struct TuneChoice {
 };
 TuneChoice autotune_projection(const os_config& base);
 
-int ensure_error_words(os_handle* h);
-
 // Sets up the resident projection (mask bit 0) and diffusion (bit 1) that
 // the grid fits (flags, error words).
 int enable_resident(os_handle* h, int mask) {
   if (h->block_k <= 0 || h->storage == OS_STORAGE_F64 || h->arena) return OS_OK;
-  const bool pressure = h->cfg.enable_pressure != 0;
   const int sms = sm_count(h->cfg.device);
   RegTile g, gd;
-  const bool proj = (mask & 1) && resident_tile(h, true, &g) &&
-                    tiles_launchable(pressure ? project_kernel<true>(g.R)
-                                              : project_kernel<false>(g.R), g, sms);
-  const bool diff = (mask & 2) && resident_tile(h, false, &gd) &&
-                    tiles_launchable(diffuse_kernel(gd.R), gd, sms);
+  const int dp = mask & 1 ? phase_tile(h, true, h->block_k, true, &g) : 0;
+  const int dd = mask & 2 ? phase_tile(h, false, h->block_k, true, &gd) : 0;
+  const bool proj = dp > 0, diff = dd > 0;
   cudaGetLastError();
   if (!proj && !diff) return OS_OK;
-  if (proj) {
-    const size_t pb = resident_packet_bytes(h->W, h->H, kPacketsPerQuad<2>);
-    CUDA_OR_RETURN(cudaMalloc(&h->rflags, resident_epoch_bytes(sms)));
-    CUDA_OR_RETURN(cudaMalloc(&h->rpackets, pb));
-    CUDA_OR_RETURN(cudaMemsetAsync(h->rflags, 0, resident_epoch_bytes(sms), h->stream));
-    CUDA_OR_RETURN(cudaMemsetAsync(h->rpackets, 0, pb, h->stream));
-  }
-  if (diff) {
-    const size_t pb = resident_packet_bytes(h->W, h->H, kPacketsPerQuad<1>);
-    CUDA_OR_RETURN(cudaMalloc(&h->dflags, resident_epoch_bytes(sms)));
-    CUDA_OR_RETURN(cudaMalloc(&h->dpackets, pb));
-    CUDA_OR_RETURN(cudaMemsetAsync(h->dflags, 0, resident_epoch_bytes(sms), h->stream));
-    CUDA_OR_RETURN(cudaMemsetAsync(h->dpackets, 0, pb, h->stream));
-  }
-  CUDA_OR_RETURN(cudaStreamSynchronize(h->stream));
-  int rc = ensure_error_words(h);
-  if (rc) return rc;
+  // One block: the exchange numbers, and the packets of the phases whose tiles
+  // exchange any.
+  const size_t head = 2 * resident_epoch_bytes(sms);
+  const size_t pb = proj && h->c.n > dp ? resident_packet_bytes(h->W, h->H, kPacketsPerQuad<2>) : 0;
+  const size_t db = diff && h->c.n > dd ? resident_packet_bytes(h->W, h->H, kPacketsPerQuad<1>) : 0;
+  h->resident_bytes = head + pb + db;
+  CUDA_OR_RETURN(cudaMalloc(&h->resident_block, h->resident_bytes));
+  CUDA_OR_RETURN(cudaMemsetAsync(h->resident_block, 0, h->resident_bytes, h->stream));
+  h->rflags = reinterpret_cast<unsigned*>(h->resident_block);
+  h->dflags = h->rflags + resident_epoch_bytes(sms) / sizeof(unsigned);
+  h->rpackets = reinterpret_cast<uint4*>(h->resident_block + head);
+  h->dpackets = reinterpret_cast<uint4*>(h->resident_block + head + pb);
   h->resident = proj;
   h->resident_diff = diff;
-  return OS_OK;
-}
-
-// Device error word and the mapped host word a kernel sets on a failed
-// bounded wait (allocated once).
-int ensure_error_words(os_handle* h) {
-  if (h->rerr) return OS_OK;
-  CUDA_OR_RETURN(cudaMalloc(&h->rerr, sizeof(int)));
-  CUDA_OR_RETURN(cudaMemset(h->rerr, 0, sizeof(int)));
-  CUDA_OR_RETURN(cudaHostAlloc(&h->host_rerr, sizeof(int), cudaHostAllocMapped));
-  *h->host_rerr = 0;
-  CUDA_OR_RETURN(cudaHostGetDevicePointer((void**)&h->d_host_rerr, h->host_rerr, 0));
   return OS_OK;
 }
 
@@ -656,15 +651,8 @@ int ensure_error_words(os_handle* h) {
 int check_resident(os_handle* h) {
   if (!h->host_rerr || *(volatile int*)h->host_rerr == 0) return OS_OK;
   *(volatile int*)h->host_rerr = 0;
-  const int sms = sm_count(h->cfg.device);
-  if (h->rflags) {
-    cudaMemsetAsync(h->rflags, 0, resident_epoch_bytes(sms), h->stream);
-    cudaMemsetAsync(h->rpackets, 0, resident_packet_bytes(h->W, h->H, kPacketsPerQuad<2>), h->stream);
-  }
-  if (h->dflags) {
-    cudaMemsetAsync(h->dflags, 0, resident_epoch_bytes(sms), h->stream);
-    cudaMemsetAsync(h->dpackets, 0, resident_packet_bytes(h->W, h->H, kPacketsPerQuad<1>), h->stream);
-  }
+  if (h->resident_block)
+    cudaMemsetAsync(h->resident_block, 0, h->resident_bytes, h->stream);
   cudaMemsetAsync(h->rerr, 0, sizeof(int), h->stream);
   cudaStreamSynchronize(h->stream);
   return set_err(OS_ERR_TIMEOUT,
@@ -679,14 +667,8 @@ void free_handle(os_handle* h) {
                   h->total_s, h->flags, h->nbr, h->d_params, h->d_pkeys, h->conv, h->diag};
   for (void* q : ptrs) dev_free(h, q);
   if (h->arena_block) h->arena->release(h->arena_block);
-  if (h->h_pkeys) cudaFreeHost(h->h_pkeys);
-  if (h->h_params) cudaFreeHost(h->h_params);
-  if (h->rflags) cudaFree(h->rflags);
-  if (h->dflags) cudaFree(h->dflags);
-  if (h->rpackets) cudaFree(h->rpackets);
-  if (h->dpackets) cudaFree(h->dpackets);
-  if (h->rerr) cudaFree(h->rerr);
-  if (h->host_rerr) cudaFreeHost(h->host_rerr);
+  if (h->pinned) cudaFreeHost(h->pinned);
+  if (h->resident_block) cudaFree(h->resident_block);
   if (h->params_event) cudaEventDestroy(h->params_event);
   if (h->stream) cudaStreamDestroy(h->stream);
   delete h;
@@ -887,15 +869,22 @@ static int create_handle(const os_config* cfg, Arena* arena, os_handle** out) {
       (e = dev_alloc(h, (void**)&h->nbr, (size_t)(h->W + 2) * (h->H + 2) * sizeof(uint16_t))) !=
           cudaSuccess ||
       (e = dev_alloc(h, (void**)&h->d_params, sizeof(StepParams))) != cudaSuccess ||
-      (e = dev_alloc(h, (void**)&h->d_pkeys, 2 * sizeof(int))) != cudaSuccess)
+      (e = dev_alloc(h, (void**)&h->d_pkeys, kKeyBytes)) != cudaSuccess)
     return fail(set_err(OS_ERR_NOMEM, "cudaMalloc: %s", cudaGetErrorString(e)));
   if (!arena) {
-    if ((e = cudaMallocHost(&h->h_pkeys, 2 * sizeof(int))) != cudaSuccess ||
-        (e = cudaMallocHost(&h->h_params, sizeof(StepParams))) != cudaSuccess)
-      return fail(set_err(OS_ERR_NOMEM, "cudaMallocHost: %s", cudaGetErrorString(e)));
+    if ((e = cudaHostAlloc((void**)&h->pinned, 256, cudaHostAllocMapped)) != cudaSuccess)
+      return fail(set_err(OS_ERR_NOMEM, "cudaHostAlloc: %s", cudaGetErrorString(e)));
+    h->h_params = reinterpret_cast<StepParams*>(h->pinned);
+    h->h_pkeys = reinterpret_cast<int*>(h->pinned + 64);
+    h->host_rerr = reinterpret_cast<int*>(h->pinned + 128);
+    *h->host_rerr = 0;
+    if ((e = cudaHostGetDevicePointer((void**)&h->d_host_rerr, h->host_rerr, 0)) != cudaSuccess)
+      return fail(set_err(OS_ERR_CUDA, "mapped word: %s", cudaGetErrorString(e)));
     if ((e = cudaEventCreateWithFlags(&h->params_event, cudaEventDisableTiming)) != cudaSuccess)
       return fail(set_err(OS_ERR_CUDA, "event: %s", cudaGetErrorString(e)));
   }
+  h->rerr = h->d_pkeys + 2;  // beside the pressure keys
+  cudaMemsetAsync(h->rerr, 0, sizeof(int), h->stream);
   cudaMemsetAsync(h->p, 0, h->N * 4, h->stream);
   MaskParams m;
   m.enable_drain = cfg->enable_drain != 0;
@@ -911,13 +900,13 @@ static int create_handle(const os_config* cfg, Arena* arena, os_handle** out) {
   k_init_neighbourhoods<<<dim3((h->W + 2 + 127) / 128, h->H + 2), 128, 0, h->stream>>>(
       h->is_solid, h->nbr, c);
   h->launches += 3;
-  if ((e = cudaGetLastError()) != cudaSuccess ||
-      (e = cudaStreamSynchronize(h->stream)) != cudaSuccess)
-    return fail(set_err(OS_ERR_CUDA, "init: %s", cudaGetErrorString(e)));
   if (resident) {
     const int rc = enable_resident(h, resident);
     if (rc) return fail(rc);
   }
+  if ((e = cudaGetLastError()) != cudaSuccess ||
+      (e = cudaStreamSynchronize(h->stream)) != cudaSuccess)
+    return fail(set_err(OS_ERR_CUDA, "init: %s", cudaGetErrorString(e)));
   const char* pdl_env = std::getenv("OPENSAYAL_GB300_PDL");
   h->pdl = !(pdl_env && pdl_env[0] == '0');
   // Tensor-copy staging of the diffusion passes is opt-in: inside a step it
@@ -925,8 +914,6 @@ static int create_handle(const os_config* cfg, Arena* arena, os_handle** out) {
   // overlap the previous kernel, the vector loads more so).
   const char* tma_env = std::getenv("OPENSAYAL_GB300_TMA");
   if (!arena && tma_env && tma_env[0] == '1' && prepare_tma_diffusion(h)) {
-    const int rc = ensure_error_words(h);
-    if (rc) return fail(rc);
     h->tma_diffusion = true;
   }
   *out = h;
@@ -1533,10 +1520,11 @@ float time_steps(os_handle* t, float dt, int warm, int reps) {
 }
 
 // Candidates: depths {2, 4, 6, 8, 12} pass by pass and, unless
-// projection_resident is -1, the resident forms the depth allows (projection
-// for even depths, diffusion for multiples of 4, alone or together) where
-// the grid fits them; a positive projection_resident fixes the forms and
-// leaves only the depth to choose.
+// projection_resident is -1, the resident forms (projection and diffusion,
+// alone or together) where the grid fits them, at one depth: a resident form
+// chooses its own sweeps between exchanges, and the depth only says how often
+// 16-bit fields are rounded. A positive projection_resident fixes the forms
+// and leaves only the depth to choose.
 TuneChoice autotune_projection(const os_config& base) {
   constexpr TuneChoice kDefault{4, 0, 0};
   const char* env = std::getenv("OPENSAYAL_GB300_AUTOTUNE");
@@ -1552,16 +1540,17 @@ TuneChoice autotune_projection(const os_config& base) {
   }
   std::vector<TuneChoice> cands;
   for (int K : {2, 4, 6, 8, 12}) {
-    if (base.projection_resident > 0) {
+    if (base.projection_resident > 0)
       cands.push_back({K, base.projection_resident, 0});
-      continue;
-    }
-    cands.push_back({K, 0, 0});
-    if (base.projection_resident == -1) continue;
-    if (K % 2 == 0 && K <= 8) cands.push_back({K, 1, 0});
+    else
+      cands.push_back({K, 0, 0});
+  }
+  if (base.projection_resident == 0) {
+    const int K = base.projection_n >= 8 ? 8 : base.projection_n >= 4 ? 4 : 2;
+    cands.push_back({K, 1, 0});
     if (K % 4 == 0 && base.viscosity != 0.0f) {
       cands.push_back({K, 2, 0});
-      if (K <= 8) cands.push_back({K, 3, 0});
+      cands.push_back({K, 3, 0});
     }
   }
   const float dt = base.d_t > 0.0f ? base.d_t : 0.05f;

@@ -1,11 +1,12 @@
 // os_tile.cuh — tiles held in registers: the red/black projection and the
-// Jacobi diffusion with every face of a tile in the registers of its CTA from
+// Jacobi diffusion with every face of a tile in the registers of its CTAs from
 // the first sweep of a pass to the last.
 //
-// A tile's region is 256 columns wide and RH = R * warps rows high. Warp w
-// holds the strip of rows [w R, (w + 1) R), lane l its columns 8 l .. 8 l + 7:
-// a patch of 8 x R cells per thread. The region of tile (tx, ty) starts at
-// cell (tx * TX, ty * TY); it carries `halo` cells on each side that has a
+// A tile's region is 256 columns wide and RH = R * warps * cluster rows high:
+// `cluster` CTAs (a thread-block cluster) of `warps` warps each, warp by warp
+// from the bottom up. A warp holds a strip of R rows, lane l its columns 8 l ..
+// 8 l + 7: a patch of 8 x R cells per thread. The region of tile (tx, ty) starts
+// at cell (tx * TX, ty * TY); it carries `halo` cells on each side that has a
 // neighbouring tile and none at the edges of the grid, so the tiles at the
 // edges own that much more and W x H takes ceil((W - 2 halo) / TX) x
 // ceil((H - 2 halo) / TY) tiles.
@@ -17,44 +18,64 @@
 // vertical faces in registers, 3 per Jacobi update). Here the only traffic
 // between threads is one shuffle per row (8 cells, two rows of a colour) for
 // the faces between lanes, and 4 words up and 4 down per lane and half-sweep
-// between strips (two 16-byte stores and loads).
+// between strips, by an asynchronous store into the neighbouring strip's inbox
+// in shared memory, in its own CTA or the next one of the cluster, which an
+// mbarrier there counts. It is on its way while the strips' inner rows are
+// updated; no barrier of the CTA is in the sweeps.
 //
 // Updates are the plain kernels' expressions in the same order, so every
 // result has the same bits.
 #pragma once
 
+#include <cuda_runtime.h>
+
+#include <type_traits>
+
+#include "../../include/opensayal_gb300.h"
+#include "os_common.cuh"
+
 namespace osg {
 
 constexpr int kTileW = 256;      // region width in cells
 constexpr int kLaneCols = 8;     // columns per lane
-constexpr int kMaxTileWarps = 24;
 constexpr uint32_t kAllLanes = 0xffffffffu;
 
-// Warps per CTA that the register file holds for strips of R rows.
-constexpr int tile_max_warps(int R) {
-  return R <= 2 ? 24 : R <= 4 ? 16 : R <= 6 ? 12 : 8;
+// Strip heights the kernels are built for, and the warps per CTA that the
+// register file holds for each: a scheduler's 16,384 registers go to whole
+// warps, so 8 warps may use 255 registers a thread, 12 warps 168, 16 warps 128.
+constexpr int kProjectRows[] = {2, 4, 6, 8, 10};
+constexpr int kDiffuseRows[] = {2, 4, 6, 8, 12};
+__host__ __device__ constexpr int project_max_warps(int R) {
+  return R <= 4 ? 16 : R <= 6 ? 12 : 8;
 }
-
-// The same for the diffusion, which holds one field and two rows of neighbours.
-constexpr int diffuse_max_warps(int R) {
-  return R <= 2 ? 24 : R <= 4 ? 16 : R <= 8 ? 12 : 8;
+// The diffusion holds one field.
+__host__ __device__ constexpr int diffuse_max_warps(int R) {
+  return R <= 4 ? 16 : R <= 8 ? 12 : 8;
 }
 
 struct RegTile {
   int halo;              // halo in cells, on sides that have a neighbour
   int TX, TY;            // pitch of the tiles: region minus both halos
-  int RH;                // region rows, R * warps
-  int R, warps;
+  int RH;                // region rows, R * warps * cluster
+  int R, warps, cluster;
   int tiles_x, tiles_y;
-  size_t smem;
+  size_t smem;           // dynamic shared memory per CTA
 };
 
 struct ResidentSync {
-  unsigned* epochs;     // one per tile: passes exchanged so far (monotonic)
+  unsigned* epochs;     // one per CTA: exchanges so far (monotonic)
   uint4* packets;       // two copies of the exchanged cells (see the exchange below)
-  int* dev_err;         // set by a warp that gave up; polled by the others
+  int* dev_err;         // set by a thread that gave up; polled by the others
   int* host_err;        // mapped host word the host reads after synchronising
 };
+
+// A bounded wait gave up: the host reports it (OS_ERR_TIMEOUT).
+__device__ __forceinline__ void record_failure(const ResidentSync& sync) {
+  if (atomicCAS(sync.dev_err, 0, 1) == 0 && sync.host_err) {
+    *(volatile int*)sync.host_err = 1;
+    __threadfence_system();
+  }
+}
 
 // ---------------------------------------------------------------------------
 // Fields in global memory: quads of 4 columns.
@@ -134,26 +155,39 @@ __device__ __forceinline__ void on_cells(int storage, Fn&& fn) {
 // Where a thread's patch lies.
 // ---------------------------------------------------------------------------
 struct Patch {
-  int tx, ty;      // tile
   int gx0, gy0;    // region origin on the grid
   int lane, warp;
   int x0, y0;      // first column and row of the patch in the region
+  int yl;          // its first row among the CTA's rows
+  int c0, c1;      // the CTA's rows of the region
   bool left, right, below, above;  // the tile has a neighbour on that side
   int ox0, ox1, oy0, oy1;          // owned columns and rows, in the region
+  bool down, up;                   // the tile has a strip below / above this one
 };
 
-__device__ __forceinline__ Patch patch_of(int tx, int ty, const RegTile& g, int R, int W, int H) {
+// Worked out anew wherever it is used outside the sweeps (the block and thread
+// numbers pass through an empty asm, so that the compiler does not keep one
+// copy alive): held across the sweep loops it costs registers that their faces
+// need.
+__device__ __forceinline__ Patch patch_of(const RegTile& g, int R, int W, int H) {
   Patch P;
-  P.tx = tx, P.ty = ty;
+  unsigned block = blockIdx.x, thread = threadIdx.x;
+  asm volatile("" : "+r"(block), "+r"(thread));
+  const int tile = block / g.cluster, rank = block % g.cluster;
+  const int tx = tile % g.tiles_x, ty = tile / g.tiles_x;
   P.gx0 = tx * g.TX, P.gy0 = ty * g.TY;
-  P.lane = threadIdx.x & 31, P.warp = threadIdx.x >> 5;
-  P.x0 = P.lane * kLaneCols, P.y0 = P.warp * R;
+  P.lane = thread & 31, P.warp = thread >> 5;
+  P.yl = P.warp * R;
+  P.c0 = rank * g.warps * R, P.c1 = P.c0 + g.warps * R;
+  P.x0 = P.lane * kLaneCols, P.y0 = P.c0 + P.yl;
   P.left = tx > 0, P.right = tx + 1 < g.tiles_x;
   P.below = ty > 0, P.above = ty + 1 < g.tiles_y;
   P.ox0 = P.left ? g.halo : 0;
   P.oy0 = P.below ? g.halo : 0;
   P.ox1 = P.right ? kTileW - g.halo : min(kTileW, W - P.gx0);
   P.oy1 = P.above ? g.RH - g.halo : min(g.RH, H - P.gy0);
+  P.down = P.warp > 0 || rank > 0;
+  P.up = P.warp < g.warps - 1 || rank + 1 < g.cluster;
   return P;
 }
 
@@ -161,6 +195,127 @@ __device__ __forceinline__ Patch patch_of(int tx, int ty, const RegTile& g, int 
 __device__ __forceinline__ uint32_t rows_in(int y0, int R, int lo, int hi) {
   const int a = min(max(lo - y0, 0), R), b = min(max(hi - y0, 0), R);
   return ((1u << b) - 1u) & ~((1u << a) - 1u);
+}
+
+// ---------------------------------------------------------------------------
+// Messages between neighbouring strips of a tile.
+//
+// Each warp has an inbox in its CTA's shared memory: for message m (buffer m %
+// 2) one part from the strip below and one from the strip above, 16 or 32 bytes
+// a lane, and an mbarrier that completes when both have arrived. A strip sends
+// by asynchronous stores that complete bytes on the receiver's mbarrier, to a
+// warp of its own CTA or of the next one in the cluster in the same way (280
+// cycles from one CTA to the next; with a store, a fence and a remote arrival
+// it took 540). Message m + 2 takes the buffer of message m: its sender has by
+// then received the receiver's own message m + 1, which that strip sent after
+// it read message m. A strip at the tile's edge sends to itself what it would
+// send to the strip that is not there.
+// ---------------------------------------------------------------------------
+constexpr int kInboxHead = 16;      // two mbarriers
+constexpr int kMessageSpin = 1 << 20;  // polls of a bounded wait
+
+__host__ __device__ constexpr int inbox_bytes(int words) { return kInboxHead + 4 * words * 128; }
+
+__device__ __forceinline__ uint32_t shared_address(const void* p) {
+  return static_cast<uint32_t>(__cvta_generic_to_shared(p));
+}
+__device__ __forceinline__ uint32_t cluster_address(uint32_t a, int rank) {
+  uint32_t r;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
+  return r;
+}
+// (Not the .aligned forms: a warp may come here with its lanes apart.)
+__device__ __forceinline__ void cluster_arrive() {
+  asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+}
+__device__ __forceinline__ void cluster_wait() {
+  asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+}
+
+// WORDS: 32-bit words per lane in each part of a message (4 or 8).
+template <int WORDS>
+struct Link {
+  static constexpr int kPart = WORDS * 128;  // bytes of a part, 512 per 4 words
+  uint32_t mine;                 // this warp's inbox (shared address)
+  uint32_t up, down;             // the neighbours' inboxes (cluster shared addresses)
+  uint32_t up_part, down_part;   // where this strip's part goes in them
+};
+
+// Prepares the warp's inbox and finds the neighbours'; the caller passes a
+// cluster barrier before the first message.
+template <int WORDS>
+__device__ __forceinline__ Link<WORDS> open_link(char* smem, const Patch& P, const RegTile& g) {
+  constexpr int kBytes = kInboxHead + 4 * Link<WORDS>::kPart;
+  Link<WORDS> k;
+  const uint32_t base = shared_address(smem);
+  const int rank = blockIdx.x % g.cluster;
+  k.mine = base + P.warp * kBytes;
+  const uint32_t self = cluster_address(k.mine, rank);
+  k.up = P.up ? (P.warp + 1 < g.warps ? cluster_address(k.mine + kBytes, rank)
+                                      : cluster_address(base, rank + 1))
+              : self;
+  k.down = P.down ? (P.warp > 0 ? cluster_address(k.mine - kBytes, rank)
+                                : cluster_address(base + (g.warps - 1) * kBytes, rank - 1))
+                  : self;
+  // Part 0 comes from below, part 1 from above.
+  k.up_part = (P.up ? 0 : Link<WORDS>::kPart) + kInboxHead + P.lane * 16;
+  k.down_part = (P.down ? Link<WORDS>::kPart : 0) + kInboxHead + P.lane * 16;
+  if (P.lane == 0) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(k.mine) : "memory");
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(k.mine + 8) : "memory");
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  return k;
+}
+
+// Four words (words 4 k ..) of message m to an inbox.
+template <int WORDS>
+__device__ __forceinline__ void post(uint32_t inbox, uint32_t part, unsigned m, int k, float4 x) {
+  const uint32_t buffer = m & 1u;
+  asm volatile(
+      "st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%1, %2, %3, %4}, "
+      "[%5];" ::"r"(inbox + part + buffer * (2 * WORDS * 128) + k * 512),
+      "f"(x.x), "f"(x.y), "f"(x.z), "f"(x.w), "r"(inbox + 8 * buffer)
+      : "memory");
+}
+
+// Waits until both parts of message m are there. A wait that gives up records
+// the failure and carries on; the host reports it.
+template <int WORDS>
+__device__ __forceinline__ void await_message(const Link<WORDS>& link, unsigned m,
+                                              const ResidentSync& sync) {
+  const uint32_t bar = link.mine + 8 * (m & 1u);
+  if ((threadIdx.x & 31) == 0)
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar),
+                 "r"(2 * Link<WORDS>::kPart)
+                 : "memory");
+  uint32_t done = 0;
+#pragma unroll 1
+  for (int it = 0; !done; it++) {
+    asm volatile(
+        "{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
+        " selp.u32 %0, 1, 0, p;\n}"
+        : "=r"(done)
+        : "r"(bar), "r"((m >> 1) & 1u)
+        : "memory");
+    if (it >= kMessageSpin) {
+      record_failure(sync);
+      break;
+    }
+  }
+  __syncwarp();  // lanes may have left the loop apart
+}
+// Words 4 k .. of the part from below (0) or above (1) of message m.
+template <int WORDS>
+__device__ __forceinline__ float4 read_message(const Link<WORDS>& link, int part, unsigned m,
+                                               int k) {
+  float4 x;
+  asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+               : "=f"(x.x), "=f"(x.y), "=f"(x.z), "=f"(x.w)
+               : "r"(link.mine + kInboxHead + ((m & 1u) * 2 + part) * Link<WORDS>::kPart +
+                     k * 512 + (threadIdx.x & 31) * 16)
+               : "memory");
+  return x;
 }
 
 // ---------------------------------------------------------------------------
@@ -173,7 +328,9 @@ __device__ __forceinline__ uint32_t rows_in(int y0, int R, int lo, int hi) {
 // access, so a reader that sees the number it waits for has the values; there
 // is no fence, no flag and no barrier between tiles. (With the band stored to
 // the fields, a fence, a flag per warp, a poll and the reload, an exchange took
-// 4.2 us; the fence and the poll alone 2.3.)
+// 4.2 us; the fence and the poll alone 2.3.) Within a cluster no halo is needed:
+// the packets carry the sides of the tiles, and their lower and upper rows
+// where tiles lie above one another.
 //
 // Packets lie by the cell they carry, in two copies that alternate. A copy is
 // written again two exchanges later: by then the writer has received the
@@ -219,10 +376,7 @@ __device__ __forceinline__ bool packet_in(bool on, const uint4* p, float& a, flo
 // has (every later wait gives up at once), and the host reports it.
 __device__ __forceinline__ bool poll_again(int it, const ResidentSync& sync) {
   if (it < kSpinLimit && (it % 64 != 63 || !*(volatile int*)sync.dev_err)) return true;
-  if (atomicCAS(sync.dev_err, 0, 1) == 0) {
-    *(volatile int*)sync.host_err = 1;
-    __threadfence_system();
-  }
+  record_failure(sync);
   return false;
 }
 
@@ -256,6 +410,22 @@ __device__ __forceinline__ void patch_in(const IO& io, float (&f)[R][8], const v
     for (int q = 0; q < 8; q++) io.load1(j0 + r < H && x + q < W, row + q, &f[r][q]);
 }
 
+// Row y of the region, the lane's eight columns, in the same way.
+template <class IO>
+__device__ __forceinline__ void row_in(const IO& io, float (&f)[8], const void* field,
+                                       const Patch& P, int y, int W, int H, bool vec) {
+  const int x = P.gx0 + P.x0, j = min(P.gy0 + y, H - 1);
+  const typename IO::Word* row =
+      static_cast<const typename IO::Word*>(field) + (int64_t)(H - 1 - j) * W;
+  if (vec) {
+    io.load4(true, row + min(x, W - 4), &f[0]);
+    io.load4(true, row + min(x + 4, W - 4), &f[4]);
+  } else {
+#pragma unroll
+    for (int q = 0; q < 8; q++) io.load1(x + q < W, row + x + q, &f[q]);
+  }
+}
+
 // The patch's rows in `rows` out to a field, the owned columns among them.
 template <int R, class IO>
 __device__ __forceinline__ void patch_out(const IO& io, const float (&f)[R][8], void* field,
@@ -284,144 +454,170 @@ __device__ __forceinline__ void patch_out(const IO& io, const float (&f)[R][8], 
 template <int FIELDS>
 constexpr int kPacketsPerQuad = FIELDS == 2 ? 3 : 2;
 
-// The cells an exchange moves, as quads: 2 halo whole rows of the region (the
-// halo rows below and above as the ring; the owned rows beside them as the
-// band) and, in every row, halo columns on either side. Row quads are taken by
-// (row, which of the lane's two quads, lane), side quads by (row, side, quad),
-// both in shared memory and in the numbering of the items.
+// The cells an exchange moves, as quads: the CTA's rows of the tile's lower and
+// upper halo (the ring) or of the owned rows beside them (the band), and in
+// every row of the CTA halo columns on either side. The ring takes one row
+// more than the CTA has, the row above its top strip, whose lower faces that
+// strip holds copies of. Row quads are taken by (row, which of the lane's two
+// quads, lane), side quads by (row, side, quad), both in shared memory and in
+// the numbering of the items.
 constexpr int kRowQuads = kTileW / 4;
-struct Exchange {
-  float4* cells;  // rows: [2 halo][FIELDS][2][32], then sides: [RH][2][halo / 4][FIELDS]
-  int* send;      // per item: its packet's place, or -1 (not sent)
-  int* take;      // per item of the ring: its packet's place, or -1 (not taken)
-  int rows, items;  // row items, all items
+struct HaloRows {
+  int a0, an, b0, bn;  // rows [a0, a0 + an) and [b0, b0 + bn) of the region
+  int rows, items;     // row items, all items
 };
-inline __host__ __device__ int exchange_items(int halo, int RH) {
-  return 2 * halo * kRowQuads + RH * (halo / 2);
+struct Exchange {
+  float4* cells;  // rows: [an + bn][FIELDS][2][32], then sides: [rows][2][halo / 4][FIELDS]
+  int* send;      // per item of the band: its packet's place, or -1 (not sent)
+  int* take;      // per item of the ring: its packet's place, or -1 (not taken)
+  HaloRows band, ring;
+};
+// Items of a CTA of L rows at most.
+inline __host__ __device__ int exchange_items(int halo, int L) {
+  const int rows = 2 * (halo < L + 1 ? halo : L + 1);
+  return rows * kRowQuads + (L + 1) * (halo / 2);
 }
-inline __host__ __device__ size_t exchange_smem(int halo, int RH, int fields) {
-  return (size_t)exchange_items(halo, RH) * (fields * 16 + 8);
+inline __host__ __device__ size_t exchange_smem(int halo, int L, int fields) {
+  return (size_t)exchange_items(halo, L) * (fields * 16 + 8);
 }
 
-// Item `it` as a row and quad of the region, for the ring or the band `in`
-// cells inside it.
-__device__ __forceinline__ void exchange_cell(int it, int in, const RegTile& g, int rows, int* y,
-                                              int* q) {
-  const int h = g.halo, hq = h / 4;
-  if (it < rows) {
-    const int k = it / kRowQuads;
-    *y = k < h ? in + k : g.RH - h - in + (k - h);
-    *q = 2 * (it & 31) + ((it >> 5) & 1);
-  } else {
-    const int s = it - rows, k = s % (2 * hq);
-    *y = s / (2 * hq);
-    *q = k < hq ? in / 4 + k : kRowQuads - hq - in / 4 + (k - hq);
-  }
+__device__ __forceinline__ HaloRows halo_rows(int in, int c0, int c1, const Patch& P,
+                                              const RegTile& g) {
+  HaloRows s;
+  const int h = g.halo;
+  s.a0 = max(c0, in);
+  s.an = P.below ? max(0, min(c1, in + h) - s.a0) : 0;
+  s.b0 = max(c0, g.RH - h - in);
+  s.bn = P.above ? max(0, min(c1, g.RH - in) - s.b0) : 0;
+  s.rows = (s.an + s.bn) * kRowQuads;
+  s.items = s.rows + (c1 - c0) * (h / 2);
+  return s;
+}
+
+// The buffer and plan of an exchange in shared memory at `base`.
+__device__ __forceinline__ Exchange exchange_view(char* base, const Patch& P, const RegTile& g,
+                                                  int fields) {
+  Exchange x;
+  x.band = halo_rows(g.halo, P.c0, P.c1, P, g);
+  x.ring = halo_rows(0, P.c0, P.c1 + 1, P, g);
+  const int most = exchange_items(g.halo, P.c1 - P.c0);
+  x.cells = reinterpret_cast<float4*>(base);
+  x.send = reinterpret_cast<int*>(x.cells + most * fields);
+  x.take = x.send + most;
+  return x;
 }
 
 // The places of all items' packets, once per launch.
-__device__ __forceinline__ Exchange exchange_plan(char* base, const Patch& P, const RegTile& g,
-                                                  int fields, int W, int H) {
-  Exchange x;
-  const int h = g.halo;
-  x.rows = 2 * h * kRowQuads;
-  x.items = exchange_items(h, g.RH);
-  x.cells = reinterpret_cast<float4*>(base);
-  x.send = reinterpret_cast<int*>(x.cells + x.items * fields);
-  x.take = x.send + x.items;
+__device__ __forceinline__ void exchange_plan(char* base, const RegTile& g, int R, int fields,
+                                              int W, int H) {
+  const Patch P = patch_of(g, R, W, H);
+  const Exchange x = exchange_view(base, P, g, fields);
+  const int h = g.halo, hq = h / 4;
   const int half = (W + 7) / 8;  // pairs of quads in a row of the grid
-  for (int it = threadIdx.x; it < x.items; it += blockDim.x) {
-#pragma unroll
-    for (int band = 0; band < 2; band++) {
+#pragma unroll 1
+  for (int band = 0; band < 2; band++) {
+    const HaloRows s = band ? x.band : x.ring;
+    const int in = band ? h : 0;
+#pragma unroll 1
+    for (int it = threadIdx.x; it < s.items; it += blockDim.x) {
       int y, q;
-      exchange_cell(it, band ? h : 0, g, x.rows, &y, &q);
-      const int i = P.gx0 + 4 * q, j = P.gy0 + y;
-      bool on = i < W && j < H;
-      if (it < x.rows) {
-        on = on && (it < x.rows / 2 ? P.below : P.above);
+      bool on;
+      if (it < s.rows) {
+        const int k = it / kRowQuads;
+        y = k < s.an ? s.a0 + k : s.b0 + (k - s.an);
+        q = 2 * (it & 31) + ((it >> 5) & 1);
+        // A row of both bands goes once.
+        on = !band || k < s.an || !(P.below && y < 2 * h);
       } else {
-        const bool left = (it - x.rows) % (h / 2) < h / 4;
-        on = on && (left ? P.left : P.right) && y >= P.oy0 && y < P.oy1;
+        const int e = it - s.rows, k = e % (2 * hq);
+        y = P.c0 + e / (2 * hq);
+        q = k < hq ? in / 4 + k : kRowQuads - hq - in / 4 + (k - hq);
+        on = (k < hq ? P.left : P.right) && y >= P.oy0 && y < P.oy1;
+        // A side quad of a band row goes with its row.
+        if (band)
+          on = on && !(P.below && y < 2 * h) && !(P.above && y >= g.RH - 2 * h);
       }
-      if (band) {
-        // A row of both bands goes once, and a side quad of a band row with
-        // its row; only owned columns go.
-        const bool low = P.below && y < 2 * h, high = P.above && y >= g.RH - 2 * h;
-        on = on && (it < x.rows / 2 || !low) && (it < x.rows || !high) && 4 * q >= P.ox0 &&
-             4 * q < P.ox1;
-      }
+      const int i = P.gx0 + 4 * q, j = P.gy0 + y;
+      on = on && i < W && j < H && y < g.RH;
+      if (band) on = on && 4 * q >= P.ox0 && 4 * q < P.ox1;  // only owned columns go
       const int Q = i / 4;
       (band ? x.send : x.take)[it] = on ? (j * 2 + (Q & 1)) * half + (Q >> 1) : -1;
     }
   }
-  return x;
 }
 // Packets of one plane (values 3 k .. 3 k + 2 of every quad of the grid).
 inline __host__ __device__ int64_t packet_plane(int W, int H) {
   return (int64_t)H * 2 * ((W + 7) / 8);
 }
 
-// The rows and side quads of a patch between registers and the buffer: `in` = 0
-// the ring into the registers, `in` = halo the band out of them.
+// A lane's two quads of rows between registers and the buffer.
+template <bool OUT>
+__device__ __forceinline__ void move_quad(float4* p, float* q) {
+  if (OUT) {
+    *p = make_float4(q[0], q[1], q[2], q[3]);
+  } else {
+    const float4 t = *p;
+    q[0] = t.x, q[1] = t.y, q[2] = t.z, q[3] = t.w;
+  }
+}
+
+// The patch's share of the band out of the registers (BAND), or of the ring
+// into them; with the ring also row R of the strip, the faces `f_top` of the
+// last field that lie on the strip's upper edge.
 template <int FIELDS, bool BAND, int R>
 __device__ __forceinline__ void exchange_patch(float (&f)[R][8], float (&f2)[R][8],
-                                               const Exchange& x, const Patch& P,
-                                               const RegTile& g) {
+                                               float (&f_top)[8], const Exchange& x,
+                                               const Patch& P, const RegTile& g) {
   const int h = g.halo, hq = h / 4, in = BAND ? h : 0;
-  auto move = [&](float4* p, float* q) {
-    if (BAND) {
-      *p = make_float4(q[0], q[1], q[2], q[3]);
-    } else {
-      const float4 t = *p;
-      q[0] = t.x, q[1] = t.y, q[2] = t.z, q[3] = t.w;
-    }
-  };
+  const HaloRows s = BAND ? x.band : x.ring;
   // Side quads of the lane (halos are whole numbers of quads).
   const int l0 = 2 * P.lane - in / 4, r0 = 2 * P.lane - (kRowQuads - hq - in / 4);
-  uint32_t side[2];
-  float4* at[2];
+  constexpr int kRows = BAND ? R : R + 1;  // row R: the strip above's first
+  const uint32_t whole = rows_in(P.y0, kRows, s.a0, s.a0 + s.an) |
+                         rows_in(P.y0, kRows, s.b0, s.b0 + s.bn);
+  const uint32_t owned = rows_in(P.y0, kRows, P.oy0, P.oy1) & ~whole;
+#pragma unroll
+  for (int r = 0; r < kRows; r++) {
+    if (((whole >> r) & 1u) == 0u) continue;  // the same for the warp
+    const int y = P.y0 + r;
+    const int k = y >= s.a0 && y < s.a0 + s.an ? y - s.a0 : s.an + y - s.b0;
+    float4* row = x.cells + k * FIELDS * 64 + P.lane;
+    if (r < R) {
+      move_quad<BAND>(row, &f[r < R ? r : 0][0]);
+      move_quad<BAND>(row + 32, &f[r < R ? r : 0][4]);
+      if (FIELDS == 2) {
+        move_quad<BAND>(row + 64, &f2[r < R ? r : 0][0]);
+        move_quad<BAND>(row + 96, &f2[r < R ? r : 0][4]);
+      }
+    } else if (FIELDS == 2 && P.up) {
+      move_quad<BAND>(row + 64, &f_top[0]);
+      move_quad<BAND>(row + 96, &f_top[4]);
+    }
+  }
 #pragma unroll
   for (int c = 0; c < 2; c++) {
     const bool left = P.left && l0 + c >= 0 && l0 + c < hq;
     const bool right = P.right && r0 + c >= 0 && r0 + c < hq;
-    side[c] = left || right ? rows_in(P.y0, R, P.oy0, P.oy1) : 0u;
-    at[c] = x.cells + x.rows * FIELDS +
-            (P.y0 * 2 * hq + (left ? l0 + c : hq + r0 + c)) * FIELDS;
-  }
-  uint32_t whole = (P.below ? rows_in(P.y0, R, in, in + h) : 0u) |
-                   (P.above ? rows_in(P.y0, R, g.RH - h - in, g.RH - in) : 0u);
+    if (!left && !right) continue;
+    float4* p = x.cells + s.rows * FIELDS + (P.yl * 2 * hq + (left ? l0 + c : hq + r0 + c)) * FIELDS;
 #pragma unroll
-  for (int r = 0; r < R; r++) {
-    if ((whole >> r) & 1u) {  // the same for the warp
-      const int y = P.y0 + r;
-      const int k = P.below && y < in + h ? y - in : h + y - (g.RH - h - in);
-      float4* row = x.cells + k * FIELDS * 64 + P.lane;
-      move(row, &f[r][0]);
-      move(row + 32, &f[r][4]);
-      if (FIELDS == 2) {
-        move(row + 64, &f2[r][0]);
-        move(row + 96, &f2[r][4]);
+    for (int r = 0; r < kRows; r++) {
+      if (((owned >> r) & 1u) == 0u) continue;
+      float4* at = p + r * 2 * hq * FIELDS;
+      if (r < R) {
+        move_quad<BAND>(at, &f[r < R ? r : 0][4 * c]);
+        if (FIELDS == 2) move_quad<BAND>(at + 1, &f2[r < R ? r : 0][4 * c]);
+      } else if (FIELDS == 2 && P.up) {
+        move_quad<BAND>(at + 1, &f_top[4 * c]);
       }
-    }
-  }
-#pragma unroll
-  for (int c = 0; c < 2; c++) {
-    const uint32_t m = side[c] & ~whole;
-    if (m == 0u) continue;
-#pragma unroll
-    for (int r = 0; r < R; r++) {
-      if (((m >> r) & 1u) == 0u) continue;
-      float4* p = at[c] + r * 2 * hq * FIELDS;
-      move(p, &f[r][4 * c]);
-      if (FIELDS == 2) move(p + 1, &f2[r][4 * c]);
     }
   }
 }
 
 // Place of an item's first field in the buffer, and the step to the second.
 template <int FIELDS>
-__device__ __forceinline__ float4* exchange_at(const Exchange& x, int it, int* step) {
-  if (it < x.rows) {
+__device__ __forceinline__ float4* exchange_at(const Exchange& x, int rows, int it, int* step) {
+  if (it < rows) {
     *step = 64;
     return x.cells + (it >> 6) * FIELDS * 64 + (it & 63);
   }
@@ -436,19 +632,24 @@ __device__ __forceinline__ float4* exchange_at(const Exchange& x, int it, int* s
 // lanes at the edges use a part, an exchange took 14000 cycles, most of it
 // instruction fetch.
 template <int FIELDS, int R>
-__device__ __forceinline__ void exchange(float (&f)[R][8], float (&f2)[R][8], const Exchange& x,
-                                         const ResidentSync& sync, const Patch& P,
-                                         const RegTile& g, int64_t plane, unsigned number) {
+__device__ __forceinline__ void exchange(float (&f)[R][8], float (&f2)[R][8], float (&f_top)[8],
+                                         char* base, const ResidentSync& sync, const RegTile& g,
+                                         int W, int H, unsigned number) {
+  const int64_t plane = packet_plane(W, H);
   constexpr int kPer = kPacketsPerQuad<FIELDS>;
   uint4* packets = sync.packets + (number & 1) * kPer * plane;
-  exchange_patch<FIELDS, true, R>(f, f2, x, P, g);
+  {
+    const Patch P = patch_of(g, R, W, H);
+    exchange_patch<FIELDS, true, R>(f, f2, f_top, exchange_view(base, P, g, FIELDS), P, g);
+  }
   __syncthreads();
+  const Exchange x = exchange_view(base, patch_of(g, R, W, H), g, FIELDS);
 #pragma unroll 1
-  for (int it = threadIdx.x; it < x.items; it += blockDim.x) {
+  for (int it = threadIdx.x; it < x.band.items; it += blockDim.x) {
     const int place = x.send[it];
     if (place < 0) continue;
     int step;
-    const float4* c = exchange_at<FIELDS>(x, it, &step);
+    const float4* c = exchange_at<FIELDS>(x, x.band.rows, it, &step);
     uint4* p = packets + place;
     const float4 a = c[0];
     packet_out(true, p, a.x, a.y, a.z, number);
@@ -460,17 +661,17 @@ __device__ __forceinline__ void exchange(float (&f)[R][8], float (&f2)[R][8], co
       packet_out(true, p + plane, a.w, 0.0f, 0.0f, number);
     }
   }
-  constexpr int kAtOnce = 2;
+  constexpr int kAtOnce = R == 4 || R == 6 ? 1 : 2;  // what those strips' registers leave
 #pragma unroll 1
-  for (int base = 0; base < x.items; base += kAtOnce * blockDim.x) {
+  for (int first = 0; first < x.ring.items; first += kAtOnce * blockDim.x) {
     float v[kAtOnce][9];
     const uint4* p[kAtOnce];
     int at[kAtOnce];
     bool on[kAtOnce], ok;
 #pragma unroll
     for (int k = 0; k < kAtOnce; k++) {
-      at[k] = base + k * blockDim.x + threadIdx.x;
-      const int place = at[k] < x.items ? x.take[at[k]] : -1;
+      at[k] = first + k * blockDim.x + threadIdx.x;
+      const int place = at[k] < x.ring.items ? x.take[at[k]] : -1;
       on[k] = place >= 0;
       p[k] = packets + max(place, 0);
     }
@@ -484,18 +685,19 @@ __device__ __forceinline__ void exchange(float (&f)[R][8], float (&f2)[R][8], co
           ok &= packet_in(on[k], p[k] + j * plane, v[k][3 * j], v[k][3 * j + 1], v[k][3 * j + 2],
                           number);
     } while (!ok && poll_again(poll++, sync));
-    if (base == 0) __syncthreads();  // the band has been read: the buffer takes the ring
+    if (first == 0) __syncthreads();  // the band has been read: the buffer takes the ring
 #pragma unroll
     for (int k = 0; k < kAtOnce; k++) {
       if (!on[k]) continue;
       int step;
-      float4* c = exchange_at<FIELDS>(x, at[k], &step);
+      float4* c = exchange_at<FIELDS>(x, x.ring.rows, at[k], &step);
       c[0] = make_float4(v[k][0], v[k][1], v[k][2], v[k][3]);
       if (FIELDS == 2) c[step] = make_float4(v[k][4], v[k][5], v[k][6], v[k][7]);
     }
   }
   __syncthreads();
-  exchange_patch<FIELDS, false, R>(f, f2, x, P, g);
+  const Patch P = patch_of(g, R, W, H);
+  exchange_patch<FIELDS, false, R>(f, f2, f_top, exchange_view(base, P, g, FIELDS), P, g);
 }
 
 // With 16-bit storage the cells a tile keeps get the rounding that a store and
@@ -507,6 +709,11 @@ __device__ __forceinline__ void round_patch(float (&f)[R][8], int storage) {
   for (int r = 0; r < R; r++)
 #pragma unroll
     for (int q = 0; q < 8; q++) f[r][q] = io.from(io.to(f[r][q]));
+}
+__device__ __forceinline__ void round_row(float (&f)[8], int storage) {
+  const HalfCells io{storage == OS_STORAGE_BF16};
+#pragma unroll
+  for (int q = 0; q < 8; q++) f[q] = io.from(io.to(f[q]));
 }
 
 // ---------------------------------------------------------------------------
@@ -626,27 +833,29 @@ __device__ __forceinline__ void row_flags(uint32_t w, float4 rs, float (&u)[8], 
   if (PRESSURE) *pw = p4;
 }
 
-// Shared memory of a projection tile: strip boundaries, the cells' reciprocal
-// neighbour counts, (PRESSURE) the pressure and the flag words.
+// Shared memory of a projection tile after the warps' inboxes: the cells'
+// reciprocal neighbour counts, (PRESSURE) the pressure and the flag words.
 struct ProjSmem {
-  float4* slot;      // [warps][2][32]
-  float4* rs;        // [RH][2][32]
-  float4* p;         // [RH][2][32]
-  uint32_t* flags;   // [RH][2][32]
+  float4* rs;        // [rows][2][32]
+  float4* p;         // [rows][2][32]
+  uint32_t* flags;   // [rows][2][32]
+  char* exchange;
 };
 
-__host__ __device__ inline size_t project_tile_smem(int RH, int warps, bool pressure, int halo,
+__host__ __device__ inline size_t project_tile_smem(int rows, int warps, bool pressure, int halo,
                                                     bool resident) {
-  return (size_t)warps * 64 * 16 + (size_t)RH * 64 * ((pressure ? 32 : 16) + 4) +
-         (resident ? exchange_smem(halo, RH, 2) : 0);
+  return (size_t)warps * inbox_bytes(4) +
+         (size_t)rows * 64 * ((pressure ? 32 : 16) + 4) +
+         (resident ? exchange_smem(halo, rows, 2) : 0);
 }
 
-__device__ __forceinline__ ProjSmem project_smem_of(char* base, int RH, int warps, bool pressure) {
+__device__ __forceinline__ ProjSmem project_smem_of(char* base, int rows, int warps,
+                                                    bool pressure) {
   ProjSmem s;
-  s.slot = reinterpret_cast<float4*>(base);
-  s.rs = s.slot + warps * 64;
-  s.p = s.rs + RH * 64;
-  s.flags = reinterpret_cast<uint32_t*>(s.p + (pressure ? RH * 64 : 0));
+  s.rs = reinterpret_cast<float4*>(base + warps * inbox_bytes(4));
+  s.p = s.rs + rows * 64;
+  s.flags = reinterpret_cast<uint32_t*>(s.p + (pressure ? rows * 64 : 0));
+  s.exchange = reinterpret_cast<char*>(s.flags + rows * 64);
   return s;
 }
 
@@ -719,7 +928,7 @@ __device__ __forceinline__ void flags_in(const uint8_t* __restrict__ flags, cons
   if (L.full) return;
 #pragma unroll
   for (int r = 0; r < R; r++) {
-    const int e = (P.y0 + r) * 64 + P.lane;
+    const int e = (P.yl + r) * 64 + P.lane;
     sm.flags[e] = raw[r][0];
     sm.flags[e + 32] = raw[r][1];
     sm.rs[e] = reciprocal_counts(raw[r][0]);
@@ -746,128 +955,119 @@ __device__ __forceinline__ void row_share(float (&u)[8], float& ur, const ProjLa
 // loop of its own, so that no loop holds the registers of another's rows.
 enum class Rows { kPlain, kWall, kFlags };
 
-// One colour half-sweep over the strip. The rows between the first and the
-// last come first, so that the faces that arrived from the other strips and
-// lanes have time to arrive, and those that go to them leave last; the rows
-// of a colour share no face, so their order is free.
+// Row r of a strip in one colour's half-sweep, and the face it shares with the
+// neighbouring lane.
 template <int COLOUR, bool PRESSURE, Rows ROWS, int R>
-__device__ __forceinline__ void strip_rows(float (&u)[R][8], float (&v)[R][8], float (&ur)[R],
-                                           float (&vt)[8], const ProjLane& L, const ProjSmem& sm,
-                                           int cell0, const Consts& c, float d_t) {
-#pragma unroll
-  for (int k = 0; k < R; k++) {
-    const int r = k + 2 < R ? k + 1 : k + 2 == R ? 0 : R - 1;  // 1 .. R - 2, 0, R - 1
-    float(&top)[8] = r + 1 < R ? v[r + 1 < R ? r + 1 : 0] : vt;
-    const int e = cell0 + r * 64 + ((r + COLOUR) & 1) * 32;
-    float4* p = PRESSURE ? sm.p + e : nullptr;
-    constexpr bool full = ROWS != Rows::kFlags;
-    if ((r + COLOUR) & 1) {
-      if (full)
-        row_full<1, PRESSURE, ROWS != Rows::kPlain>(u[r], ur[r], v[r], top, L, c, d_t, p);
-      else
-        row_flags<1, PRESSURE>(sm.flags[e], sm.rs[e], u[r], ur[r], v[r], top, c, d_t, p);
-      row_share<1>(u[r], ur[r], L);
-    } else {
-      if (full)
-        row_full<0, PRESSURE, ROWS != Rows::kPlain>(u[r], ur[r], v[r], top, L, c, d_t, p);
-      else
-        row_flags<0, PRESSURE>(sm.flags[e], sm.rs[e], u[r], ur[r], v[r], top, c, d_t, p);
-      row_share<0>(u[r], ur[r], L);
-    }
+__device__ __forceinline__ void strip_row(int r, float (&u)[R][8], float (&v)[R][8],
+                                          float (&ur)[R], float (&vt)[8], const ProjLane& L,
+                                          const ProjSmem& sm, int cell0, const Consts& c,
+                                          float d_t) {
+  float(&top)[8] = r + 1 < R ? v[r + 1 < R ? r + 1 : 0] : vt;
+  const int e = cell0 + r * 64 + ((r + COLOUR) & 1) * 32;
+  float4* p = PRESSURE ? sm.p + e : nullptr;
+  constexpr bool full = ROWS != Rows::kFlags;
+  if ((r + COLOUR) & 1) {
+    if (full)
+      row_full<1, PRESSURE, ROWS != Rows::kPlain>(u[r], ur[r], v[r], top, L, c, d_t, p);
+    else
+      row_flags<1, PRESSURE>(sm.flags[e], sm.rs[e], u[r], ur[r], v[r], top, c, d_t, p);
+    row_share<1>(u[r], ur[r], L);
+  } else {
+    if (full)
+      row_full<0, PRESSURE, ROWS != Rows::kPlain>(u[r], ur[r], v[r], top, L, c, d_t, p);
+    else
+      row_flags<0, PRESSURE>(sm.flags[e], sm.rs[e], u[r], ur[r], v[r], top, c, d_t, p);
+    row_share<0>(u[r], ur[r], L);
   }
 }
 
-// The faces between strips after a half-sweep, through the slots, 4 words each
-// way: a strip sends those its half-sweep changed, and after the barrier that
-// ends the half-sweep reads those its neighbours changed. A slot is next
-// written by the side that read it, so one barrier per half-sweep suffices.
+// The faces on a strip's edges after a half-sweep, 4 words each way: a strip
+// sends those its half-sweep changed, and receives those its neighbours
+// changed.
 template <int COLOUR, int R>
 __device__ __forceinline__ void strip_send(const float (&v)[R][8], const float (&vt)[8],
-                                           const Patch& P, const ProjSmem& sm, int warps) {
+                                           const Link<4>& link, unsigned m) {
   constexpr int cb = COLOUR, ct = (COLOUR + R - 1) & 1;  // of the bottom and the top row
-  if (P.warp + 1 < warps)
-    sm.slot[(P.warp * 2 + ct) * 32 + P.lane] = make_float4(vt[ct], vt[ct + 2], vt[ct + 4], vt[ct + 6]);
-  if (P.warp > 0)
-    sm.slot[((P.warp - 1) * 2 + cb) * 32 + P.lane] =
-        make_float4(v[0][cb], v[0][cb + 2], v[0][cb + 4], v[0][cb + 6]);
+  post<4>(link.up, link.up_part, m, 0, make_float4(vt[ct], vt[ct + 2], vt[ct + 4], vt[ct + 6]));
+  post<4>(link.down, link.down_part, m, 0,
+          make_float4(v[0][cb], v[0][cb + 2], v[0][cb + 4], v[0][cb + 6]));
 }
 
 template <int COLOUR, int R>
-__device__ __forceinline__ void strip_receive(float (&v)[R][8], float (&vt)[8], const Patch& P,
-                                              const ProjSmem& sm, int warps) {
+__device__ __forceinline__ void strip_receive(float (&v)[R][8], float (&vt)[8],
+                                              const Link<4>& link, unsigned m, bool down,
+                                              const ResidentSync& sync) {
   constexpr int nb = 1 - COLOUR, nt = 1 - ((COLOUR + R - 1) & 1);
-  if (P.warp + 1 < warps) {
-    const float4 t = sm.slot[(P.warp * 2 + nt) * 32 + P.lane];
-    vt[nt] = t.x, vt[nt + 2] = t.y, vt[nt + 4] = t.z, vt[nt + 6] = t.w;
-  }
-  if (P.warp > 0) {
-    const float4 t = sm.slot[((P.warp - 1) * 2 + nb) * 32 + P.lane];
-    v[0][nb] = t.x, v[0][nb + 2] = t.y, v[0][nb + 4] = t.z, v[0][nb + 6] = t.w;
-  }
+  await_message(link, m, sync);
+  const float4 b = read_message(link, 0, m, 0), t = read_message(link, 1, m, 0);
+  // Without a strip above, the top face is one that nothing owned depends on;
+  // without a strip below, the bottom face stays.
+  vt[nt] = t.x, vt[nt + 2] = t.y, vt[nt + 4] = t.z, vt[nt + 6] = t.w;
+  v[0][nb] = down ? b.x : v[0][nb], v[0][nb + 2] = down ? b.y : v[0][nb + 2];
+  v[0][nb + 4] = down ? b.z : v[0][nb + 4], v[0][nb + 6] = down ? b.w : v[0][nb + 6];
+}
+
+// A half-sweep: the strip's inner rows, then (while those ran, the last
+// half-sweep's faces came in) its first and last row, whose faces go out. The
+// rows of a colour share no face, so their order is free. Message m comes in,
+// m + 1 goes out.
+template <int COLOUR, bool PRESSURE, Rows ROWS, int R>
+__device__ __forceinline__ void half_sweep(float (&u)[R][8], float (&v)[R][8], float (&ur)[R],
+                                           float (&vt)[8], const ProjLane& L, const ProjSmem& sm,
+                                           const Link<4>& link, const ResidentSync& sync,
+                                           int cell0, bool down, unsigned m, const Consts& c,
+                                           float d_t) {
+#pragma unroll
+  for (int r = 1; r < R - 1; r++)
+    strip_row<COLOUR, PRESSURE, ROWS, R>(r, u, v, ur, vt, L, sm, cell0, c, d_t);
+  strip_receive<1 - COLOUR, R>(v, vt, link, m, down, sync);
+  strip_row<COLOUR, PRESSURE, ROWS, R>(0, u, v, ur, vt, L, sm, cell0, c, d_t);
+  strip_row<COLOUR, PRESSURE, ROWS, R>(R - 1, u, v, ur, vt, L, sm, cell0, c, d_t);
+  strip_send<COLOUR, R>(v, vt, link, m + 1);
 }
 
 template <bool PRESSURE, Rows ROWS, int R>
 __device__ __forceinline__ void sweep_loop(float (&u)[R][8], float (&v)[R][8], float (&ur)[R],
-                                           float (&vt)[8], const Patch& P, const ProjLane& L,
-                                           const ProjSmem& sm, const RegTile& g, const Consts& c,
-                                           float d_t, int sweeps) {
-  const int warps = g.warps, cell0 = P.y0 * 64 + P.lane;
+                                           float (&vt)[8], const ProjLane& L, const ProjSmem& sm,
+                                           const Link<4>& link, const ResidentSync& sync,
+                                           int cell0, bool down, const Consts& c, float d_t,
+                                           int sweeps, unsigned m) {
 #pragma unroll 1
-  for (int t = 0; t < sweeps; t++) {
-    const int reach = 2 * (sweeps - t) - 1;  // half-sweeps after the even one
-    // Rows [halo - 1 - reach, RH - halo + reach) reach an owned face, on
-    // sides that have a halo at all.
-    const bool even = (!P.below || P.y0 + R > g.halo - 1 - reach) &&
-                      (!P.above || P.y0 < g.RH - g.halo + reach);
-    const bool odd = (!P.below || P.y0 + R > g.halo - reach) &&
-                     (!P.above || P.y0 < g.RH - g.halo + reach - 1);
-    if (even) strip_rows<0, PRESSURE, ROWS, R>(u, v, ur, vt, L, sm, cell0, c, d_t);
-    strip_send<0, R>(v, vt, P, sm, warps);
-    __syncthreads();
-    strip_receive<0, R>(v, vt, P, sm, warps);
-    if (odd) strip_rows<1, PRESSURE, ROWS, R>(u, v, ur, vt, L, sm, cell0, c, d_t);
-    strip_send<1, R>(v, vt, P, sm, warps);
-    __syncthreads();
-    strip_receive<1, R>(v, vt, P, sm, warps);
+  for (int t = 0; t < sweeps; t++, m += 2) {
+    half_sweep<0, PRESSURE, ROWS, R>(u, v, ur, vt, L, sm, link, sync, cell0, down, m, c, d_t);
+    half_sweep<1, PRESSURE, ROWS, R>(u, v, ur, vt, L, sm, link, sync, cell0, down, m + 1, c, d_t);
   }
 }
 
-// `sweeps` red/black sweeps of the region. Rows that cannot reach an owned
-// face any more are skipped strip by strip; within a strip every cell is
-// updated: a cell off the cone of dependence writes faces that only cells off
-// the cone read from then on.
+// Messages of a segment of sweeps.
+__device__ __forceinline__ unsigned project_messages(int sweeps) { return 2 * sweeps + 1; }
+
+// `sweeps` red/black sweeps of the region, messages m .. m + 2 sweeps. Every
+// cell of the region is updated: validity shrinks by one cell per half-sweep
+// from the edges that have a halo, and a cell beyond writes faces that only
+// cells beyond read from then on.
 template <bool PRESSURE, int R>
-__device__ __forceinline__ void tile_sweeps(float (&u)[R][8], float (&v)[R][8], const Patch& P,
+__device__ __forceinline__ void tile_sweeps(float (&u)[R][8], float (&v)[R][8], float (&vt)[8],
                                             const ProjLane& L, const ProjSmem& sm,
-                                            const RegTile& g, const Consts& c, float d_t,
-                                            int sweeps) {
+                                            const Link<4>& link, const ResidentSync& sync,
+                                            int cell0, bool down, const Consts& c, float d_t,
+                                            int sweeps, unsigned m) {
   static_assert(R % 2 == 0, "strips start on even rows");
-  const int warps = g.warps;
-  float ur[R], vt[8];
-  __syncthreads();  // the slots' last readers
-  if (P.warp > 0) {
-    float4* s = sm.slot + (P.warp - 1) * 64 + P.lane;
-    s[0] = make_float4(v[0][0], v[0][2], v[0][4], v[0][6]);
-    s[32] = make_float4(v[0][1], v[0][3], v[0][5], v[0][7]);
-  }
-  __syncthreads();
-#pragma unroll
-  for (int q = 0; q < 8; q++) vt[q] = 0.0f;
-  if (P.warp + 1 < warps) {
-    const float4* s = sm.slot + P.warp * 64 + P.lane;
-    const float4 e = s[0], o = s[32];
-    vt[0] = e.x, vt[2] = e.y, vt[4] = e.z, vt[6] = e.w;
-    vt[1] = o.x, vt[3] = o.y, vt[5] = o.z, vt[7] = o.w;
-  }
+  float ur[R];
 #pragma unroll
   for (int r = 0; r < R; r++) ur[r] = __shfl_down_sync(kAllLanes, u[r][0], 1);
-  __syncthreads();  // every strip has its copies before a slot is rewritten
+  // The faces as they are, for the first half-sweep to receive.
+  strip_send<1, R>(v, vt, link, m);
   if (!L.full)
-    sweep_loop<PRESSURE, Rows::kFlags, R>(u, v, ur, vt, P, L, sm, g, c, d_t, sweeps);
+    sweep_loop<PRESSURE, Rows::kFlags, R>(u, v, ur, vt, L, sm, link, sync, cell0, down, c, d_t,
+                                          sweeps, m);
   else if (L.wall)
-    sweep_loop<PRESSURE, Rows::kWall, R>(u, v, ur, vt, P, L, sm, g, c, d_t, sweeps);
+    sweep_loop<PRESSURE, Rows::kWall, R>(u, v, ur, vt, L, sm, link, sync, cell0, down, c, d_t,
+                                         sweeps, m);
   else
-    sweep_loop<PRESSURE, Rows::kPlain, R>(u, v, ur, vt, P, L, sm, g, c, d_t, sweeps);
+    sweep_loop<PRESSURE, Rows::kPlain, R>(u, v, ur, vt, L, sm, link, sync, cell0, down, c, d_t,
+                                          sweeps, m);
+  strip_receive<1, R>(v, vt, link, m + 2 * sweeps, down, sync);
 }
 
 // apply_extrapolation_at (src/fluid.cu:720-733) on a patch, in
@@ -929,7 +1129,7 @@ __device__ __forceinline__ void pressure_in(const ProjSmem& sm, const float* p, 
   }
 #pragma unroll
   for (int r = 0; r < R; r++) {
-    float4* out = sm.p + (P.y0 + r) * 64 + P.lane;
+    float4* out = sm.p + (P.yl + r) * 64 + P.lane;
     out[0] = make_float4(f[r][0], f[r][2], f[r][4], f[r][6]);
     out[32] = make_float4(f[r][1], f[r][3], f[r][5], f[r][7]);
   }
@@ -941,7 +1141,7 @@ __device__ __forceinline__ void pressure_out(const ProjSmem& sm, float* p, const
   float f[R][8];
 #pragma unroll
   for (int r = 0; r < R; r++) {
-    const float4* in = sm.p + (P.y0 + r) * 64 + P.lane;
+    const float4* in = sm.p + (P.yl + r) * 64 + P.lane;
     const float4 e = in[0], o = in[32];
     f[r][0] = e.x, f[r][2] = e.y, f[r][4] = e.z, f[r][6] = e.w;
     f[r][1] = o.x, f[r][3] = o.y, f[r][5] = o.z, f[r][7] = o.w;
@@ -977,83 +1177,92 @@ struct ProjectArgs {
 // K sweeps through memory: with 16-bit storage the fields are rounded after
 // every K sweeps, and they end in the copy those passes would end in.
 template <int R, bool PRESSURE>
-__global__ void __launch_bounds__(32 * tile_max_warps(R), 1)
+__global__ void __launch_bounds__(32 * project_max_warps(R), 1)
 k_project_tiles(const __grid_constant__ ProjectArgs a) {
   extern __shared__ __align__(16) char tile_smem[];
   const Consts& c = a.c;
-  const int W = c.W, H = c.H;
-  const Patch P = patch_of(blockIdx.x % a.g.tiles_x, blockIdx.x / a.g.tiles_x, a.g, R, W, H);
-  const ProjSmem sm = project_smem_of(tile_smem, a.g.RH, a.g.warps, PRESSURE);
+  const int W = c.W, H = c.H, rows = a.g.warps * R;
+  const Patch P = patch_of(a.g, R, W, H);
+  const ProjSmem sm = project_smem_of(tile_smem, rows, a.g.warps, PRESSURE);
+  const Link<4> link = open_link<4>(tile_smem, P, a.g);
+  cluster_arrive();
   const bool vec = ((W | a.g.halo) & 3) == 0;
   ProjLane L;
   // The flags do not change after creation: staged before the wait for the
   // kernel before.
   flags_in<R>(a.flags, P, sm, W, H, vec, L);
   pdl_entry();
-  float u[R][8], v[R][8];
+  float u[R][8], v[R][8], vt[8];
 #pragma unroll
   for (int r = 0; r < R; r++)
 #pragma unroll
     for (int q = 0; q < 8; q++) u[r][q] = v[r][q] = 0.0f;
+#pragma unroll
+  for (int q = 0; q < 8; q++) vt[q] = 0.0f;
   if (PRESSURE) pressure_in<R>(sm, a.p, P, W, a.zero_pressure, H, vec);
   const float d_t = a.prm->dt;
   on_cells(a.storage, [&](auto io) {
+    const void* vi = a.cv ? a.V1 : a.V0;
     patch_in<R>(io, u, a.cu ? a.U1 : a.U0, P, W, H, vec);
-    patch_in<R>(io, v, a.cv ? a.V1 : a.V0, P, W, H, vec);
+    patch_in<R>(io, v, vi, P, W, H, vec);
+    if (P.up) row_in(io, vt, vi, P, P.y0 + R, W, H, vec);
   });
   const unsigned epoch = a.n > a.D ? ld_acquire_gpu(a.sync.epochs + blockIdx.x) : 0u;
   unsigned number = epoch;
-  Exchange x;
-  if (a.n > a.D)
-    x = exchange_plan(reinterpret_cast<char*>(sm.flags + a.g.RH * 64), P, a.g, 2, W, H);
-  const int64_t plane = packet_plane(W, H);
+  if (a.n > a.D) exchange_plan(sm.exchange, a.g, R, 2, W, H);
+  cluster_wait();  // every inbox of the cluster is open
+  unsigned message = 0;
 #pragma unroll 1
   for (int done = 0; done < a.n;) {
     if (done > 0) {
       if (a.storage != OS_STORAGE_F32 && done % a.K == 0) {
         round_patch<R>(u, a.storage);
         round_patch<R>(v, a.storage);
+        round_row(vt, a.storage);
       }
-      number++;
-      exchange<2, R>(u, v, x, a.sync, P, a.g, plane, number);
+      if (a.n > a.D) {
+        number++;
+        exchange<2, R>(u, v, vt, sm.exchange, a.sync, a.g, W, H, number);
+      }
     }
     const int sweeps = tile_segment(a.n, a.K, a.D, done, a.storage);
-    tile_sweeps<PRESSURE, R>(u, v, P, L, sm, a.g, c, d_t, sweeps);
+    tile_sweeps<PRESSURE, R>(u, v, vt, L, sm, link, a.sync, P.yl * 64 + P.lane, P.down, c, d_t,
+                             sweeps, message);
+    message += project_messages(sweeps);
     done += sweeps;
   }
   if (number != epoch && threadIdx.x == 0) a.sync.epochs[blockIdx.x] = number;
+  const Patch Q = patch_of(a.g, R, W, H);
   // The owned cells to the copies that ceil(n / K) passes through memory would
   // end in.
   const bool swap = ((a.n + a.K - 1) / a.K) & 1;
   void* uo = (a.cu != 0) != swap ? a.U1 : a.U0;
   void* vo = (a.cv != 0) != swap ? a.V1 : a.V0;
-  const uint32_t own = rows_in(P.y0, R, P.oy0, P.oy1);
+  const uint32_t own = rows_in(Q.y0, R, Q.oy0, Q.oy1);
   uint32_t own_u = own, top = 0u;
   if (a.extrapolate) {
-    extrapolate_patch<R>(u, v, P, W);
-    own_u &= ~rows_in(P.y0, R, H - 1 - P.gy0, H - P.gy0);
-    top = own & rows_in(P.y0, R, H - 2 - P.gy0, H - 1 - P.gy0);
+    extrapolate_patch<R>(u, v, Q, W);
+    own_u &= ~rows_in(Q.y0, R, H - 1 - Q.gy0, H - Q.gy0);
+    top = own & rows_in(Q.y0, R, H - 2 - Q.gy0, H - 1 - Q.gy0);
   }
   on_cells(a.storage, [&](auto io) {
-    patch_out<R>(io, u, uo, P, own_u, W, H, vec);
-    patch_out<R>(io, v, vo, P, own, W, H, vec);
+    patch_out<R>(io, u, uo, Q, own_u, W, H, vec);
+    patch_out<R>(io, v, vo, Q, own, W, H, vec);
     if (top)  // row H - 2 of u to row H - 1, which lies one row before it
-      patch_out<R>(io, u, static_cast<typename decltype(io)::Word*>(uo) - W, P, top, W, H, vec);
+      patch_out<R>(io, u, static_cast<typename decltype(io)::Word*>(uo) - W, Q, top, W, H, vec);
   });
-  if (PRESSURE) pressure_out<R>(sm, a.p, P, W, H, vec);
+  if (PRESSURE) pressure_out<R>(sm, a.p, Q, W, H, vec);
+  cluster_arrive();  // no CTA leaves while another may still send to it
+  cluster_wait();
 }
 
 // ---------------------------------------------------------------------------
 // Jacobi diffusion of u (apply_diffusion_at, src/fluid.cu:176-183).
 // ---------------------------------------------------------------------------
 
-// Shared memory of a diffusion tile: each strip's bottom and top row, in two
-// buffers (a sweep writes one while the other may still be read).
-struct DiffSmem {
-  float4* rows;   // [2][warps][bottom, top][2][32]
-};
-__host__ __device__ inline size_t diffuse_tile_smem(int RH, int warps, int halo, bool resident) {
-  return (size_t)2 * warps * 4 * 32 * 16 + (resident ? exchange_smem(halo, RH, 1) : 0);
+// Shared memory of a diffusion tile: the warps' inboxes and the exchange.
+__host__ __device__ inline size_t diffuse_tile_smem(int rows, int warps, int halo, bool resident) {
+  return (size_t)warps * inbox_bytes(8) + (resident ? exchange_smem(halo, rows, 1) : 0);
 }
 
 // How a strip's cells are taken: no row or column of it kept, the columns 0, 3
@@ -1068,85 +1277,91 @@ struct DiffLane {
   uint32_t cols, rows;
 };
 
-// One sweep of the strip, row by row in place: `down` holds the old row below.
-// `below` / `above`: the neighbouring strips' rows in shared memory (null: none,
-// and the row beside it is off the cone or kept).
-template <int R, Kept KEPT>
-__device__ __forceinline__ void jacobi_strip(float (&u)[R][8], const float4* below,
-                                             const float4* above, const DiffLane& L, float a,
-                                             float den, float rden, bool rcp) {
-  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-  const float4 b0 = below ? below[0] : zero, b1 = below ? below[32] : zero;
-  float down[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
+// One row of a sweep in place: `down` holds the old row below and takes the old
+// row itself, `up` is the old row above.
+template <Kept KEPT>
+__device__ __forceinline__ void jacobi_row(float (&u)[8], float (&down)[8], const float (&up)[8],
+                                           bool kept_row, const DiffLane& L, float a, float den,
+                                           float rden, bool rcp) {
+  float left = __shfl_up_sync(kAllLanes, u[7], 1);
+  const float right = __shfl_down_sync(kAllLanes, u[0], 1);
+  const uint32_t kept = KEPT == Kept::kAny && kept_row ? 0xffu : L.cols;
 #pragma unroll
-  for (int r = 0; r < R; r++) {
-    float left = __shfl_up_sync(kAllLanes, u[r][7], 1);
-    const float right = __shfl_down_sync(kAllLanes, u[r][0], 1);
-    float up[8];
-    if (r + 1 < R) {
-#pragma unroll
-      for (int q = 0; q < 8; q++) up[q] = u[r + 1 < R ? r + 1 : 0][q];
-    } else {
-      const float4 t0 = above ? above[0] : zero, t1 = above ? above[32] : zero;
-      up[0] = t0.x, up[1] = t0.y, up[2] = t0.z, up[3] = t0.w;
-      up[4] = t1.x, up[5] = t1.y, up[6] = t1.z, up[7] = t1.w;
-    }
-    const uint32_t kept = KEPT == Kept::kAny && ((L.rows >> r) & 1u) ? 0xffu : L.cols;
-#pragma unroll
-    for (int q = 0; q < 8; q++) {
-      const float old = u[r][q];
-      const float rt = q < 7 ? u[r][q < 7 ? q + 1 : 7] : right;
-      // src/fluid.cu:178-182: neighbours (i-1, j), (i+1, j), (i, j-1), (i, j+1)
-      const float x = fma_rn(a, left + rt + down[q] + up[q], old);
-      float y = KEPT != Kept::kAny || rcp ? mul_rn(x, rden) : x / den;
-      if (KEPT == Kept::kAny || (KEPT == Kept::kQuadEdges && (q == 0 || q == 3 || q == 7)))
-        y = (kept >> q) & 1u ? old : y;
-      u[r][q] = y;
-      down[q] = left = old;
-    }
+  for (int q = 0; q < 8; q++) {
+    const float old = u[q];
+    const float rt = q < 7 ? u[q < 7 ? q + 1 : 7] : right;
+    // src/fluid.cu:178-182: neighbours (i-1, j), (i+1, j), (i, j-1), (i, j+1)
+    const float x = fma_rn(a, left + rt + down[q] + up[q], old);
+    float y = KEPT != Kept::kAny || rcp ? mul_rn(x, rden) : x / den;
+    if (KEPT == Kept::kAny || (KEPT == Kept::kQuadEdges && (q == 0 || q == 3 || q == 7)))
+      y = (kept >> q) & 1u ? old : y;
+    u[q] = y;
+    down[q] = left = old;
   }
 }
 
-template <int R, Kept KEPT>
-__device__ __forceinline__ void jacobi_loop(float (&u)[R][8], const Patch& P, const DiffSmem& sm,
-                                            const RegTile& g, const DiffLane& L, float a,
-                                            float den, float rden, bool rcp, int sweeps) {
-  const int warps = g.warps;
-#pragma unroll 1
-  for (int t = 0; t < sweeps; t++) {
-    float4* mine = sm.rows + ((t & 1) * warps + P.warp) * 128 + P.lane;
-    mine[0] = make_float4(u[0][0], u[0][1], u[0][2], u[0][3]);
-    mine[32] = make_float4(u[0][4], u[0][5], u[0][6], u[0][7]);
-    mine[64] = make_float4(u[R - 1][0], u[R - 1][1], u[R - 1][2], u[R - 1][3]);
-    mine[96] = make_float4(u[R - 1][4], u[R - 1][5], u[R - 1][6], u[R - 1][7]);
-    __syncthreads();
-    const int reach = sweeps - 1 - t;  // sweeps after this one
-    if ((P.below && P.y0 + R <= g.halo - reach) || (P.above && P.y0 >= g.RH - g.halo + reach))
-      continue;
-    jacobi_strip<R, KEPT>(u, P.warp > 0 ? mine + 64 - 128 : nullptr,
-                          P.warp + 1 < warps ? mine + 128 : nullptr, L, a, den, rden, rcp);
-  }
-}
-
+// The strip's first and last row to the strips below and above, message m.
 template <int R>
-__device__ __forceinline__ void jacobi_sweeps(float (&u)[R][8], const Patch& P,
-                                              const DiffSmem& sm, const RegTile& g, int W, int H,
-                                              float a, int sweeps) {
+__device__ __forceinline__ void rows_send(const float (&u)[R][8], const Link<8>& link,
+                                          unsigned m) {
+#pragma unroll
+  for (int k = 0; k < 2; k++) {
+    post<8>(link.down, link.down_part, m, k,
+            make_float4(u[0][4 * k], u[0][4 * k + 1], u[0][4 * k + 2], u[0][4 * k + 3]));
+    post<8>(link.up, link.up_part, m, k,
+            make_float4(u[R - 1][4 * k], u[R - 1][4 * k + 1], u[R - 1][4 * k + 2],
+                        u[R - 1][4 * k + 3]));
+  }
+}
+__device__ __forceinline__ void row_receive(float (&f)[8], const Link<8>& link, int part,
+                                            unsigned m) {
+  const float4 x = read_message(link, part, m, 0), y = read_message(link, part, m, 1);
+  f[0] = x.x, f[1] = x.y, f[2] = x.z, f[3] = x.w;
+  f[4] = y.x, f[5] = y.y, f[6] = y.z, f[7] = y.w;
+}
+
+template <int R, Kept KEPT>
+__device__ __forceinline__ void jacobi_loop(float (&u)[R][8], const Link<8>& link,
+                                            const ResidentSync& sync, const DiffLane& L, float a,
+                                            float den, float rden, bool rcp, int sweeps,
+                                            unsigned m) {
+#pragma unroll 1
+  for (int t = 0; t < sweeps; t++, m++) {
+    rows_send<R>(u, link, m);
+    // The inner rows first, while the neighbours' rows come in.
+    float down[8], second[8], row[8];
+#pragma unroll
+    for (int q = 0; q < 8; q++) down[q] = u[0][q], second[q] = u[1][q];
+#pragma unroll
+    for (int r = 1; r < R - 1; r++)
+      jacobi_row<KEPT>(u[r], down, u[r + 1], (L.rows >> r) & 1u, L, a, den, rden, rcp);
+    await_message(link, m, sync);
+    row_receive(row, link, 1, m);
+    jacobi_row<KEPT>(u[R - 1], down, row, (L.rows >> (R - 1)) & 1u, L, a, den, rden, rcp);
+    row_receive(row, link, 0, m);
+    jacobi_row<KEPT>(u[0], row, second, L.rows & 1u, L, a, den, rden, rcp);
+  }
+}
+
+// `sweeps` sweeps of the region, messages m .. m + sweeps - 1. A row without a
+// strip beyond it is the grid's first or last, which is kept, or further than
+// the sweeps reach from the owned rows.
+template <int R>
+__device__ __forceinline__ void jacobi_sweeps(float (&u)[R][8], const DiffLane& L,
+                                              const Link<8>& link, const ResidentSync& sync,
+                                              float a, int sweeps, unsigned m) {
   const float den = fma_rn(4.0f, a, 1.0f);
   const float rden = __fdividef(1.0f, den);
-  const bool rcp = den < 1048576.0f;  // jacobi_divide
-  const int gx = P.gx0 + P.x0, gy = P.gy0 + P.y0;
-  DiffLane L;
-  L.cols = (gx == 0 ? 1u : 0u) | (W - 1 - gx >= 0 && W - 1 - gx < 8 ? 1u << (W - 1 - gx) : 0u);
-  L.rows = (gy == 0 ? 1u : 0u) | (H - 1 - gy >= 0 && H - 1 - gy < R ? 1u << (H - 1 - gy) : 0u);
+  // The division by den as the product with its reciprocal: the same bits for
+  // every float input (tests/cpp/reciprocal_product.cu), used below 2^20.
+  const bool rcp = den < 1048576.0f;
   const uint32_t cols = __reduce_or_sync(kAllLanes, L.cols);
-  __syncthreads();  // the rows' last readers
   if (!rcp || L.rows || (cols & ~0x89u))
-    jacobi_loop<R, Kept::kAny>(u, P, sm, g, L, a, den, rden, rcp, sweeps);
+    jacobi_loop<R, Kept::kAny>(u, link, sync, L, a, den, rden, rcp, sweeps, m);
   else if (cols)
-    jacobi_loop<R, Kept::kQuadEdges>(u, P, sm, g, L, a, den, rden, true, sweeps);
+    jacobi_loop<R, Kept::kQuadEdges>(u, link, sync, L, a, den, rden, true, sweeps, m);
   else
-    jacobi_loop<R, Kept::kNone>(u, P, sm, g, L, a, den, rden, true, sweeps);
+    jacobi_loop<R, Kept::kNone>(u, link, sync, L, a, den, rden, true, sweeps, m);
 }
 
 struct DiffuseArgs {
@@ -1167,294 +1382,62 @@ k_diffuse_tiles(const __grid_constant__ DiffuseArgs a) {
   extern __shared__ __align__(16) char tile_smem[];
   const Consts& c = a.c;
   const int W = c.W, H = c.H;
-  const Patch P = patch_of(blockIdx.x % a.g.tiles_x, blockIdx.x / a.g.tiles_x, a.g, R, W, H);
-  float4* rows = reinterpret_cast<float4*>(tile_smem);
-  const DiffSmem sm{rows};
+  const Patch P = patch_of(a.g, R, W, H);
+  const Link<8> link = open_link<8>(tile_smem, P, a.g);
+  cluster_arrive();
   const bool vec = ((W | a.g.halo) & 3) == 0;
   pdl_entry();
-  float u[R][8];
+  float u[R][8], none[8];
 #pragma unroll
   for (int r = 0; r < R; r++)
 #pragma unroll
     for (int q = 0; q < 8; q++) u[r][q] = 0.0f;
-  const float coeff = diffusion_coeff<float>(c, a.prm->dt);
   on_cells(a.storage, [&](auto io) { patch_in<R>(io, u, a.cu ? a.U1 : a.U0, P, W, H, vec); });
+  DiffLane L;
+  {
+    const int gx = P.gx0 + P.x0, gy = P.gy0 + P.y0;
+    L.cols = (gx == 0 ? 1u : 0u) | (W - 1 - gx >= 0 && W - 1 - gx < 8 ? 1u << (W - 1 - gx) : 0u);
+    L.rows = (gy == 0 ? 1u : 0u) | (H - 1 - gy >= 0 && H - 1 - gy < R ? 1u << (H - 1 - gy) : 0u);
+  }
+  const float coeff = diffusion_coeff<float>(c, a.prm->dt);
   const unsigned epoch = a.n > a.D ? ld_acquire_gpu(a.sync.epochs + blockIdx.x) : 0u;
   unsigned number = epoch;
-  Exchange x;
-  if (a.n > a.D)
-    x = exchange_plan(reinterpret_cast<char*>(rows + 2 * a.g.warps * 4 * 32), P, a.g, 1, W, H);
-  const int64_t plane = packet_plane(W, H);
+  if (a.n > a.D) exchange_plan(tile_smem + a.g.warps * inbox_bytes(8), a.g, R, 1, W, H);
+  cluster_wait();  // every inbox of the cluster is open
+  unsigned message = 0;
 #pragma unroll 1
   for (int done = 0; done < a.n;) {
     if (done > 0) {
       if (a.storage != OS_STORAGE_F32 && done % a.K == 0) round_patch<R>(u, a.storage);
-      number++;
-      exchange<1, R>(u, u, x, a.sync, P, a.g, plane, number);
+      if (a.n > a.D) {
+        number++;
+        exchange<1, R>(u, u, none, tile_smem + a.g.warps * inbox_bytes(8), a.sync, a.g, W, H,
+                       number);
+      }
     }
     const int sweeps = tile_segment(a.n, a.K, a.D, done, a.storage);
-    jacobi_sweeps<R>(u, P, sm, a.g, W, H, coeff, sweeps);
+    jacobi_sweeps<R>(u, L, link, a.sync, coeff, sweeps, message);
+    message += sweeps;
     done += sweeps;
   }
   if (number != epoch && threadIdx.x == 0) a.sync.epochs[blockIdx.x] = number;
   const bool swap = ((a.n + a.K - 1) / a.K) & 1;
   void* uo = (a.cu != 0) != swap ? a.U1 : a.U0;
+  const Patch Q = patch_of(a.g, R, W, H);
   on_cells(a.storage, [&](auto io) {
-    patch_out<R>(io, u, uo, P, rows_in(P.y0, R, P.oy0, P.oy1), W, H, vec);
+    patch_out<R>(io, u, uo, Q, rows_in(Q.y0, R, Q.oy0, Q.oy1), W, H, vec);
   });
-}
-
-// ---------------------------------------------------------------------------
-// Host: geometry and launches.
-// ---------------------------------------------------------------------------
-
-inline RegTile reg_tile(int W, int H, int halo, int R, int warps) {
-  RegTile g{};
-  g.halo = halo;
-  g.R = R, g.warps = warps;
-  g.RH = R * warps;
-  g.TX = kTileW - 2 * halo;
-  g.TY = g.RH - 2 * halo;
-  g.tiles_x = W <= kTileW ? 1 : (W - 2 * halo + g.TX - 1) / g.TX;
-  if (H <= g.RH)
-    g.tiles_y = 1;
-  else
-    g.tiles_y = g.TY >= 2 ? (H - 2 * halo + g.TY - 1) / g.TY : 0;  // 0: does not cover the grid
-  return g;
-}
-
-// Strip heights the kernels are built for.
-constexpr int kProjectRows[] = {2, 4, 6, 8, 12};
-constexpr int kDiffuseRows[] = {2, 4, 6, 8, 12};
-
-// The tile that takes the least time by a model of n sweeps, `D` between
-// exchanges or passes: issue slots on the fullest of the SM's four schedulers,
-// the region once in and out (or an exchange), in as many waves as the tiles
-// take. With `resident` every tile must have an SM of its own and be at least
-// a halo wide and high (the ring then comes from adjacent tiles). Returns the
-// modelled cycles, 0 when no tile covers the grid.
-inline double choose_tile(int W, int H, int D, bool projection, bool pressure, bool resident,
-                          int n, int sms, RegTile* out) {
-  double best = 0.0;
-  const int halo = projection ? 2 * D : D;
-  const int* heights = projection ? kProjectRows : kDiffuseRows;
-  const int count = projection ? (int)std::size(kProjectRows) : (int)std::size(kDiffuseRows);
-  for (int k = 0; k < count; k++) {
-    const int R = heights[k];
-    const int most = projection ? tile_max_warps(R) : diffuse_max_warps(R);
-    for (int warps = 1; warps <= most; warps++) {
-      RegTile g = reg_tile(W, H, halo, R, warps);
-      if (g.tiles_y < 1) continue;
-      const int64_t tiles = (int64_t)g.tiles_x * g.tiles_y;
-      if (resident && (tiles > sms || (g.tiles_y > 1 && g.TY < halo) || g.TX < halo)) continue;
-      g.smem = projection ? project_tile_smem(g.RH, warps, pressure, halo, resident)
-                          : diffuse_tile_smem(g.RH, warps, halo, resident);
-      if (g.smem + kStaticSmem > kMaxSmem) continue;
-      const int64_t waves = (tiles + sms - 1) / sms;
-      // Cycles of a sweep: the strips on a scheduler, and a barrier and the
-      // faces' way between strips for each half-sweep.
-      const double strip = projection ? (pressure ? 116.0 : 78.0) * R + 40.0 : 46.0 * R + 60.0;
-      const double sweep = ((warps + 3) / 4) * strip + (projection ? 350.0 : 150.0);
-      const double trip = resident ? 4000.0 + 40.0 * R
-                                   : 5000.0 + g.RH * (projection ? 50.0 : 25.0);
-      const double rounds = (n + D - 1) / D;
-      const double cost = (double)waves * (n * sweep + rounds * trip);
-      if (best == 0.0 || cost < best) {
-        best = cost;
-        *out = g;
-      }
-    }
-  }
-  return best;
+  cluster_arrive();  // no CTA leaves while another may still send to it
+  cluster_wait();
 }
 
 using ProjectKernel = void (*)(const ProjectArgs);
 using DiffuseKernel = void (*)(const DiffuseArgs);
 
-template <bool PRESSURE>
-inline ProjectKernel project_kernel(int R) {
-  switch (R) {
-    case 2: return k_project_tiles<2, PRESSURE>;
-    case 4: return k_project_tiles<4, PRESSURE>;
-    case 6: return k_project_tiles<6, PRESSURE>;
-    case 8: return k_project_tiles<8, PRESSURE>;
-    default: return k_project_tiles<12, PRESSURE>;
-  }
-}
-inline DiffuseKernel diffuse_kernel(int R) {
-  switch (R) {
-    case 2: return k_diffuse_tiles<2>;
-    case 4: return k_diffuse_tiles<4>;
-    case 6: return k_diffuse_tiles<6>;
-    case 8: return k_diffuse_tiles<8>;
-    default: return k_diffuse_tiles<12>;
-  }
-}
-
-// A launch of `tiles` CTAs: cooperative when its CTAs wait on one another,
-// else with programmatic stream serialisation where the handle uses it.
-template <class Args>
-inline cudaError_t launch_tiles(void (*kernel)(const Args), const Args& a, const RegTile& g,
-                                bool cooperative, bool pdl, cudaStream_t st) {
-  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)g.smem);
-  if (e != cudaSuccess) return e;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(g.tiles_x * g.tiles_y);
-  cfg.blockDim = dim3(32 * g.warps);
-  cfg.dynamicSmemBytes = g.smem;
-  cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  if (cooperative) {
-    attr[0].id = cudaLaunchAttributeCooperative;
-    attr[0].val.cooperative = 1;
-  } else {
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-  }
-  cfg.attrs = attr;
-  cfg.numAttrs = (cooperative || pdl) ? 1 : 0;
-  return cudaLaunchKernelEx(&cfg, kernel, a);
-}
-
-// The resident forms' tiles, all of one launch resident together, and the
-// sweeps between their exchanges. (block_k is not their depth: it says which
-// copy the fields end in and, with 16-bit storage, how often they are rounded.)
-inline int resident_tile(const os_handle* h, bool projection, RegTile* g) {
-  const bool pressure = h->cfg.enable_pressure != 0;
-  const int K = h->block_k;
-  if (K < 2 || K % (projection ? 2 : 4)) return 0;
-  int depth = 0;
-  double best = 0.0;
-  for (int D : {2, 4, 6, 8, 12, 16}) {  // halos in multiples of 4 cells
-    if (!projection && D % 4) continue;
-    RegTile t;
-    const double cost = choose_tile(h->W, h->H, D, projection, pressure, true, std::max(h->c.n, 1),
-                                    sm_count(h->cfg.device), &t);
-    if (cost > 0.0 && (depth == 0 || cost < best)) {
-      best = cost;
-      depth = D;
-      *g = t;
-    }
-  }
-  return depth;
-}
-
-// The projection phase: one launch for all its passes (resident), or one per
-// pass of block_k sweeps. `cur_u` / `cur_v` say which copy holds the live
-// field (0: u, v; 1: ub, vb) and advance by the passes. `extrapolate`: the
-// last pass applies the extrapolation that follows in a step. Returns the
-// launches, or -1.
-inline int enqueue_tiled_projection(os_handle* h, cudaStream_t st, int* cur_u, int* cur_v,
-                                    bool zero_first, bool extrapolate) {
-  const int K = h->block_k, n = h->c.n;
-  const bool pressure = h->cfg.enable_pressure != 0;
-  ProjectArgs a{};
-  a.U0 = h->u, a.U1 = h->ub, a.V0 = h->v, a.V1 = h->vb;
-  a.storage = h->storage;
-  a.p = h->p;
-  a.flags = h->flags;
-  a.c = h->c;
-  a.prm = h->d_params;
-  a.K = K;
-  a.sync = ResidentSync{h->rflags, h->rpackets, h->rerr, h->d_host_rerr};
-  const int passes = (n + K - 1) / K;
-  int launches = 0;
-  if (h->resident) {
-    if (!(a.D = resident_tile(h, true, &a.g))) return -1;
-    a.n = n;
-    a.cu = *cur_u, a.cv = *cur_v;
-    a.zero_pressure = zero_first;
-    a.extrapolate = extrapolate;
-    if (passes > 0 &&
-        launch_tiles(pressure ? project_kernel<true>(a.g.R) : project_kernel<false>(a.g.R), a, a.g,
-                     n > a.D, h->pdl, st) != cudaSuccess)
-      return -1;
-    launches = passes > 0;
-  } else {
-    a.D = K;
-    if (projection_smem(2 + 4 * K, pressure) + kStaticSmem > kMaxSmem ||
-        choose_tile(h->W, h->H, K, true, pressure, false, n, sm_count(h->cfg.device), &a.g) == 0.0)
-      return -1;
-    for (int p = 0; p < passes; p++, launches++) {
-      a.n = std::min(K, n - p * K);
-      a.cu = (*cur_u + p) & 1, a.cv = (*cur_v + p) & 1;
-      a.zero_pressure = zero_first && p == 0;
-      a.extrapolate = extrapolate && p == passes - 1;
-      if (launch_tiles(pressure ? project_kernel<true>(a.g.R) : project_kernel<false>(a.g.R), a,
-                       a.g, false, h->pdl, st) != cudaSuccess)
-        return -1;
-    }
-  }
-  *cur_u = (*cur_u + passes) & 1;
-  *cur_v = (*cur_v + passes) & 1;
-  return launches;
-}
-
-// The diffusion phase in the same way, block_k sweeps per pass when resident,
-// else diffusion_depth.
-inline int enqueue_tiled_diffusion(os_handle* h, cudaStream_t st, int* cur_u) {
-  const int K = h->resident_diff ? h->block_k : diffusion_depth(h), n = h->c.n;
-  DiffuseArgs a{};
-  a.U0 = h->u, a.U1 = h->ub;
-  a.storage = h->storage;
-  a.c = h->c;
-  a.prm = h->d_params;
-  a.K = K;
-  a.sync = ResidentSync{h->dflags, h->dpackets, h->rerr, h->d_host_rerr};
-  const int passes = (n + K - 1) / K;
-  int launches = 0;
-  if (h->resident_diff) {
-    if (!(a.D = resident_tile(h, false, &a.g))) return -1;
-    a.n = n;
-    a.cu = *cur_u;
-    if (passes > 0 && launch_tiles(diffuse_kernel(a.g.R), a, a.g, n > a.D, h->pdl, st) !=
-                          cudaSuccess)
-      return -1;
-    launches = passes > 0;
-  } else {
-    a.D = K;
-    if (choose_tile(h->W, h->H, K, false, false, false, n, sm_count(h->cfg.device), &a.g) == 0.0)
-      return -1;
-    for (int p = 0; p < passes; p++, launches++) {
-      a.n = std::min(K, n - p * K);
-      a.cu = (*cur_u + p) & 1;
-      if (launch_tiles(diffuse_kernel(a.g.R), a, a.g, false, h->pdl, st) != cudaSuccess) return -1;
-    }
-  }
-  *cur_u = (*cur_u + passes) & 1;
-  return launches;
-}
-
-// Device bytes of a resident phase's epochs, and of its packets.
-inline size_t resident_epoch_bytes(int sms) { return (size_t)sms * sizeof(unsigned); }
-inline size_t resident_packet_bytes(int W, int H, int per_quad) {
-  return (size_t)2 * packet_plane(W, H) * per_quad * sizeof(uint4);
-}
-
-// Whether the resident forms can be launched cooperatively on this device.
-template <class Args>
-inline bool tiles_launchable(void (*kernel)(const Args), const RegTile& g, int sms) {
-  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g.smem) !=
-      cudaSuccess)
-    return false;
-  int per_sm = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, 32 * g.warps, g.smem) !=
-      cudaSuccess)
-    return false;
-  return per_sm >= 1 && g.tiles_x * g.tiles_y <= per_sm * sms;
-}
-
-// Failure-detection self-test: a warp waits for a packet that nothing sends, so
-// the wait must give up and report.
-__global__ void k_wait_selftest(ResidentSync sync) {
-  float a = 0.0f, b = 0.0f, c = 0.0f;
-  bool again = true;
-  for (int it = 0; again; it++) {
-    const bool ok = packet_in(threadIdx.x == 0, sync.packets, a, b, c, 1u);
-    again = !__all_sync(kAllLanes, ok) && poll_again(it, sync);
-    again = __any_sync(kAllLanes, again);
-  }
-}
+// The kernels of one strip height, each instantiated in a translation unit of
+// its own (os_tile_project.cu, os_tile_diffuse.cu).
+template <int R> ProjectKernel project_kernel(bool pressure);
+template <int R> DiffuseKernel diffuse_kernel();
 
 }  // namespace osg
+

@@ -1,0 +1,9 @@
+// os_tile_diffuse.cu — the diffusion kernel of one strip height, OS_TILE_ROWS.
+#include "os_tile.cuh"
+
+namespace osg {
+template <>
+DiffuseKernel diffuse_kernel<OS_TILE_ROWS>() {
+  return k_diffuse_tiles<OS_TILE_ROWS>;
+}
+}  // namespace osg

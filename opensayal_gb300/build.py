@@ -31,7 +31,7 @@ NVCC_FLAGS = [
 # Translation units, compiled side by side: (source, defines). The tile kernels
 # take one unit per strip height.
 TILE_ROWS = {"project": (10, 8, 6, 4, 2), "diffuse": (12, 8, 6, 4, 2)}
-UNITS = [("os_fluid.cu", ())]
+UNITS = [("os_fluid.cu", ()), ("os_tile_batch.cu", ())]
 UNITS += [(f"os_tile_{phase}.cu", (f"OS_TILE_ROWS={rows}",))
           for phase, heights in TILE_ROWS.items() for rows in heights]
 

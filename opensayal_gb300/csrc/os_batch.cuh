@@ -27,48 +27,9 @@
 // between steps every member's state is in its public arrays.
 #pragma once
 
+#include "os_batch_plan.cuh"
+
 namespace osg {
-
-constexpr int kBatchMaxPasses = 128;  // blocked passes per phase (n <= 128 * K)
-
-struct ScenarioDesc {
-  Consts c;
-  int storage;       // OS_STORAGE_F32, OS_STORAGE_F16 or OS_STORAGE_BF16
-  int smoke_period;
-  int smoke_on;      // enable_smoke && wind_tunnel.smoke != 0
-  int diff_passes;   // blocked diffusion passes per step (0 when viscosity == 0)
-  int proj_passes;   // blocked projection passes per step
-  int diff_tiles_x;  // tile columns under the diffusion geometry
-  int proj_tiles_x;  // tile columns under the projection geometry
-  const StepParams* prm;
-  void *u, *v, *ub, *vb, *s, *sb;
-  const uint8_t* flags;
-  const uint16_t* nbr;  // fluid neighbourhoods (samplers)
-};
-
-struct TileRef {
-  int slot;
-  int16_t tx, ty;
-};
-
-// Head of the device plan; the arrays follow at the given byte offsets.
-struct PlanHeader {
-  int members;
-  int admits;     // (slot, steps) pairs in the admit list
-  int64_t cells;  // cells over all members
-  int off_desc;                       // ScenarioDesc[slots]
-  int off_slot;                       // int[members]
-  int off_cell_cum;                   // int64_t[members]: cells before member k
-  int off_diff_tiles, off_proj_tiles; // TileRef[tiles of pass 0]
-  int off_admit;                      // int2[admits]
-  int diff_items[kBatchMaxPasses];    // tiles in diffusion pass p
-  int proj_items[kBatchMaxPasses];    // tiles in projection pass p
-};
-
-template <class T>
-__device__ __forceinline__ const T* plan_array(const PlanHeader* P, int off) {
-  return reinterpret_cast<const T*>(reinterpret_cast<const char*>(P) + off);
-}
 
 // Member whose cell range [cum[k], cum[k+1]) holds cell `it` (cum[0] = 0).
 __device__ __forceinline__ int member_of(const int64_t* __restrict__ cum, int n, int64_t it) {
@@ -89,13 +50,6 @@ __device__ __forceinline__ void with_storage(int storage, Fn&& fn) {
     case OS_STORAGE_BF16: fn(static_cast<__nv_bfloat16*>(nullptr)); break;
     default: fn(static_cast<float*>(nullptr)); break;
   }
-}
-
-__device__ __forceinline__ void stage_desc(const ScenarioDesc* src, ScenarioDesc* dst) {
-  static_assert(sizeof(ScenarioDesc) % 4 == 0, "descriptor is copied in words");
-  constexpr int kWords = sizeof(ScenarioDesc) / 4;
-  if (threadIdx.x < kWords)
-    reinterpret_cast<uint32_t*>(dst)[threadIdx.x] = reinterpret_cast<const uint32_t*>(src)[threadIdx.x];
 }
 
 template <class S>
@@ -138,6 +92,7 @@ __device__ __forceinline__ void for_cells(const PlanHeader* __restrict__ P,
 }
 
 __global__ void k_batch_forces(const PlanHeader* __restrict__ P, const int* __restrict__ remaining) {
+  pdl_entry();
   for_cells(P, remaining, [&](const ScenarioDesc& d, int j, int i0, int i1) {
     with_storage(d.storage, [&](auto tag) {
       using S = std::remove_pointer_t<decltype(tag)>;
@@ -151,75 +106,16 @@ __global__ void k_batch_forces(const PlanHeader* __restrict__ P, const int* __re
   });
 }
 
-__global__ void __launch_bounds__(kBlockThreads, 1)
-k_batch_diffuse(const PlanHeader* __restrict__ P, const int* __restrict__ remaining, int pass,
-                int K, int halo, int TX, int TY) {
-  extern __shared__ __align__(16) float smem[];
-  const int n_items = P->diff_items[pass];
-  const TileRef* tiles = plan_array<TileRef>(P, P->off_diff_tiles);
-  const ScenarioDesc* T = plan_array<ScenarioDesc>(P, P->off_desc);
-  for (int it = blockIdx.x; it < n_items; it += gridDim.x) {
-    const TileRef t = tiles[it];
-    const int slot = t.slot;
-    if (remaining[slot] == 0) continue;  // uniform over the block
-    const ScenarioDesc& d = T[slot];
-    const int tx = t.tx, ty = t.ty;
-    const int sweeps = min(K, d.c.n - pass * K);
-    const int in = pass & 1;
-    with_storage(d.storage, [&](auto tag) {
-      using S = std::remove_pointer_t<decltype(tag)>;
-      diffuse_tile<S>(smem, tx, ty, copy_of<S>(d.u, d.ub, in), copy_of<S>(d.u, d.ub, 1 - in),
-                      d.c, d.prm, sweeps, halo, TX, TY);
-    });
-    __syncthreads();  // the next item restages shared memory
-  }
-}
-
-__global__ void __launch_bounds__(kBlockThreads, 1)
-k_batch_project(const PlanHeader* __restrict__ P, const int* __restrict__ remaining, int pass,
-                int K, int halo, int TX, int TY) {
-  extern __shared__ __align__(16) float smem[];
-  const int n_items = P->proj_items[pass];
-  const TileRef* tiles = plan_array<TileRef>(P, P->off_proj_tiles);
-  const ScenarioDesc* T = plan_array<ScenarioDesc>(P, P->off_desc);
-  // The descriptor is staged in shared memory: its constants are then read
-  // from there inside the sweeps instead of being held in registers.
-  __shared__ ScenarioDesc sd;
-  for (int it = blockIdx.x; it < n_items; it += gridDim.x) {
-    const TileRef t = tiles[it];
-    const int slot = t.slot;
-    if (remaining[slot] == 0) continue;
-    stage_desc(T + slot, &sd);
-    __syncthreads();
-    const ScenarioDesc& d = sd;
-    const int tx = t.tx, ty = t.ty;
-    const int sweeps = min(K, d.c.n - pass * K);
-    const int iu = (d.diff_passes + pass) & 1, iv = pass & 1;
-    // project_tile in three parts, so that the sweeps are instantiated once.
-    with_storage(d.storage, [&](auto tag) {
-      using S = std::remove_pointer_t<decltype(tag)>;
-      proj_stage_in<false, S>(smem, tx, ty, copy_of<S>(d.u, d.ub, iu), copy_of<S>(d.v, d.vb, iv),
-                              nullptr, d.flags, d.c, halo, TX, TY, 0);
-    });
-    __syncthreads();
-    proj_sweeps_fast<false>(smem, d.c, d.prm, sweeps, halo, TY);
-    with_storage(d.storage, [&](auto tag) {
-      using S = std::remove_pointer_t<decltype(tag)>;
-      proj_stage_out<false, S>(smem, tx, ty, copy_of<S>(d.u, d.ub, 1 - iu),
-                               copy_of<S>(d.v, d.vb, 1 - iv), nullptr, d.c, halo, TX, TY);
-    });
-    __syncthreads();
-  }
-}
-
 __global__ void k_batch_extrapolate(const PlanHeader* __restrict__ P,
                                     const int* __restrict__ remaining) {
+  pdl_entry();
   const int* slot_of = plan_array<int>(P, P->off_slot);
   const ScenarioDesc* T = plan_array<ScenarioDesc>(P, P->off_desc);
   for (int k = blockIdx.x; k < P->members; k += gridDim.x) {
     const int slot = slot_of[k];
     if (remaining[slot] == 0) continue;
     const ScenarioDesc& d = T[slot];
+    if (d.proj_passes > 0) continue;  // its last pass has done it
     const int iu = (d.diff_passes + d.proj_passes) & 1, iv = d.proj_passes & 1;
     with_storage(d.storage, [&](auto tag) {
       using S = std::remove_pointer_t<decltype(tag)>;
@@ -231,6 +127,7 @@ __global__ void k_batch_extrapolate(const PlanHeader* __restrict__ P,
 
 __global__ void k_batch_advect_velocity(const PlanHeader* __restrict__ P,
                                         const int* __restrict__ remaining) {
+  pdl_entry();
   for_cells(P, remaining, [&](const ScenarioDesc& d, int j, int i0, int i1) {
     const int iu = (d.diff_passes + d.proj_passes) & 1, iv = d.proj_passes & 1;
     with_storage(d.storage, [&](auto tag) {
@@ -247,6 +144,7 @@ __global__ void k_batch_advect_velocity(const PlanHeader* __restrict__ P,
 // sits in a buffer); scenarios without smoke only copy back.
 __global__ void k_batch_advect_smoke(const PlanHeader* __restrict__ P,
                                      const int* __restrict__ remaining) {
+  pdl_entry();
   for_cells(P, remaining, [&](const ScenarioDesc& d, int j, int i0, int i1) {
     const int iu = 1 - ((d.diff_passes + d.proj_passes) & 1), iv = 1 - (d.proj_passes & 1);
     with_storage(d.storage, [&](auto tag) {
@@ -271,6 +169,7 @@ __global__ void k_batch_advect_smoke(const PlanHeader* __restrict__ P,
 
 __global__ void k_batch_finish_smoke(const PlanHeader* __restrict__ P,
                                      const int* __restrict__ remaining) {
+  pdl_entry();
   for_cells(P, remaining, [&](const ScenarioDesc& d, int j, int i0, int i1) {
     if (!d.smoke_on) return;
     with_storage(d.storage, [&](auto tag) {
@@ -284,6 +183,7 @@ __global__ void k_batch_finish_smoke(const PlanHeader* __restrict__ P,
 
 // End of a step: every live member has one step fewer to go.
 __global__ void k_batch_tick(const PlanHeader* __restrict__ P, int* __restrict__ remaining) {
+  pdl_entry();
   const int* slot_of = plan_array<int>(P, P->off_slot);
   for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < P->members; k += gridDim.x * blockDim.x) {
     const int slot = slot_of[k];

@@ -32,11 +32,15 @@ struct os_batch {
   };
   int device = 0;
   int K = 8;
-  int ty_div = 1;  // tile height: the largest that fits, divided by this
+  int cluster = 4;  // CTAs per cluster of the tile kernels: the tiles' height
   int sms = 152;
   cudaStream_t stream = nullptr;
   Arena* arena = nullptr;  // null: members allocate with cudaMalloc
-  TileGeom gd{}, gp{};
+  RegTile gd{}, gp{};
+  int gd_clusters = 0, gp_clusters = 0;  // clusters resident together
+  // Error word of the tile kernels' bounded waits: device, and mapped host.
+  int* d_err = nullptr;
+  int* h_err = nullptr;
   std::map<int64_t, Member> members;  // by id
   int64_t next_id = 0;
   std::vector<int> free_slots;
@@ -70,26 +74,35 @@ struct os_batch {
 
 namespace {
 
-// Largest even tile height whose region fits shared memory, divided by
-// `ty_div` (rounded to even): shorter tiles balance better across the SMs at
-// the price of more halo rows.
-TileGeom batch_geom(int halo, bool projection, int ty_div = 1) {
-  TileGeom g{};
-  g.halo = halo;
-  g.TX = kRegionW - 2 * halo;
-  int TY = 2;
-  while (true) {
-    const int next = TY + 2;
-    const size_t sm = projection ? projection_smem(next + 2 * halo, false)
-                                 : diffusion_smem(next + 2 * halo);
-    if (sm + kStaticSmem > kMaxSmem) break;  // room for the kernels' static shared memory
-    TY = next;
-  }
-  TY = std::max(2, (TY / std::max(1, ty_div)) & ~1);
-  g.TY = TY;
-  g.RH = TY + 2 * halo;
-  g.smem = projection ? projection_smem(g.RH, false) : diffusion_smem(g.RH);
+// The tiles of a phase: clusters of `cluster` CTAs.
+RegTile batch_geom(int K, bool projection, int cluster) {
+  RegTile g = reg_tile(1 << 30, 1 << 30, projection ? 2 * K : K, kBatchRows, kBatchWarps, cluster);
+  const int rows = kBatchRows * kBatchWarps;
+  g.smem = projection ? project_tile_smem(rows, kBatchWarps, false, g.halo, false)
+                      : diffuse_tile_smem(rows, kBatchWarps, g.halo, false);
   return g;
+}
+
+int batch_tiles(int size, int pitch, int halo, int region) {
+  return size <= region ? 1 : (size - 2 * halo + pitch - 1) / pitch;
+}
+
+// Clusters of the kernel that are resident together (several CTAs to an SM).
+int batch_clusters(BatchTileKernel kernel, const RegTile& g, cudaLaunchAttribute* attr) {
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g.smem) !=
+      cudaSuccess)
+    return 0;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(g.cluster * 1024);
+  cfg.blockDim = dim3(32 * g.warps);
+  cfg.dynamicSmemBytes = g.smem;
+  attr->id = cudaLaunchAttributeClusterDimension;
+  attr->val.clusterDim.x = g.cluster;
+  attr->val.clusterDim.y = attr->val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  int n = 0;
+  return cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) == cudaSuccess ? n : 0;
 }
 
 size_t align16(size_t x) { return (x + 15) & ~size_t(15); }
@@ -112,6 +125,8 @@ void free_batch(os_batch* b) {
   }
   for (auto& f : b->inflight) cudaEventDestroy(f.second);
   for (cudaEvent_t e : b->event_pool) cudaEventDestroy(e);
+  if (b->d_err) cudaFree(b->d_err);
+  if (b->h_err) cudaFreeHost(b->h_err);
   if (b->stream) cudaStreamDestroy(b->stream);
   delete b->arena;
   delete b;
@@ -135,20 +150,33 @@ int build_batch_graph(os_batch* b, int dpasses, int ppasses) {
   int* R = b->d_remaining;
   const int row_grid = b->sms * 16;
   CUDA_OR_RETURN(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-  k_batch_forces<<<row_grid, 128, 0, st>>>(P, R);
-  kernels++;
-  for (int p = 0; p < dpasses; p++, kernels++)
-    k_batch_diffuse<<<b->sms, kBlockThreads, b->gd.smem, st>>>(P, R, p, b->K, b->gd.halo,
-                                                                b->gd.TX, b->gd.TY);
-  for (int p = 0; p < ppasses; p++, kernels++)
-    k_batch_project<<<b->sms, kBlockThreads, b->gp.smem, st>>>(P, R, p, b->K, b->gp.halo,
-                                                                b->gp.TX, b->gp.TY);
-  k_batch_extrapolate<<<b->sms * 4, 1024, 0, st>>>(P, R);
-  k_batch_advect_velocity<<<row_grid, 128, 0, st>>>(P, R);
-  k_batch_advect_smoke<<<row_grid, 128, 0, st>>>(P, R);
-  k_batch_finish_smoke<<<row_grid, 128, 0, st>>>(P, R);
-  k_batch_tick<<<1, 256, 0, st>>>(P, R);
-  kernels += 5;
+  auto tile_pass = [&](BatchTileKernel kernel, const RegTile& g, int clusters, int pass) {
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = g.cluster;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(clusters * g.cluster);
+    cfg.blockDim = dim3(32 * g.warps);
+    cfg.dynamicSmemBytes = g.smem;
+    cfg.stream = st;
+    cfg.attrs = attr;
+    cfg.numAttrs = 2;
+    cudaLaunchKernelEx(&cfg, kernel, P, (const int*)R, pass, b->K, g,
+                       ResidentSync{nullptr, nullptr, b->d_err, b->h_err});
+    kernels++;
+  };
+  launch_pdl(true, k_batch_forces, row_grid, 128, 0, st, P, (const int*)R);
+  for (int p = 0; p < dpasses; p++) tile_pass(batch_diffuse_kernel(), b->gd, b->gd_clusters, p);
+  for (int p = 0; p < ppasses; p++) tile_pass(batch_project_kernel(), b->gp, b->gp_clusters, p);
+  launch_pdl(true, k_batch_extrapolate, b->sms * 4, 1024, 0, st, P, (const int*)R);
+  launch_pdl(true, k_batch_advect_velocity, row_grid, 128, 0, st, P, (const int*)R);
+  launch_pdl(true, k_batch_advect_smoke, row_grid, 128, 0, st, P, (const int*)R);
+  launch_pdl(true, k_batch_finish_smoke, row_grid, 128, 0, st, P, (const int*)R);
+  launch_pdl(true, k_batch_tick, 1, 256, 0, st, P, R);
+  kernels += 6;
   const cudaError_t le = cudaGetLastError();
   cudaGraph_t g = nullptr;
   const cudaError_t ce = cudaStreamEndCapture(st, &g);
@@ -174,8 +202,10 @@ ScenarioDesc describe(const os_batch* b, const os_handle* h) {
   d.smoke_on = h->cfg.enable_smoke && h->cfg.tunnel_smoke != 0.0f;
   d.proj_passes = (h->c.n + b->K - 1) / b->K;
   d.diff_passes = h->cfg.viscosity != 0.0f ? d.proj_passes : 0;
-  d.diff_tiles_x = (h->W + b->gd.TX - 1) / b->gd.TX;
-  d.proj_tiles_x = (h->W + b->gp.TX - 1) / b->gp.TX;
+  d.diff_tiles_x = batch_tiles(h->W, b->gd.TX, b->gd.halo, kTileW);
+  d.diff_tiles_y = batch_tiles(h->H, b->gd.TY, b->gd.halo, b->gd.RH);
+  d.proj_tiles_x = batch_tiles(h->W, b->gp.TX, b->gp.halo, kTileW);
+  d.proj_tiles_y = batch_tiles(h->H, b->gp.TY, b->gp.halo, b->gp.RH);
   d.prm = h->d_params;
   d.u = h->u;
   d.v = h->v;
@@ -212,9 +242,8 @@ int write_plan(os_batch* b, cudaStream_t st) {
     e.id = kv.first;
     e.d = describe(b, m.h);
     e.slot = m.slot;
-    const int ty_d = (m.h->H + b->gd.TY - 1) / b->gd.TY, ty_p = (m.h->H + b->gp.TY - 1) / b->gp.TY;
-    e.dtiles = e.d.diff_tiles_x * ty_d;
-    e.ptiles = e.d.proj_tiles_x * ty_p;
+    e.dtiles = e.d.diff_tiles_x * e.d.diff_tiles_y;
+    e.ptiles = e.d.proj_tiles_x * e.d.proj_tiles_y;
     live.push_back(e);
     max_slot = std::max(max_slot, m.slot);
     dpasses = std::max(dpasses, e.d.diff_passes);
@@ -327,14 +356,13 @@ int write_plan(os_batch* b, cudaStream_t st) {
     for (int k = 0; k < members; k++) idx[k] = k;
     auto passes = [&](int k) { return diffusion ? live[k].d.diff_passes : live[k].d.proj_passes; };
     std::stable_sort(idx.begin(), idx.end(), [&](int a, int c) { return passes(a) > passes(c); });
-    const TileGeom& g = diffusion ? b->gd : b->gp;
     std::vector<int64_t> cum(members + 1);
     int64_t n = 0;
     for (int k = 0; k < members; k++) {
       const Entry& e = live[idx[k]];
       cum[k] = n;
       const int tiles_x = diffusion ? e.d.diff_tiles_x : e.d.proj_tiles_x;
-      const int tiles_y = (e.d.c.H + g.TY - 1) / g.TY;
+      const int tiles_y = diffusion ? e.d.diff_tiles_y : e.d.proj_tiles_y;
       for (int ty = 0; ty < tiles_y; ty++)
         for (int tx = 0; tx < tiles_x; tx++)
           out[n++] = TileRef{e.slot, (int16_t)tx, (int16_t)ty};
@@ -377,6 +405,13 @@ int batch_progress(os_batch* b) {
     const cudaError_t q = cudaEventQuery(b->inflight.front().second);
     if (q == cudaErrorNotReady) break;
     if (q != cudaSuccess) return set_err(OS_ERR_CUDA, "batch step: %s", cudaGetErrorString(q));
+    if (*(volatile int*)b->h_err) {
+      *(volatile int*)b->h_err = 0;
+      cudaMemsetAsync(b->d_err, 0, sizeof(int), b->stream);
+      return set_err(OS_ERR_TIMEOUT,
+                     "batch step: a wait between the strips of a tile gave up; the fields are "
+                     "undefined");
+    }
     b->steps_done = std::max(b->steps_done, b->inflight.front().first);
     b->event_pool.push_back(b->inflight.front().second);
     b->inflight.pop_front();
@@ -397,23 +432,31 @@ int batch_progress(os_batch* b) {
   return OS_OK;
 }
 
+// Tiles of `cluster` CTAs at depth K, as many as fit the GPU at once.
+int size_tiles(os_batch* b, int K, int cluster) {
+  b->K = K;
+  b->cluster = cluster;
+  b->gd = batch_geom(K, false, cluster);
+  b->gp = batch_geom(K, true, cluster);
+  cudaLaunchAttribute attr;
+  b->gd_clusters = batch_clusters(batch_diffuse_kernel(), b->gd, &attr);
+  b->gp_clusters = batch_clusters(batch_project_kernel(), b->gp, &attr);
+  if (b->gd_clusters < 1 || b->gp_clusters < 1)
+    return set_err(OS_ERR_CUDA, "batch set-up: %s", cudaGetErrorString(cudaGetLastError()));
+  return OS_OK;
+}
+
 // Blocking depth and tile height for the whole batch; the plan and graph are
 // rewritten at the next step.
-int set_geometry(os_batch* b, int K, int ty_div) {
+int set_geometry(os_batch* b, int K, int cluster) {
   if (b->graph) {
     CUDA_OR_RETURN(cudaStreamSynchronize(b->stream));
     cudaGraphExecDestroy(b->graph);
     b->graph = nullptr;
   }
   b->graph_dpasses = b->graph_ppasses = -1;
-  b->K = K;
-  b->ty_div = ty_div;
-  b->gd = batch_geom(K, false, ty_div);
-  b->gp = batch_geom(2 * K, true, ty_div);
-  cudaFuncSetAttribute(k_batch_diffuse, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)b->gd.smem);
-  cudaFuncSetAttribute(k_batch_project, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)b->gp.smem);
+  const int rc = size_tiles(b, K, cluster);
+  if (rc) return rc;
   for (auto& kv : b->members) {
     kv.second.h->block_k = K;
     kv.second.h->cfg.projection_block = K;
@@ -431,22 +474,22 @@ int write_plan(os_batch* b, cudaStream_t st);
 // os_create leaves them.
 int tune_batch(os_batch* b) {
   struct Cand {
-    int K, div;
+    int K, cluster;
   };
   std::vector<Cand> cands;
   for (int K : {4, 6, 8, 12})
-    for (int div : {1, 2}) cands.push_back({K, div});
+    for (int cluster : {4, 8}) cands.push_back({K, cluster});
   int max_n = 0;
   for (auto& kv : b->members) max_n = std::max(max_n, kv.second.h->c.n);
   cudaEvent_t a = nullptr, z = nullptr;
   CUDA_OR_RETURN(cudaEventCreate(&a));
   CUDA_OR_RETURN(cudaEventCreate(&z));
-  Cand best{b->K, b->ty_div};
+  Cand best{b->K, b->cluster};
   float best_ms = 0.0f;
   int rc = OS_OK;
   for (const Cand& cd : cands) {
     if ((max_n + cd.K - 1) / cd.K > kBatchMaxPasses) continue;
-    if ((rc = set_geometry(b, cd.K, cd.div)) || (rc = write_plan(b, b->stream))) break;
+    if ((rc = set_geometry(b, cd.K, cd.cluster)) || (rc = write_plan(b, b->stream))) break;
     CUDA_OR_RETURN(cudaGraphLaunch(b->graph, b->stream));  // warm-up
     cudaEventRecord(a, b->stream);
     for (int t = 0; t < 3; t++) CUDA_OR_RETURN(cudaGraphLaunch(b->graph, b->stream));
@@ -463,7 +506,7 @@ int tune_batch(os_batch* b) {
   cudaEventDestroy(a);
   cudaEventDestroy(z);
   if (rc) return rc;
-  if ((rc = set_geometry(b, best.K, best.div)) || (rc = write_plan(b, b->stream))) return rc;
+  if ((rc = set_geometry(b, best.K, best.cluster)) || (rc = write_plan(b, b->stream))) return rc;
   for (auto& kv : b->members) {
     os_handle* h = kv.second.h;
     const size_t fb = h->N * h->esize;
@@ -499,12 +542,12 @@ int new_batch(int device, int block_k, uint64_t budget, os_batch** out) {
       return fail(set_err(OS_ERR_NOMEM, "device budget of %llu bytes could not be reserved",
                           (unsigned long long)budget));
   }
-  b->gd = batch_geom(b->K, false);
-  b->gp = batch_geom(2 * b->K, true);
-  cudaFuncSetAttribute(k_batch_diffuse, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)b->gd.smem);
-  cudaFuncSetAttribute(k_batch_project, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)b->gp.smem);
+  if ((e = cudaMalloc(&b->d_err, sizeof(int))) != cudaSuccess ||
+      (e = cudaHostAlloc(&b->h_err, sizeof(int), cudaHostAllocMapped)) != cudaSuccess)
+    return fail(set_err(OS_ERR_NOMEM, "batch set-up: %s", cudaGetErrorString(e)));
+  *b->h_err = 0;
+  cudaMemset(b->d_err, 0, sizeof(int));
+  if (const int rc = size_tiles(b, b->K, b->cluster)) return fail(rc);
   if ((e = cudaGetLastError()) != cudaSuccess)
     return fail(set_err(OS_ERR_CUDA, "batch set-up: %s", cudaGetErrorString(e)));
   *out = b;

@@ -163,32 +163,45 @@ struct Patch {
   bool left, right, below, above;  // the tile has a neighbour on that side
   int ox0, ox1, oy0, oy1;          // owned columns and rows, in the region
   bool down, up;                   // the tile has a strip below / above this one
+  bool idle;                       // every row of the strip is off the grid
+};
+
+// A tile of a grid.
+struct TilePlace {
+  int tx, ty, tiles_x, tiles_y;
 };
 
 // Worked out anew wherever it is used outside the sweeps (the block and thread
 // numbers pass through an empty asm, so that the compiler does not keep one
 // copy alive): held across the sweep loops it costs registers that their faces
 // need.
-__device__ __forceinline__ Patch patch_of(const RegTile& g, int R, int W, int H) {
+__device__ __forceinline__ Patch patch_at(const TilePlace& t, const RegTile& g, int R, int W,
+                                          int H) {
   Patch P;
   unsigned block = blockIdx.x, thread = threadIdx.x;
   asm volatile("" : "+r"(block), "+r"(thread));
-  const int tile = block / g.cluster, rank = block % g.cluster;
-  const int tx = tile % g.tiles_x, ty = tile / g.tiles_x;
-  P.gx0 = tx * g.TX, P.gy0 = ty * g.TY;
+  const int rank = block % g.cluster;
+  P.gx0 = t.tx * g.TX, P.gy0 = t.ty * g.TY;
   P.lane = thread & 31, P.warp = thread >> 5;
   P.yl = P.warp * R;
   P.c0 = rank * g.warps * R, P.c1 = P.c0 + g.warps * R;
   P.x0 = P.lane * kLaneCols, P.y0 = P.c0 + P.yl;
-  P.left = tx > 0, P.right = tx + 1 < g.tiles_x;
-  P.below = ty > 0, P.above = ty + 1 < g.tiles_y;
+  P.left = t.tx > 0, P.right = t.tx + 1 < t.tiles_x;
+  P.below = t.ty > 0, P.above = t.ty + 1 < t.tiles_y;
   P.ox0 = P.left ? g.halo : 0;
   P.oy0 = P.below ? g.halo : 0;
   P.ox1 = P.right ? kTileW - g.halo : min(kTileW, W - P.gx0);
   P.oy1 = P.above ? g.RH - g.halo : min(g.RH, H - P.gy0);
   P.down = P.warp > 0 || rank > 0;
   P.up = P.warp < g.warps - 1 || rank + 1 < g.cluster;
+  P.idle = P.gy0 + P.y0 >= H;
   return P;
+}
+__device__ __forceinline__ Patch patch_of(const RegTile& g, int R, int W, int H) {
+  unsigned tile = blockIdx.x / g.cluster;
+  asm volatile("" : "+r"(tile));
+  return patch_at(TilePlace{(int)tile % g.tiles_x, (int)tile / g.tiles_x, g.tiles_x, g.tiles_y}, g,
+                  R, W, H);
 }
 
 // Rows of a strip of R that are in [lo, hi) of the region, as a bit mask.
@@ -316,6 +329,23 @@ __device__ __forceinline__ float4 read_message(const Link<WORDS>& link, int part
                      k * 512 + (threadIdx.x & 31) * 16)
                : "memory");
   return x;
+}
+
+// The messages of a strip off the grid, m .. m + count - 1: it takes part so
+// that the strips beside it wait for nothing, and its cells stay as they are
+// (zero, as a neighbour's face off the grid is).
+template <int WORDS>
+__device__ __forceinline__ void idle_messages(const Link<WORDS>& link, unsigned m, int count,
+                                              const ResidentSync& sync) {
+#pragma unroll 1
+  for (const unsigned end = m + count; m != end; m++) {
+#pragma unroll
+    for (int k = 0; k < WORDS / 4; k++) {
+      post<WORDS>(link.down, link.down_part, m, k, make_float4(0.0f, 0.0f, 0.0f, 0.0f));
+      post<WORDS>(link.up, link.up_part, m, k, make_float4(0.0f, 0.0f, 0.0f, 0.0f));
+    }
+    await_message(link, m, sync);
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -737,6 +767,7 @@ struct ProjLane {
   bool wall_r;   // column W - 1 is the lane's last column
   bool closed_r; // and it is solid
   float rs_l, rs_r;  // reciprocal neighbour counts of the cells beside them
+  bool idle;     // the strip is off the grid
   bool full;     // row_full takes every row of the strip
   bool wall;     // some lane of the warp has wall_l or wall_r
   bool own_first;  // no lane changes this lane's first face u from the left
@@ -877,6 +908,7 @@ __device__ __forceinline__ void flags_in(const uint8_t* __restrict__ flags, cons
                                          ProjLane& L) {
   const int gx = P.gx0 + P.x0;
   const bool off = gx >= W;
+  L.idle = P.idle;
   L.wall_l = gx == 0;
   L.wall_r = gx + 7 == W - 1;
   // What row_full takes in this lane: column 0 of the grid and its last column
@@ -1053,6 +1085,7 @@ __device__ __forceinline__ void tile_sweeps(float (&u)[R][8], float (&v)[R][8], 
                                             int cell0, bool down, const Consts& c, float d_t,
                                             int sweeps, unsigned m) {
   static_assert(R % 2 == 0, "strips start on even rows");
+  if (L.idle) return idle_messages(link, m, project_messages(sweeps), sync);
   float ur[R];
 #pragma unroll
   for (int r = 0; r < R; r++) ur[r] = __shfl_down_sync(kAllLanes, u[r][0], 1);
@@ -1101,6 +1134,26 @@ __device__ __forceinline__ void extrapolate_patch(float (&u)[R][8], float (&v)[R
     for (int q = 0; q < 8; q++)
       if (last == q) v[r][q] = q ? v[r][q ? q - 1 : 0] : before;
   }
+}
+
+// The owned cells out to fields uo and vo, extrapolated where asked.
+template <int R>
+__device__ __forceinline__ void faces_out(float (&u)[R][8], float (&v)[R][8], void* uo, void* vo,
+                                          int storage, const Patch& P, int W, int H, bool vec,
+                                          bool extrapolate) {
+  const uint32_t own = rows_in(P.y0, R, P.oy0, P.oy1);
+  uint32_t own_u = own, top = 0u;
+  if (extrapolate) {
+    extrapolate_patch<R>(u, v, P, W);
+    own_u &= ~rows_in(P.y0, R, H - 1 - P.gy0, H - P.gy0);
+    top = own & rows_in(P.y0, R, H - 2 - P.gy0, H - 1 - P.gy0);
+  }
+  on_cells(storage, [&](auto io) {
+    patch_out<R>(io, u, uo, P, own_u, W, H, vec);
+    patch_out<R>(io, v, vo, P, own, W, H, vec);
+    if (top)  // row H - 2 of u to row H - 1, which lies one row before it
+      patch_out<R>(io, u, static_cast<typename decltype(io)::Word*>(uo) - W, P, top, W, H, vec);
+  });
 }
 
 // The pressure of the owned cells, between its field and the tile's planes.
@@ -1233,24 +1286,10 @@ k_project_tiles(const __grid_constant__ ProjectArgs a) {
   }
   if (number != epoch && threadIdx.x == 0) a.sync.epochs[blockIdx.x] = number;
   const Patch Q = patch_of(a.g, R, W, H);
-  // The owned cells to the copies that ceil(n / K) passes through memory would
-  // end in.
+  // To the copies that ceil(n / K) passes through memory would end in.
   const bool swap = ((a.n + a.K - 1) / a.K) & 1;
-  void* uo = (a.cu != 0) != swap ? a.U1 : a.U0;
-  void* vo = (a.cv != 0) != swap ? a.V1 : a.V0;
-  const uint32_t own = rows_in(Q.y0, R, Q.oy0, Q.oy1);
-  uint32_t own_u = own, top = 0u;
-  if (a.extrapolate) {
-    extrapolate_patch<R>(u, v, Q, W);
-    own_u &= ~rows_in(Q.y0, R, H - 1 - Q.gy0, H - Q.gy0);
-    top = own & rows_in(Q.y0, R, H - 2 - Q.gy0, H - 1 - Q.gy0);
-  }
-  on_cells(a.storage, [&](auto io) {
-    patch_out<R>(io, u, uo, Q, own_u, W, H, vec);
-    patch_out<R>(io, v, vo, Q, own, W, H, vec);
-    if (top)  // row H - 2 of u to row H - 1, which lies one row before it
-      patch_out<R>(io, u, static_cast<typename decltype(io)::Word*>(uo) - W, Q, top, W, H, vec);
-  });
+  faces_out<R>(u, v, (a.cu != 0) != swap ? a.U1 : a.U0, (a.cv != 0) != swap ? a.V1 : a.V0,
+               a.storage, Q, W, H, vec, a.extrapolate != 0);
   if (PRESSURE) pressure_out<R>(sm, a.p, Q, W, H, vec);
   cluster_arrive();  // no CTA leaves while another may still send to it
   cluster_wait();
@@ -1267,7 +1306,7 @@ __host__ __device__ inline size_t diffuse_tile_smem(int rows, int warps, int hal
 
 // How a strip's cells are taken: no row or column of it kept, the columns 0, 3
 // and 7 of its lanes where DiffLane says so, or any row or column, and the
-// division may be one (jacobi_divide).
+// division may be one.
 enum class Kept { kNone, kQuadEdges, kAny };
 
 // What a patch holds that no sweep changes: the grid's first and last column
@@ -1276,6 +1315,15 @@ enum class Kept { kNone, kQuadEdges, kAny };
 struct DiffLane {
   uint32_t cols, rows;
 };
+constexpr uint32_t kIdleRows = ~0u;  // DiffLane::rows of a strip off the grid
+__device__ __forceinline__ DiffLane diff_lane(const Patch& P, int R, int W, int H) {
+  DiffLane L;
+  const int gx = P.gx0 + P.x0, gy = P.gy0 + P.y0;
+  L.cols = (gx == 0 ? 1u : 0u) | (W - 1 - gx >= 0 && W - 1 - gx < 8 ? 1u << (W - 1 - gx) : 0u);
+  L.rows = (gy == 0 ? 1u : 0u) | (H - 1 - gy >= 0 && H - 1 - gy < R ? 1u << (H - 1 - gy) : 0u);
+  if (R <= 8 && P.idle) L.rows = kIdleRows;
+  return L;
+}
 
 // One row of a sweep in place: `down` holds the old row below and takes the old
 // row itself, `up` is the old row above.
@@ -1356,7 +1404,9 @@ __device__ __forceinline__ void jacobi_sweeps(float (&u)[R][8], const DiffLane& 
   // every float input (tests/cpp/reciprocal_product.cu), used below 2^20.
   const bool rcp = den < 1048576.0f;
   const uint32_t cols = __reduce_or_sync(kAllLanes, L.cols);
-  if (!rcp || L.rows || (cols & ~0x89u))
+  if (R <= 8 && L.rows == kIdleRows)  // (at 12 rows no predicate is left for it)
+    idle_messages(link, m, sweeps, sync);
+  else if (!rcp || L.rows || (cols & ~0x89u))
     jacobi_loop<R, Kept::kAny>(u, link, sync, L, a, den, rden, rcp, sweeps, m);
   else if (cols)
     jacobi_loop<R, Kept::kQuadEdges>(u, link, sync, L, a, den, rden, true, sweeps, m);
@@ -1393,12 +1443,7 @@ k_diffuse_tiles(const __grid_constant__ DiffuseArgs a) {
 #pragma unroll
     for (int q = 0; q < 8; q++) u[r][q] = 0.0f;
   on_cells(a.storage, [&](auto io) { patch_in<R>(io, u, a.cu ? a.U1 : a.U0, P, W, H, vec); });
-  DiffLane L;
-  {
-    const int gx = P.gx0 + P.x0, gy = P.gy0 + P.y0;
-    L.cols = (gx == 0 ? 1u : 0u) | (W - 1 - gx >= 0 && W - 1 - gx < 8 ? 1u << (W - 1 - gx) : 0u);
-    L.rows = (gy == 0 ? 1u : 0u) | (H - 1 - gy >= 0 && H - 1 - gy < R ? 1u << (H - 1 - gy) : 0u);
-  }
+  const DiffLane L = diff_lane(P, R, W, H);
   const float coeff = diffusion_coeff<float>(c, a.prm->dt);
   const unsigned epoch = a.n > a.D ? ld_acquire_gpu(a.sync.epochs + blockIdx.x) : 0u;
   unsigned number = epoch;

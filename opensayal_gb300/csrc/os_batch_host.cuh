@@ -76,10 +76,11 @@ namespace {
 
 // The tiles of a phase: clusters of `cluster` CTAs.
 RegTile batch_geom(int K, bool projection, int cluster) {
-  RegTile g = reg_tile(1 << 30, 1 << 30, projection ? 2 * K : K, kBatchRows, kBatchWarps, cluster);
-  const int rows = kBatchRows * kBatchWarps;
-  g.smem = projection ? project_tile_smem(rows, kBatchWarps, false, g.halo, false)
-                      : diffuse_tile_smem(rows, kBatchWarps, g.halo, false);
+  const int R = projection ? kBatchProjectRows : kBatchDiffuseRows;
+  const int warps = projection ? kBatchProjectWarps : kBatchDiffuseWarps;
+  RegTile g = reg_tile(1 << 30, 1 << 30, projection ? 2 * K : K, R, warps, cluster);
+  g.smem = projection ? project_tile_smem(R * warps, warps, false, g.halo, false)
+                      : diffuse_tile_smem(R * warps, warps, g.halo, false);
   return g;
 }
 

@@ -47,10 +47,11 @@ __device__ __forceinline__ const T* plan_array(const PlanHeader* P, int off) {
   return reinterpret_cast<const T*>(reinterpret_cast<const char*>(P) + off);
 }
 
-// The batch's tile kernels: clusters of `kBatchRows` x `kBatchWarps` CTAs that
-// walk the tiles of one pass. With 4 warps of 255 registers an SM holds two
-// CTAs (three of the diffusion's), so that one stages while the other sweeps.
-constexpr int kBatchRows = 8, kBatchWarps = 4;
+// The batch's tile kernels: clusters of CTAs of so many strips that walk the
+// tiles of one pass, two CTAs to an SM (three of the diffusion's), so that one
+// loads and stores while the other sweeps.
+constexpr int kBatchProjectRows = 6, kBatchProjectWarps = 6;
+constexpr int kBatchDiffuseRows = 8, kBatchDiffuseWarps = 4;
 using BatchTileKernel = void (*)(const PlanHeader*, const int*, int, int, const RegTile,
                                  const ResidentSync);
 BatchTileKernel batch_project_kernel();

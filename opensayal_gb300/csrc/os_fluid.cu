@@ -1519,7 +1519,7 @@ float time_steps(os_handle* t, float dt, int warm, int reps) {
   return ms;
 }
 
-// Candidates: depths {2, 4, 6, 8, 12} pass by pass and, unless
+// Candidates: depths {4, 6, 8, 12, 16} pass by pass (2 for fewer sweeps than 4) and, unless
 // projection_resident is -1, the resident forms (projection and diffusion,
 // alone or together) where the grid fits them, at one depth: a resident form
 // chooses its own sweeps between exchanges, and the depth only says how often
@@ -1539,7 +1539,7 @@ TuneChoice autotune_projection(const os_config& base) {
     if (it != g_tuned.end()) return it->second;
   }
   std::vector<TuneChoice> cands;
-  for (int K : {2, 4, 6, 8, 12}) {
+  for (int K : {base.projection_n < 4 ? 2 : 4, 6, 8, 12, 16}) {
     if (base.projection_resident > 0)
       cands.push_back({K, base.projection_resident, 0});
     else
@@ -1593,19 +1593,23 @@ TuneChoice autotune_projection(const os_config& base) {
     }
   }
   // Deeper diffusion passes than the projection's (the Jacobi halo is half
-  // the red/black one), when the diffusion runs pass by pass.
+  // the red/black one), or a resident diffusion beside the projection's passes,
+  // when the diffusion runs pass by pass.
   if (base.viscosity != 0.0f && base.diffusion_block == 0 && best_ms > 0.0f &&
       !(best.resident & 2)) {
     const TuneChoice chosen = best;
-    for (int dk : {12, 16, 20})
-      if (dk > chosen.K && dk <= base.projection_n) {
-        const TuneChoice cand{chosen.K, chosen.resident, dk};
-        const float ms = time_choice(cand, 60);
-        if (ms > 0.0f && ms < best_ms) {
-          best_ms = ms;
-          best = cand;
-        }
+    auto consider = [&](const TuneChoice& cand) {
+      const float ms = time_choice(cand, 60);
+      if (ms > 0.0f && ms < best_ms) {
+        best_ms = ms;
+        best = cand;
       }
+    };
+    for (int dk : {12, 16})
+      if (dk > chosen.K && dk <= base.projection_n)
+        consider(TuneChoice{chosen.K, chosen.resident, dk});
+    if (base.projection_resident == 0 && chosen.resident == 0 && chosen.K % 4 == 0)
+      consider(TuneChoice{chosen.K, 2, 0});
   }
   g_err[0] = '\0';  // a candidate that failed is not the caller's error
   std::lock_guard<std::mutex> lock(g_tune_mu);

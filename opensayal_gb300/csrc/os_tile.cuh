@@ -1321,7 +1321,7 @@ __device__ __forceinline__ DiffLane diff_lane(const Patch& P, int R, int W, int 
   const int gx = P.gx0 + P.x0, gy = P.gy0 + P.y0;
   L.cols = (gx == 0 ? 1u : 0u) | (W - 1 - gx >= 0 && W - 1 - gx < 8 ? 1u << (W - 1 - gx) : 0u);
   L.rows = (gy == 0 ? 1u : 0u) | (H - 1 - gy >= 0 && H - 1 - gy < R ? 1u << (H - 1 - gy) : 0u);
-  if (R <= 8 && P.idle) L.rows = kIdleRows;
+  if (P.idle) L.rows = kIdleRows;
   return L;
 }
 
@@ -1329,11 +1329,17 @@ __device__ __forceinline__ DiffLane diff_lane(const Patch& P, int R, int W, int 
 // row itself, `up` is the old row above.
 template <Kept KEPT>
 __device__ __forceinline__ void jacobi_row(float (&u)[8], float (&down)[8], const float (&up)[8],
-                                           bool kept_row, const DiffLane& L, float a, float den,
+                                           int r, const DiffLane& L, float a, float den,
                                            float rden, bool rcp) {
   float left = __shfl_up_sync(kAllLanes, u[7], 1);
   const float right = __shfl_down_sync(kAllLanes, u[0], 1);
-  const uint32_t kept = KEPT == Kept::kAny && kept_row ? 0xffu : L.cols;
+  uint32_t kept = L.cols;
+  if (KEPT == Kept::kAny) {
+    // (Worked out in each sweep: hoisted, the rows' and columns' conditions
+    // are more than the seven predicates there are.)
+    asm volatile("{\n .reg .s32 m;\n bfe.s32 m, %1, %2, 1;\n or.b32 %0, %0, m;\n}"
+                 : "+r"(kept) : "r"(L.rows), "r"(r));
+  }
 #pragma unroll
   for (int q = 0; q < 8; q++) {
     const float old = u[q];
@@ -1382,12 +1388,12 @@ __device__ __forceinline__ void jacobi_loop(float (&u)[R][8], const Link<8>& lin
     for (int q = 0; q < 8; q++) down[q] = u[0][q], second[q] = u[1][q];
 #pragma unroll
     for (int r = 1; r < R - 1; r++)
-      jacobi_row<KEPT>(u[r], down, u[r + 1], (L.rows >> r) & 1u, L, a, den, rden, rcp);
+      jacobi_row<KEPT>(u[r], down, u[r + 1], r, L, a, den, rden, rcp);
     await_message(link, m, sync);
     row_receive(row, link, 1, m);
-    jacobi_row<KEPT>(u[R - 1], down, row, (L.rows >> (R - 1)) & 1u, L, a, den, rden, rcp);
+    jacobi_row<KEPT>(u[R - 1], down, row, R - 1, L, a, den, rden, rcp);
     row_receive(row, link, 0, m);
-    jacobi_row<KEPT>(u[0], row, second, L.rows & 1u, L, a, den, rden, rcp);
+    jacobi_row<KEPT>(u[0], row, second, 0, L, a, den, rden, rcp);
   }
 }
 
@@ -1404,7 +1410,7 @@ __device__ __forceinline__ void jacobi_sweeps(float (&u)[R][8], const DiffLane& 
   // every float input (tests/cpp/reciprocal_product.cu), used below 2^20.
   const bool rcp = den < 1048576.0f;
   const uint32_t cols = __reduce_or_sync(kAllLanes, L.cols);
-  if (R <= 8 && L.rows == kIdleRows)  // (at 12 rows no predicate is left for it)
+  if (L.rows == kIdleRows)
     idle_messages(link, m, sweeps, sync);
   else if (!rcp || L.rows || (cols & ~0x89u))
     jacobi_loop<R, Kept::kAny>(u, link, sync, L, a, den, rden, rcp, sweeps, m);
@@ -1485,4 +1491,3 @@ template <int R> ProjectKernel project_kernel(bool pressure);
 template <int R> DiffuseKernel diffuse_kernel();
 
 }  // namespace osg
-

@@ -5,18 +5,20 @@
 // Bound by the sweeps' instructions and by the faces' way from strip to strip;
 // the loads and stores of one tile run beside the sweeps of the other on the
 // SM. 21 tunnels of 128 to 1024 cells a side (6.85 M cells in all): a step
-// takes 2188 us, and took 2968 us with tiles held in shared memory; 6 tunnels
-// of mixed storage 2094 us, and 3378 us.
+// takes 2079 us, and took 2968 us with tiles held in shared memory; 6 tunnels
+// of mixed storage 2036 us, and 3378 us.
 #include "os_batch_plan.cuh"
 
 namespace osg {
 namespace {
 
-// Two CTAs of the projection's 255 registers fill an SM's register file.
-__global__ void __launch_bounds__(32 * kBatchWarps, 2)
+// Two CTAs of six warps with 168 registers fill an SM's register file: three
+// warps to a scheduler hide the faces' way better than two of four warps with
+// 255 (2079 us against 2188 us for the 21 tunnels above).
+__global__ void __launch_bounds__(32 * kBatchProjectWarps, 2)
 k_batch_project_tiles(const PlanHeader* __restrict__ plan, const int* __restrict__ remaining,
                       int pass, int K, const RegTile g, const ResidentSync sync) {
-  constexpr int R = kBatchRows;
+  constexpr int R = kBatchProjectRows;
   extern __shared__ __align__(16) char tile_smem[];
   const ProjSmem sm = project_smem_of(tile_smem, g.warps * R, g.warps, false);
   const Link<4> link = open_link<4>(tile_smem, patch_at(TilePlace{0, 0, 1, 1}, g, R, 1, 1), g);
@@ -72,10 +74,10 @@ k_batch_project_tiles(const PlanHeader* __restrict__ plan, const int* __restrict
   cluster_wait();
 }
 
-__global__ void __launch_bounds__(32 * kBatchWarps, 3)
+__global__ void __launch_bounds__(32 * kBatchDiffuseWarps, 3)
 k_batch_diffuse_tiles(const PlanHeader* __restrict__ plan, const int* __restrict__ remaining,
                       int pass, int K, const RegTile g, const ResidentSync sync) {
-  constexpr int R = kBatchRows;
+  constexpr int R = kBatchDiffuseRows;
   extern __shared__ __align__(16) char tile_smem[];
   const Link<8> link = open_link<8>(tile_smem, patch_at(TilePlace{0, 0, 1, 1}, g, R, 1, 1), g);
   cluster_arrive();

@@ -59,16 +59,25 @@ inline RegTile reg_tile(int W, int H, int halo, int R, int warps, int cluster) {
 // clusters of 2, 144 of 4, 138 of 6, 120 of 8, 130 of 10, 96 of 12, 112 of 16).
 constexpr int kClusters[] = {2, 4, 6, 8, 10, 12, 16};
 
-// Clusters of `cluster` CTAs, one CTA per SM, that are resident together.
-inline int resident_clusters(int device, int cluster) {
+// CTAs of a tile kernel that an SM holds, by the registers that its launch
+// bounds allow it, its shared memory and its threads.
+inline int ctas_per_sm(int R, int warps, bool projection, size_t smem) {
+  const int regs = R <= 4 ? 128 : R <= (projection ? 6 : 8) ? 168 : 256;
+  const int by_regs = 65536 / (regs * 32 * warps), by_smem = (int)((228 << 10) / (smem + 1024));
+  return std::max(1, std::min({by_regs, by_smem, 64 / warps, 4}));
+}
+
+// Clusters of `cluster` CTAs that are resident together with `ctas` CTAs to an
+// SM.
+inline int resident_clusters(int device, int cluster, int ctas) {
   static std::mutex mu;
-  static std::map<std::pair<int, int>, int> known;
+  static std::map<std::tuple<int, int, int>, int> known;
   std::lock_guard<std::mutex> lock(mu);
-  const auto key = std::make_pair(device, cluster);
+  const auto key = std::make_tuple(device, cluster, ctas);
   auto it = known.find(key);
   if (it != known.end()) return it->second;
-  const auto kernel = project_kernel<8>(false);
-  const size_t smem = 200 * 1024;
+  const auto kernel = diffuse_kernel<2>();
+  const size_t smem = (227 / ctas - 1) * 1024;  // as much as leaves room for no more CTAs
   int n = 0;
   if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) ==
           cudaSuccess &&
@@ -76,7 +85,7 @@ inline int resident_clusters(int device, int cluster) {
           cudaSuccess) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(cluster * 152);
-    cfg.blockDim = dim3(32 * project_max_warps(8));
+    cfg.blockDim = dim3(128);
     cfg.dynamicSmemBytes = smem;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -105,8 +114,8 @@ inline double choose_tile(int W, int H, int D, bool projection, bool pressure, b
   const int* heights = projection ? kProjectRows : kDiffuseRows;
   const int count = projection ? (int)std::size(kProjectRows) : (int)std::size(kDiffuseRows);
   for (int cluster : kClusters) {
-    const int fit = resident_clusters(device, cluster);
-    if (fit < 1) continue;
+    const int alone = resident_clusters(device, cluster, 1);
+    if (alone < 1) continue;
     for (int k = 0; k < count; k++) {
       const int R = heights[k];
       const int most = projection ? project_max_warps(R) : diffuse_max_warps(R);
@@ -115,23 +124,32 @@ inline double choose_tile(int W, int H, int D, bool projection, bool pressure, b
         if (g.tiles_y < 1) continue;
         const int64_t tiles = (int64_t)g.tiles_x * g.tiles_y;
         const bool one = tiles == 1;
-        if (resident && (tiles > fit || (g.tiles_y > 1 && g.TY < halo) || g.TX < halo)) continue;
+        if (resident && (tiles > alone || (g.tiles_y > 1 && g.TY < halo) || g.TX < halo)) continue;
         const int rows = R * warps;
         g.smem = projection
                      ? project_tile_smem(rows, warps, pressure, g.halo, resident && !one)
                      : diffuse_tile_smem(rows, warps, g.halo, resident && !one);
         if (g.smem + kStaticSmem > kMaxSmem) continue;
+        // Pass by pass, several CTAs share an SM: over three waves or more they
+        // drift apart, and one loads and stores beside the other's sweeps (in
+        // fewer they do the same at the same time: 1920 x 1080 in passes of 8
+        // sweeps took 170 us so, and 142 us with an SM to each CTA).
+        int share = resident ? 1 : ctas_per_sm(R, warps, projection, g.smem);
+        int fit = share > 1 ? resident_clusters(device, cluster, share) : alone;
+        if (share > 1 && tiles <= 2 * fit) share = 1, fit = alone;
+        if (fit < 1) continue;
         const int64_t waves = (tiles + fit - 1) / fit;
         // Cycles of a sweep: the slowest strip (one by the flags, or with kept
         // rows), the other strips of its scheduler, and the messages' way.
-        const int others = (warps + 3) / 4 - 1;
+        const int others = (share * warps + 3) / 4 - 1;
         const double sweep =
             projection ? 650.0 + (pressure ? 230.0 : 170.0) * R +
                              others * ((pressure ? 115.0 : 72.0) * R + 90.0)
                        : 450.0 + 130.0 * R + others * (50.0 * R + 60.0);
         // A round: the exchange of the rows and sides, or the region in and
         // out of memory.
-        double trip = 5000.0 + rows * (projection ? 50.0 : 25.0);
+        double trip = 5000.0 + share * rows * (projection ? 50.0 : 25.0);
+        if (share > 1) trip *= 0.8;
         if (resident) {
           const int halo_rows = g.tiles_y > 1 ? std::min(2 * halo, rows) : 0;
           const double quads = 64.0 * halo_rows + rows * (halo / 2.0);

@@ -64,6 +64,24 @@ def test_phases_equal_plain(gpu, w, h, k, n, resident, wild):
     b.close()
 
 
+@pytest.mark.parametrize("w,h", [(2400, 2100), (3001, 1999)])
+@pytest.mark.parametrize("k", [4, 16])
+def test_many_tiles_equal_plain(gpu, w, h, k):
+    """Enough tiles for three rounds of CTAs that share their SMs."""
+    base = tunnel(w, h, projection_n=k + 2)
+    state = state_of(base, 9)
+    plain, tiles = base.copy(), base.copy()
+    plain.projection_block = -1
+    tiles.projection_block, tiles.projection_resident = k, -1
+    a, b = load_lib(plain, state), load_lib(tiles, state)
+    for phase in (native.PHASE_DIFFUSION, native.PHASE_PROJECTION):
+        a.run_phase(phase, None, 0.05)
+        b.run_phase(phase, None, 0.05)
+    equal(a, b, FIELDS)
+    a.close()
+    b.close()
+
+
 @pytest.mark.parametrize("w,h", [(257, 129), (480, 97), (1280, 300)])
 @pytest.mark.parametrize("storage", [native.STORAGE_F16, native.STORAGE_BF16])
 def test_16_bit_resident_equals_passes(gpu, w, h, storage):
@@ -84,7 +102,7 @@ def test_16_bit_resident_equals_passes(gpu, w, h, storage):
 def test_batch_members_equal_alone(gpu, block_k):
     cfgs = []
     for i, (w, h) in enumerate([(8, 8), (255, 127), (256, 128), (257, 129), (241, 200), (33, 400),
-                                (600, 113), (64, 257)]):
+                                (600, 113), (64, 257), (320, 144), (96, 145)]):
         c = tunnel(w, h, projection_n=2 * block_k + 1 + i, projection_block=block_k)
         c.storage = (native.STORAGE_F32, native.STORAGE_F16, native.STORAGE_BF16)[i % 3]
         if i == 4:

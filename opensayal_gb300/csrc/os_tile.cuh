@@ -364,9 +364,10 @@ __device__ __forceinline__ void idle_messages(const Link<WORDS>& link, unsigned 
 //
 // Packets lie by the cell they carry, in two copies that alternate. A copy is
 // written again two exchanges later: by then the writer has received the
-// exchange between from every neighbouring tile, whose warps sent it after the
-// sweeps that follow their reads of this one (the sweeps hold barriers of the
-// CTA, and a CTA receives from all its neighbours).
+// exchange between from every neighbouring tile, whose CTAs sent it after their
+// reads of this one: a CTA sends behind its own barrier, and the CTAs of a
+// tile whose rows lie within a halo of each other have since exchanged
+// messages in the sweeps between, as many strips far as a halo has rows.
 // ---------------------------------------------------------------------------
 constexpr int kSpinLimit = 1 << 20;  // polls per wait
 

@@ -142,7 +142,7 @@ inline double choose_tile(int W, int H, int D, bool projection, bool pressure, b
         // Cycles of a sweep: the slowest strip (one by the flags, or with kept
         // rows), the other strips of its scheduler, and the messages' way.
         const int others = (share * warps + 3) / 4 - 1;
-        const double sweep =
+        double sweep =
             projection ? 650.0 + (pressure ? 230.0 : 170.0) * R +
                              others * ((pressure ? 115.0 : 72.0) * R + 90.0)
                        : 450.0 + 130.0 * R + others * (50.0 * R + 60.0);
@@ -153,7 +153,19 @@ inline double choose_tile(int W, int H, int D, bool projection, bool pressure, b
         if (resident) {
           const int halo_rows = g.tiles_y > 1 ? std::min(2 * halo, rows) : 0;
           const double quads = 64.0 * halo_rows + rows * (halo / 2.0);
-          trip = 3500.0 + quads * (projection ? 4.0 : 2.7);
+          // Fitted to the times of every tile that ten grids from 333 x 187 to
+          // 1280 x 720 take (projection with and without the pressure,
+          // diffusion; 10,000 times in all, within 5 to 7%). The choice is 1
+          // to 2% behind the best of them in the mean and 9% at most; with the
+          // terms of the passes above it was up to 28% (projection) and 48%
+          // (diffusion) behind: four warps to a scheduler cost more than they
+          // said, and the rows of an exchange less.
+          sweep = !projection ? 360.0 + 140.0 * R + 280.0 * others
+                  : pressure  ? 680.0 + (350.0 + 118.0 * others) * R
+                              : 750.0 + (200.0 + 87.0 * others) * R;
+          trip = !projection ? 3900.0 + 0.2 * quads
+                 : pressure  ? 4000.0 + 0.85 * quads
+                             : 4300.0 + 1.1 * quads;
         }
         const double rounds = resident ? (one ? 0 : (n + D - 1) / D - 1) : (n + D - 1) / D;
         const double cost = (double)waves * (n * sweep + rounds * trip);
@@ -211,7 +223,7 @@ inline int resident_tile(const os_handle* h, bool projection, RegTile* g) {
   if (K < 2 || K % (projection ? 2 : 4)) return 0;
   int depth = 0;
   double best = 0.0;
-  for (int D : {2, 4, 6, 8, 12, 16}) {  // halos in multiples of 4 cells
+  for (int D : {2, 4, 6, 8, 12, 16, 20}) {  // halos in multiples of 4 cells
     if (!projection && D % 4) continue;
     RegTile t;
     const double cost = choose_tile(h->W, h->H, D, projection, pressure, true, n, h->cfg.device, &t);

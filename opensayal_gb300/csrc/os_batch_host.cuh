@@ -81,6 +81,7 @@ RegTile batch_geom(int K, bool projection, int cluster) {
   RegTile g = reg_tile(1 << 30, 1 << 30, projection ? 2 * K : K, R, warps, cluster);
   g.smem = projection ? project_tile_smem(R * warps, warps, false, g.halo, false)
                       : diffuse_tile_smem(R * warps, warps, g.halo, false);
+  g.smem += stage_smem(1, g.halo, warps);  // members may have any width
   return g;
 }
 

@@ -98,6 +98,7 @@ struct F32Cells {
     asm volatile("{\n .reg .pred p;\n setp.ne.s32 p, %2, 0;\n @p ld.global.cg.f32 %0, [%1];\n}"
                  : "+f"(*q) : "l"(p), "r"((int)on) : "memory");
   }
+  __device__ __forceinline__ float value(float q) const { return q; }
   __device__ __forceinline__ void store4(bool on, float* p, const float* q) const {
     asm volatile(
         "{\n .reg .pred p;\n setp.ne.s32 p, %5, 0;\n @p st.global.v4.f32 [%4], {%0, %1, %2, %3};\n}"
@@ -125,12 +126,14 @@ struct HalfCells {
     q[0] = on ? from(a & 0xffffu) : q[0], q[1] = on ? from(a >> 16) : q[1];
     q[2] = on ? from(b & 0xffffu) : q[2], q[3] = on ? from(b >> 16) : q[3];
   }
+  // The cell's bits, which value() turns into the cell: as it came, a patch's
+  // conversions stood between its loads, and few of them were in flight.
   __device__ __forceinline__ void load1(bool on, const uint16_t* p, float* q) const {
-    uint16_t a = 0;
-    asm volatile("{\n .reg .pred p;\n setp.ne.s32 p, %2, 0;\n @p ld.global.cg.u16 %0, [%1];\n}"
-                 : "+h"(a) : "l"(p), "r"((int)on) : "memory");
-    *q = on ? from(a) : *q;
+    asm volatile("{\n .reg .pred p;\n .reg .b32 t;\n mov.b32 t, %0;\n setp.ne.s32 p, %2, 0;\n"
+                 " @p ld.global.cg.u16 t, [%1];\n mov.b32 %0, t;\n}"
+                 : "+f"(*q) : "l"(p), "r"((int)on) : "memory");
   }
+  __device__ __forceinline__ float value(float q) const { return from(__float_as_uint(q)); }
   __device__ __forceinline__ void store4(bool on, uint16_t* p, const float* q) const {
     asm volatile("{\n .reg .pred p;\n setp.ne.s32 p, %3, 0;\n @p st.global.v2.u32 [%2], {%0, %1};\n}"
                  ::"r"(to(q[0]) | to(q[1]) << 16), "r"(to(q[2]) | to(q[3]) << 16), "l"(p),
@@ -411,18 +414,60 @@ __device__ __forceinline__ bool poll_again(int it, const ResidentSync& sync) {
   return false;
 }
 
-// The whole patch from a field (row j of the grid at (H - 1 - j) W). `vec`: W and
-// the columns of the region's quads are multiples of 4; the loads then carry
-// no condition (a kernel's code is fetched cold once per launch, so what it
+// Where quads of the region are not aligned (W or the halo is no multiple of
+// 4), a warp takes a row's cells one by one, lanes on consecutive columns, and
+// turns them between that order (lane l: columns l, l + 32, ..) and the patch's
+// through a row of shared memory of its own. With each lane on its own eight
+// columns every access touched a sector per lane (307 x 479 in FP16, passes of
+// 4 sweeps: 245 us a step, now 156; 3001 x 1500: 735 us, now 531).
+constexpr int kStageBytes = kTileW * 4;  // per warp
+__host__ __device__ inline bool quads_aligned(int W, int halo) { return ((W | halo) & 3) == 0; }
+__host__ __device__ inline size_t stage_smem(int W, int halo, int warps) {
+  return quads_aligned(W, halo) ? 0 : (size_t)warps * kStageBytes;
+}
+// The warp's row, at the end of the CTA's shared memory. (The kernels of a
+// single grid are built for aligned quads and for others: with both ways in
+// one kernel the strips of 10 rows spilled, 272 us a step at 1920 x 1080
+// instead of 236.)
+__device__ __forceinline__ float* stage_of(char* smem, const RegTile& g) {
+  unsigned thread = threadIdx.x;
+  asm volatile("" : "+r"(thread));  // worked out anew where it is used, as patch_at
+  float* row = reinterpret_cast<float*>(smem + g.smem - (g.warps - (thread >> 5)) * kStageBytes);
+  __builtin_assume(row != nullptr);
+  return row;
+}
+template <class IO>
+__device__ __forceinline__ void turn_in(const IO& io, float (&f)[8], float* stage, int lane) {
+#pragma unroll
+  for (int k = 0; k < 8; k++) stage[lane + 32 * k] = io.value(f[k]);
+  __syncwarp();
+  const float4 a = reinterpret_cast<const float4*>(stage)[2 * lane];
+  const float4 b = reinterpret_cast<const float4*>(stage)[2 * lane + 1];
+  __syncwarp();
+  f[0] = a.x, f[1] = a.y, f[2] = a.z, f[3] = a.w;
+  f[4] = b.x, f[5] = b.y, f[6] = b.z, f[7] = b.w;
+}
+__device__ __forceinline__ void turn_out(const float (&f)[8], float (&g)[8], float* stage,
+                                         int lane) {
+  reinterpret_cast<float4*>(stage)[2 * lane] = make_float4(f[0], f[1], f[2], f[3]);
+  reinterpret_cast<float4*>(stage)[2 * lane + 1] = make_float4(f[4], f[5], f[6], f[7]);
+  __syncwarp();
+#pragma unroll
+  for (int k = 0; k < 8; k++) g[k] = stage[lane + 32 * k];
+  __syncwarp();
+}
+
+// The whole patch from a field (row j of the grid at (H - 1 - j) W). `stage`: see
+// above; null where quads are aligned: the loads then carry no condition (a kernel's code is fetched cold once per launch, so what it
 // does once has to be short), and a cell off the grid reads the nearest quad
 // or row of it: cells off the grid may hold any value, no cell of the grid
 // depends on them.
 template <int R, class IO>
 __device__ __forceinline__ void patch_in(const IO& io, float (&f)[R][8], const void* field,
-                                         const Patch& P, int W, int H, bool vec) {
+                                         const Patch& P, int W, int H, float* stage) {
   const int x = P.gx0 + P.x0, j0 = P.gy0 + P.y0;
   const typename IO::Word* base = static_cast<const typename IO::Word*>(field);
-  if (vec) {
+  if (!stage) {
     const int xa = min(x, W - 4), xb = min(x + 4, W - 4);
     const int step = H - 1 - j0;  // rows of the grid above row j0
     const typename IO::Word* row = base + (int64_t)max(step, 0) * W;
@@ -434,37 +479,44 @@ __device__ __forceinline__ void patch_in(const IO& io, float (&f)[R][8], const v
     }
     return;
   }
-  const typename IO::Word* row = base + (int64_t)(H - 1 - j0) * W + x;
+  const int xl = P.gx0 + P.lane;
+  const typename IO::Word* row = base + (int64_t)(H - 1 - j0) * W + xl;
 #pragma unroll
   for (int r = 0; r < R; r++, row -= W)
 #pragma unroll
-    for (int q = 0; q < 8; q++) io.load1(j0 + r < H && x + q < W, row + q, &f[r][q]);
+    for (int k = 0; k < 8; k++) io.load1(j0 + r < H && xl + 32 * k < W, row + 32 * k, &f[r][k]);
+#pragma unroll
+  for (int r = 0; r < R; r++) turn_in(io, f[r], stage, P.lane);
 }
 
 // Row y of the region, the lane's eight columns, in the same way.
 template <class IO>
 __device__ __forceinline__ void row_in(const IO& io, float (&f)[8], const void* field,
-                                       const Patch& P, int y, int W, int H, bool vec) {
+                                       const Patch& P, int y, int W, int H, float* stage) {
   const int x = P.gx0 + P.x0, j = min(P.gy0 + y, H - 1);
   const typename IO::Word* row =
       static_cast<const typename IO::Word*>(field) + (int64_t)(H - 1 - j) * W;
-  if (vec) {
+  if (!stage) {
     io.load4(true, row + min(x, W - 4), &f[0]);
     io.load4(true, row + min(x + 4, W - 4), &f[4]);
   } else {
+    const int xl = P.gx0 + P.lane;
 #pragma unroll
-    for (int q = 0; q < 8; q++) io.load1(x + q < W, row + x + q, &f[q]);
+    for (int k = 0; k < 8; k++) io.load1(xl + 32 * k < W, row + xl + 32 * k, &f[k]);
+    turn_in(io, f, stage, P.lane);
   }
 }
 
 // The patch's rows in `rows` out to a field, the owned columns among them.
 template <int R, class IO>
 __device__ __forceinline__ void patch_out(const IO& io, const float (&f)[R][8], void* field,
-                                          const Patch& P, uint32_t rows, int W, int H, bool vec) {
-  const int lo = P.ox0 - P.x0, hi = P.ox1 - P.x0;  // owned columns of the patch
+                                          const Patch& P, uint32_t rows, int W, int H,
+                                          float* stage) {
   typename IO::Word* row = static_cast<typename IO::Word*>(field) +
-                           (int64_t)(H - 1 - (P.gy0 + P.y0)) * W + P.gx0 + P.x0;
-  if (vec) {
+                           (int64_t)(H - 1 - (P.gy0 + P.y0)) * W + P.gx0 +
+                           (stage ? P.lane : P.x0);
+  if (!stage) {
+    const int lo = P.ox0 - P.x0, hi = P.ox1 - P.x0;  // owned columns of the patch
     const bool qa = 0 >= lo && 0 < hi, qb = 4 >= lo && 4 < hi;
 #pragma unroll
     for (int r = 0; r < R; r++, row -= W) {
@@ -475,10 +527,16 @@ __device__ __forceinline__ void patch_out(const IO& io, const float (&f)[R][8], 
     return;
   }
 #pragma unroll
-  for (int r = 0; r < R; r++, row -= W)
+  for (int r = 0; r < R; r++, row -= W) {
+    if (((rows >> r) & 1u) == 0u) continue;
+    float g[8];
+    turn_out(f[r], g, stage, P.lane);
 #pragma unroll
-    for (int q = 0; q < 8; q++)
-      io.store1(((rows >> r) & 1u) && q >= lo && q < hi, row + q, &f[r][q]);
+    for (int k = 0; k < 8; k++) {
+      const int x = P.lane + 32 * k;
+      io.store1(x >= P.ox0 && x < P.ox1, row + 32 * k, &g[k]);
+    }
+  }
 }
 
 // Packets of a quad of cells: three for u and v (8 values), two for u alone.
@@ -1140,7 +1198,7 @@ __device__ __forceinline__ void extrapolate_patch(float (&u)[R][8], float (&v)[R
 // The owned cells out to fields uo and vo, extrapolated where asked.
 template <int R>
 __device__ __forceinline__ void faces_out(float (&u)[R][8], float (&v)[R][8], void* uo, void* vo,
-                                          int storage, const Patch& P, int W, int H, bool vec,
+                                          int storage, const Patch& P, int W, int H, float* stage,
                                           bool extrapolate) {
   const uint32_t own = rows_in(P.y0, R, P.oy0, P.oy1);
   uint32_t own_u = own, top = 0u;
@@ -1150,17 +1208,17 @@ __device__ __forceinline__ void faces_out(float (&u)[R][8], float (&v)[R][8], vo
     top = own & rows_in(P.y0, R, H - 2 - P.gy0, H - 1 - P.gy0);
   }
   on_cells(storage, [&](auto io) {
-    patch_out<R>(io, u, uo, P, own_u, W, H, vec);
-    patch_out<R>(io, v, vo, P, own, W, H, vec);
+    patch_out<R>(io, u, uo, P, own_u, W, H, stage);
+    patch_out<R>(io, v, vo, P, own, W, H, stage);
     if (top)  // row H - 2 of u to row H - 1, which lies one row before it
-      patch_out<R>(io, u, static_cast<typename decltype(io)::Word*>(uo) - W, P, top, W, H, vec);
+      patch_out<R>(io, u, static_cast<typename decltype(io)::Word*>(uo) - W, P, top, W, H, stage);
   });
 }
 
 // The pressure of the owned cells, between its field and the tile's planes.
 template <int R>
 __device__ __forceinline__ void pressure_in(const ProjSmem& sm, const float* p, const Patch& P,
-                                            int W, bool zero, int H, bool vec) {
+                                            int W, bool zero, int H, float* stage) {
   float f[R][8];
 #pragma unroll
   for (int r = 0; r < R; r++)
@@ -1168,18 +1226,26 @@ __device__ __forceinline__ void pressure_in(const ProjSmem& sm, const float* p, 
     for (int q = 0; q < 8; q++) f[r][q] = 0.0f;
   const int lo = P.ox0 - P.x0, hi = P.ox1 - P.x0;
   const uint32_t own = zero ? 0u : rows_in(P.y0, R, P.oy0, P.oy1);
-  const float* row = p + (int64_t)(H - 1 - (P.gy0 + P.y0)) * W + P.gx0 + P.x0;
+  const float* row =
+      p + (int64_t)(H - 1 - (P.gy0 + P.y0)) * W + P.gx0 + (stage ? P.lane : P.x0);
   const F32Cells io;
 #pragma unroll
   for (int r = 0; r < R; r++, row -= W) {
     const bool on = (own >> r) & 1u;
-    if (vec) {
+    if (!stage) {
       io.load4(on && 0 >= lo && 0 < hi, row, &f[r][0]);
       io.load4(on && 4 >= lo && 4 < hi, row + 4, &f[r][4]);
     } else {
 #pragma unroll
-      for (int q = 0; q < 8; q++) io.load1(on && q >= lo && q < hi, row + q, &f[r][q]);
+      for (int k = 0; k < 8; k++) {
+        const int x = P.lane + 32 * k;
+        io.load1(on && x >= P.ox0 && x < P.ox1, row + 32 * k, &f[r][k]);
+      }
     }
+  }
+  if (stage && own) {
+#pragma unroll
+    for (int r = 0; r < R; r++) turn_in(io, f[r], stage, P.lane);
   }
 #pragma unroll
   for (int r = 0; r < R; r++) {
@@ -1191,7 +1257,7 @@ __device__ __forceinline__ void pressure_in(const ProjSmem& sm, const float* p, 
 
 template <int R>
 __device__ __forceinline__ void pressure_out(const ProjSmem& sm, float* p, const Patch& P, int W,
-                                             int H, bool vec) {
+                                             int H, float* stage) {
   float f[R][8];
 #pragma unroll
   for (int r = 0; r < R; r++) {
@@ -1200,7 +1266,7 @@ __device__ __forceinline__ void pressure_out(const ProjSmem& sm, float* p, const
     f[r][0] = e.x, f[r][2] = e.y, f[r][4] = e.z, f[r][6] = e.w;
     f[r][1] = o.x, f[r][3] = o.y, f[r][5] = o.z, f[r][7] = o.w;
   }
-  patch_out<R>(F32Cells{}, f, p, P, rows_in(P.y0, R, P.oy0, P.oy1), W, H, vec);
+  patch_out<R>(F32Cells{}, f, p, P, rows_in(P.y0, R, P.oy0, P.oy1), W, H, stage);
 }
 
 // Sweeps from `done` to the next exchange or, with 16-bit storage, the next
@@ -1230,7 +1296,7 @@ struct ProjectArgs {
 // together (a cooperative launch). The result is that of ceil(n / K) passes of
 // K sweeps through memory: with 16-bit storage the fields are rounded after
 // every K sweeps, and they end in the copy those passes would end in.
-template <int R, bool PRESSURE>
+template <int R, bool PRESSURE, bool ALIGNED>
 __global__ void __launch_bounds__(32 * project_max_warps(R), 1)
 k_project_tiles(const __grid_constant__ ProjectArgs a) {
   extern __shared__ __align__(16) char tile_smem[];
@@ -1240,11 +1306,11 @@ k_project_tiles(const __grid_constant__ ProjectArgs a) {
   const ProjSmem sm = project_smem_of(tile_smem, rows, a.g.warps, PRESSURE);
   const Link<4> link = open_link<4>(tile_smem, P, a.g);
   cluster_arrive();
-  const bool vec = ((W | a.g.halo) & 3) == 0;
+  float* const stage = ALIGNED ? nullptr : stage_of(tile_smem, a.g);
   ProjLane L;
   // The flags do not change after creation: staged before the wait for the
   // kernel before.
-  flags_in<R>(a.flags, P, sm, W, H, vec, L);
+  flags_in<R>(a.flags, P, sm, W, H, ALIGNED, L);
   pdl_entry();
   float u[R][8], v[R][8], vt[8];
 #pragma unroll
@@ -1253,17 +1319,18 @@ k_project_tiles(const __grid_constant__ ProjectArgs a) {
     for (int q = 0; q < 8; q++) u[r][q] = v[r][q] = 0.0f;
 #pragma unroll
   for (int q = 0; q < 8; q++) vt[q] = 0.0f;
-  if (PRESSURE) pressure_in<R>(sm, a.p, P, W, a.zero_pressure, H, vec);
   const float d_t = a.prm->dt;
   on_cells(a.storage, [&](auto io) {
     const void* vi = a.cv ? a.V1 : a.V0;
-    patch_in<R>(io, u, a.cu ? a.U1 : a.U0, P, W, H, vec);
-    patch_in<R>(io, v, vi, P, W, H, vec);
-    if (P.up) row_in(io, vt, vi, P, P.y0 + R, W, H, vec);
+    patch_in<R>(io, u, a.cu ? a.U1 : a.U0, P, W, H, stage);
+    patch_in<R>(io, v, vi, P, W, H, stage);
+    if (P.up) row_in(io, vt, vi, P, P.y0 + R, W, H, stage);
   });
   const unsigned epoch = a.n > a.D ? ld_acquire_gpu(a.sync.epochs + blockIdx.x) : 0u;
   unsigned number = epoch;
   if (a.n > a.D) exchange_plan(sm.exchange, a.g, R, 2, W, H);
+  // (Behind the faces, and with its own patch: ahead of them the sweeps spilled.)
+  if (PRESSURE) pressure_in<R>(sm, a.p, patch_of(a.g, R, W, H), W, a.zero_pressure, H, stage);
   cluster_wait();  // every inbox of the cluster is open
   unsigned message = 0;
 #pragma unroll 1
@@ -1287,11 +1354,12 @@ k_project_tiles(const __grid_constant__ ProjectArgs a) {
   }
   if (number != epoch && threadIdx.x == 0) a.sync.epochs[blockIdx.x] = number;
   const Patch Q = patch_of(a.g, R, W, H);
+  float* const out = ALIGNED ? nullptr : stage_of(tile_smem, a.g);
   // To the copies that ceil(n / K) passes through memory would end in.
   const bool swap = ((a.n + a.K - 1) / a.K) & 1;
   faces_out<R>(u, v, (a.cu != 0) != swap ? a.U1 : a.U0, (a.cv != 0) != swap ? a.V1 : a.V0,
-               a.storage, Q, W, H, vec, a.extrapolate != 0);
-  if (PRESSURE) pressure_out<R>(sm, a.p, Q, W, H, vec);
+               a.storage, Q, W, H, out, a.extrapolate != 0);
+  if (PRESSURE) pressure_out<R>(sm, a.p, Q, W, H, out);
   cluster_arrive();  // no CTA leaves while another may still send to it
   cluster_wait();
 }
@@ -1433,7 +1501,7 @@ struct DiffuseArgs {
 };
 
 // As k_project_tiles, with a halo of D cells.
-template <int R>
+template <int R, bool ALIGNED>
 __global__ void __launch_bounds__(32 * diffuse_max_warps(R), 1)
 k_diffuse_tiles(const __grid_constant__ DiffuseArgs a) {
   extern __shared__ __align__(16) char tile_smem[];
@@ -1442,14 +1510,14 @@ k_diffuse_tiles(const __grid_constant__ DiffuseArgs a) {
   const Patch P = patch_of(a.g, R, W, H);
   const Link<8> link = open_link<8>(tile_smem, P, a.g);
   cluster_arrive();
-  const bool vec = ((W | a.g.halo) & 3) == 0;
+  float* const stage = ALIGNED ? nullptr : stage_of(tile_smem, a.g);
   pdl_entry();
   float u[R][8], none[8];
 #pragma unroll
   for (int r = 0; r < R; r++)
 #pragma unroll
     for (int q = 0; q < 8; q++) u[r][q] = 0.0f;
-  on_cells(a.storage, [&](auto io) { patch_in<R>(io, u, a.cu ? a.U1 : a.U0, P, W, H, vec); });
+  on_cells(a.storage, [&](auto io) { patch_in<R>(io, u, a.cu ? a.U1 : a.U0, P, W, H, stage); });
   const DiffLane L = diff_lane(P, R, W, H);
   const float coeff = diffusion_coeff<float>(c, a.prm->dt);
   const unsigned epoch = a.n > a.D ? ld_acquire_gpu(a.sync.epochs + blockIdx.x) : 0u;
@@ -1476,8 +1544,9 @@ k_diffuse_tiles(const __grid_constant__ DiffuseArgs a) {
   const bool swap = ((a.n + a.K - 1) / a.K) & 1;
   void* uo = (a.cu != 0) != swap ? a.U1 : a.U0;
   const Patch Q = patch_of(a.g, R, W, H);
+  float* const out = ALIGNED ? nullptr : stage_of(tile_smem, a.g);
   on_cells(a.storage, [&](auto io) {
-    patch_out<R>(io, u, uo, Q, rows_in(Q.y0, R, Q.oy0, Q.oy1), W, H, vec);
+    patch_out<R>(io, u, uo, Q, rows_in(Q.y0, R, Q.oy0, Q.oy1), W, H, out);
   });
   cluster_arrive();  // no CTA leaves while another may still send to it
   cluster_wait();
@@ -1488,7 +1557,7 @@ using DiffuseKernel = void (*)(const DiffuseArgs);
 
 // The kernels of one strip height, each instantiated in a translation unit of
 // its own (os_tile_project.cu, os_tile_diffuse.cu).
-template <int R> ProjectKernel project_kernel(bool pressure);
-template <int R> DiffuseKernel diffuse_kernel();
+template <int R> ProjectKernel project_kernel(bool pressure, bool aligned);
+template <int R> DiffuseKernel diffuse_kernel(bool aligned);
 
 }  // namespace osg

@@ -39,7 +39,7 @@ k_batch_project_tiles(const PlanHeader* __restrict__ plan, const int* __restrict
     const TilePlace place{t.tx, t.ty, d.proj_tiles_x, d.proj_tiles_y};
     const int sweeps = min(K, c.n - pass * K);
     const int iu = (d.diff_passes + pass) & 1, iv = pass & 1;
-    const bool vec = ((W | g.halo) & 3) == 0;
+    float* const stage = quads_aligned(W, g.halo) ? nullptr : stage_of(tile_smem, g);
     float u[R][8], v[R][8], vt[8];
 #pragma unroll
     for (int r = 0; r < R; r++)
@@ -54,20 +54,21 @@ k_batch_project_tiles(const PlanHeader* __restrict__ plan, const int* __restrict
       const Patch P = patch_at(place, g, R, W, H);
       cell0 = P.yl * 64 + P.lane;
       down = P.down;
-      flags_in<R>(d.flags, P, sm, W, H, vec, L);
+      flags_in<R>(d.flags, P, sm, W, H, !stage, L);
       const void* vi = iv ? d.vb : d.v;
       if (!P.idle)
         on_cells(d.storage, [&](auto io) {
-          patch_in<R>(io, u, iu ? d.ub : d.u, P, W, H, vec);
-          patch_in<R>(io, v, vi, P, W, H, vec);
-          if (P.up) row_in(io, vt, vi, P, P.y0 + R, W, H, vec);
+          patch_in<R>(io, u, iu ? d.ub : d.u, P, W, H, stage);
+          patch_in<R>(io, v, vi, P, W, H, stage);
+          if (P.up) row_in(io, vt, vi, P, P.y0 + R, W, H, stage);
         });
     }
     tile_sweeps<false, R>(u, v, vt, L, sm, link, sync, cell0, down, c, 0.0f, sweeps, message);
     message += project_messages(sweeps);
     const Patch P = patch_at(place, g, R, W, H);
+    float* const out = quads_aligned(W, g.halo) ? nullptr : stage_of(tile_smem, g);
     if (!P.idle)
-      faces_out<R>(u, v, iu ? d.u : d.ub, iv ? d.v : d.vb, d.storage, P, W, H, vec,
+      faces_out<R>(u, v, iu ? d.u : d.ub, iv ? d.v : d.vb, d.storage, P, W, H, out,
                    pass + 1 == d.proj_passes);
   }
   cluster_arrive();  // no CTA leaves while another may still send to it
@@ -95,7 +96,7 @@ k_batch_diffuse_tiles(const PlanHeader* __restrict__ plan, const int* __restrict
     const int W = d.c.W, H = d.c.H;
     const TilePlace place{t.tx, t.ty, d.diff_tiles_x, d.diff_tiles_y};
     const int sweeps = min(K, d.c.n - pass * K);
-    const bool vec = ((W | g.halo) & 3) == 0;
+    float* const stage = quads_aligned(W, g.halo) ? nullptr : stage_of(tile_smem, g);
     float u[R][8];
 #pragma unroll
     for (int r = 0; r < R; r++)
@@ -107,14 +108,15 @@ k_batch_diffuse_tiles(const PlanHeader* __restrict__ plan, const int* __restrict
       L = diff_lane(P, R, W, H);
       if (!P.idle)
         on_cells(d.storage,
-                 [&](auto io) { patch_in<R>(io, u, pass & 1 ? d.ub : d.u, P, W, H, vec); });
+                 [&](auto io) { patch_in<R>(io, u, pass & 1 ? d.ub : d.u, P, W, H, stage); });
     }
     jacobi_sweeps<R>(u, L, link, sync, diffusion_coeff<float>(d.c, d.prm->dt), sweeps, message);
     message += sweeps;
     const Patch P = patch_at(place, g, R, W, H);
+    float* const out = quads_aligned(W, g.halo) ? nullptr : stage_of(tile_smem, g);
     if (!P.idle)
       on_cells(d.storage, [&](auto io) {
-        patch_out<R>(io, u, pass & 1 ? d.u : d.ub, P, rows_in(P.y0, R, P.oy0, P.oy1), W, H, vec);
+        patch_out<R>(io, u, pass & 1 ? d.u : d.ub, P, rows_in(P.y0, R, P.oy0, P.oy1), W, H, out);
       });
   }
   cluster_arrive();

@@ -3,7 +3,7 @@
 
 namespace osg {
 template <>
-DiffuseKernel diffuse_kernel<OS_TILE_ROWS>() {
-  return k_diffuse_tiles<OS_TILE_ROWS>;
+DiffuseKernel diffuse_kernel<OS_TILE_ROWS>(bool aligned) {
+  return aligned ? k_diffuse_tiles<OS_TILE_ROWS, true> : k_diffuse_tiles<OS_TILE_ROWS, false>;
 }
 }  // namespace osg

@@ -6,33 +6,33 @@
 
 namespace osg {
 
-template <> ProjectKernel project_kernel<2>(bool);
-template <> ProjectKernel project_kernel<4>(bool);
-template <> ProjectKernel project_kernel<6>(bool);
-template <> ProjectKernel project_kernel<8>(bool);
-template <> ProjectKernel project_kernel<10>(bool);
-template <> DiffuseKernel diffuse_kernel<2>();
-template <> DiffuseKernel diffuse_kernel<4>();
-template <> DiffuseKernel diffuse_kernel<6>();
-template <> DiffuseKernel diffuse_kernel<8>();
-template <> DiffuseKernel diffuse_kernel<12>();
+template <> ProjectKernel project_kernel<2>(bool, bool);
+template <> ProjectKernel project_kernel<4>(bool, bool);
+template <> ProjectKernel project_kernel<6>(bool, bool);
+template <> ProjectKernel project_kernel<8>(bool, bool);
+template <> ProjectKernel project_kernel<10>(bool, bool);
+template <> DiffuseKernel diffuse_kernel<2>(bool);
+template <> DiffuseKernel diffuse_kernel<4>(bool);
+template <> DiffuseKernel diffuse_kernel<6>(bool);
+template <> DiffuseKernel diffuse_kernel<8>(bool);
+template <> DiffuseKernel diffuse_kernel<12>(bool);
 
-inline ProjectKernel project_kernel_of(int R, bool pressure) {
+inline ProjectKernel project_kernel_of(int R, bool pressure, bool aligned) {
   switch (R) {
-    case 2: return project_kernel<2>(pressure);
-    case 4: return project_kernel<4>(pressure);
-    case 6: return project_kernel<6>(pressure);
-    case 8: return project_kernel<8>(pressure);
-    default: return project_kernel<10>(pressure);
+    case 2: return project_kernel<2>(pressure, aligned);
+    case 4: return project_kernel<4>(pressure, aligned);
+    case 6: return project_kernel<6>(pressure, aligned);
+    case 8: return project_kernel<8>(pressure, aligned);
+    default: return project_kernel<10>(pressure, aligned);
   }
 }
-inline DiffuseKernel diffuse_kernel_of(int R) {
+inline DiffuseKernel diffuse_kernel_of(int R, bool aligned) {
   switch (R) {
-    case 2: return diffuse_kernel<2>();
-    case 4: return diffuse_kernel<4>();
-    case 6: return diffuse_kernel<6>();
-    case 8: return diffuse_kernel<8>();
-    default: return diffuse_kernel<12>();
+    case 2: return diffuse_kernel<2>(aligned);
+    case 4: return diffuse_kernel<4>(aligned);
+    case 6: return diffuse_kernel<6>(aligned);
+    case 8: return diffuse_kernel<8>(aligned);
+    default: return diffuse_kernel<12>(aligned);
   }
 }
 
@@ -76,7 +76,7 @@ inline int resident_clusters(int device, int cluster, int ctas) {
   const auto key = std::make_tuple(device, cluster, ctas);
   auto it = known.find(key);
   if (it != known.end()) return it->second;
-  const auto kernel = diffuse_kernel<2>();
+  const auto kernel = diffuse_kernel<2>(true);
   const size_t smem = (227 / ctas - 1) * 1024;  // as much as leaves room for no more CTAs
   int n = 0;
   if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) ==
@@ -129,6 +129,7 @@ inline double choose_tile(int W, int H, int D, bool projection, bool pressure, b
         g.smem = projection
                      ? project_tile_smem(rows, warps, pressure, g.halo, resident && !one)
                      : diffuse_tile_smem(rows, warps, g.halo, resident && !one);
+        g.smem += stage_smem(W, g.halo, warps);
         if (g.smem + kStaticSmem > kMaxSmem) continue;
         // Pass by pass, several CTAs share an SM: over three waves or more they
         // drift apart, and one loads and stores beside the other's sweeps (in
@@ -281,7 +282,7 @@ inline int enqueue_tiled_projection(os_handle* h, cudaStream_t st, int* cur_u, i
     a.zero_pressure = zero_first;
     a.extrapolate = extrapolate;
     if (passes > 0 &&
-        launch_tiles(project_kernel_of(a.g.R, pressure), a, a.g, n > a.D, h->pdl, st) !=
+        launch_tiles(project_kernel_of(a.g.R, pressure, quads_aligned(h->W, a.g.halo)), a, a.g, n > a.D, h->pdl, st) !=
             cudaSuccess)
       return -1;
     launches = passes > 0;
@@ -294,7 +295,7 @@ inline int enqueue_tiled_projection(os_handle* h, cudaStream_t st, int* cur_u, i
       a.cu = (*cur_u + p) & 1, a.cv = (*cur_v + p) & 1;
       a.zero_pressure = zero_first && p == 0;
       a.extrapolate = extrapolate && p == passes - 1;
-      if (launch_tiles(project_kernel_of(a.g.R, pressure), a, a.g, false, h->pdl, st) !=
+      if (launch_tiles(project_kernel_of(a.g.R, pressure, quads_aligned(h->W, a.g.halo)), a, a.g, false, h->pdl, st) !=
           cudaSuccess)
         return -1;
     }
@@ -321,7 +322,7 @@ inline int enqueue_tiled_diffusion(os_handle* h, cudaStream_t st, int* cur_u) {
     if (!(a.D = phase_tile(h, false, K, true, &a.g))) return -1;
     a.n = n;
     a.cu = *cur_u;
-    if (passes > 0 && launch_tiles(diffuse_kernel_of(a.g.R), a, a.g, n > a.D, h->pdl, st) !=
+    if (passes > 0 && launch_tiles(diffuse_kernel_of(a.g.R, quads_aligned(h->W, a.g.halo)), a, a.g, n > a.D, h->pdl, st) !=
                           cudaSuccess)
       return -1;
     launches = passes > 0;
@@ -330,7 +331,7 @@ inline int enqueue_tiled_diffusion(os_handle* h, cudaStream_t st, int* cur_u) {
     for (int p = 0; p < passes; p++, launches++) {
       a.n = std::min(K, n - p * K);
       a.cu = (*cur_u + p) & 1;
-      if (launch_tiles(diffuse_kernel_of(a.g.R), a, a.g, false, h->pdl, st) != cudaSuccess)
+      if (launch_tiles(diffuse_kernel_of(a.g.R, quads_aligned(h->W, a.g.halo)), a, a.g, false, h->pdl, st) != cudaSuccess)
         return -1;
     }
   }

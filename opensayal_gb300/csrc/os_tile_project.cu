@@ -4,7 +4,11 @@
 
 namespace osg {
 template <>
-ProjectKernel project_kernel<OS_TILE_ROWS>(bool pressure) {
-  return pressure ? k_project_tiles<OS_TILE_ROWS, true> : k_project_tiles<OS_TILE_ROWS, false>;
+ProjectKernel project_kernel<OS_TILE_ROWS>(bool pressure, bool aligned) {
+  if (aligned)
+    return pressure ? k_project_tiles<OS_TILE_ROWS, true, true>
+                    : k_project_tiles<OS_TILE_ROWS, false, true>;
+  return pressure ? k_project_tiles<OS_TILE_ROWS, true, false>
+                  : k_project_tiles<OS_TILE_ROWS, false, false>;
 }
 }  // namespace osg

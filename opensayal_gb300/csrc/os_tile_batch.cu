@@ -5,7 +5,7 @@
 // Bound by the sweeps' instructions and by the faces' way from strip to strip;
 // the loads and stores of one tile run beside the sweeps of the other on the
 // SM. 21 tunnels of 128 to 1024 cells a side (6.85 M cells in all): a step
-// takes 2079 us, and took 2968 us with tiles held in shared memory; 6 tunnels
+// takes 2035 us, and took 2968 us with tiles held in shared memory; 6 tunnels
 // of mixed storage 2036 us, and 3378 us.
 #include "os_batch_plan.cuh"
 

@@ -1277,8 +1277,8 @@ __device__ __forceinline__ int tile_segment(int n, int K, int D, int done, int s
 }
 
 struct ProjectArgs {
-  void *U0, *U1, *V0, *V1;  // the two copies of the fields
-  int cu, cv;               // which of them holds the input
+  const void *ui, *vi;      // the copies of the fields that are loaded
+  void *uo, *vo;            // the other copies, which take the result
   int storage;
   float* p;
   const uint8_t* flags;
@@ -1295,7 +1295,9 @@ struct ProjectArgs {
 // and the launch may hold any number of tiles; else all tiles must be resident
 // together (a cooperative launch). The result is that of ceil(n / K) passes of
 // K sweeps through memory: with 16-bit storage the fields are rounded after
-// every K sweeps, and they end in the copy those passes would end in.
+// every K sweeps. It goes to the other copy of the fields, however many passes
+// that stands for: nothing orders a tile's stores behind the loads of the halos
+// of the tiles around it (they may not have started yet).
 template <int R, bool PRESSURE, bool ALIGNED>
 __global__ void __launch_bounds__(32 * project_max_warps(R), 1)
 k_project_tiles(const __grid_constant__ ProjectArgs a) {
@@ -1321,10 +1323,9 @@ k_project_tiles(const __grid_constant__ ProjectArgs a) {
   for (int q = 0; q < 8; q++) vt[q] = 0.0f;
   const float d_t = a.prm->dt;
   on_cells(a.storage, [&](auto io) {
-    const void* vi = a.cv ? a.V1 : a.V0;
-    patch_in<R>(io, u, a.cu ? a.U1 : a.U0, P, W, H, stage);
-    patch_in<R>(io, v, vi, P, W, H, stage);
-    if (P.up) row_in(io, vt, vi, P, P.y0 + R, W, H, stage);
+    patch_in<R>(io, u, a.ui, P, W, H, stage);
+    patch_in<R>(io, v, a.vi, P, W, H, stage);
+    if (P.up) row_in(io, vt, a.vi, P, P.y0 + R, W, H, stage);
   });
   const unsigned epoch = a.n > a.D ? ld_acquire_gpu(a.sync.epochs + blockIdx.x) : 0u;
   unsigned number = epoch;
@@ -1355,10 +1356,7 @@ k_project_tiles(const __grid_constant__ ProjectArgs a) {
   if (number != epoch && threadIdx.x == 0) a.sync.epochs[blockIdx.x] = number;
   const Patch Q = patch_of(a.g, R, W, H);
   float* const out = ALIGNED ? nullptr : stage_of(tile_smem, a.g);
-  // To the copies that ceil(n / K) passes through memory would end in.
-  const bool swap = ((a.n + a.K - 1) / a.K) & 1;
-  faces_out<R>(u, v, (a.cu != 0) != swap ? a.U1 : a.U0, (a.cv != 0) != swap ? a.V1 : a.V0,
-               a.storage, Q, W, H, out, a.extrapolate != 0);
+  faces_out<R>(u, v, a.uo, a.vo, a.storage, Q, W, H, out, a.extrapolate != 0);
   if (PRESSURE) pressure_out<R>(sm, a.p, Q, W, H, out);
   cluster_arrive();  // no CTA leaves while another may still send to it
   cluster_wait();
@@ -1490,8 +1488,8 @@ __device__ __forceinline__ void jacobi_sweeps(float (&u)[R][8], const DiffLane& 
 }
 
 struct DiffuseArgs {
-  void *U0, *U1;  // the two copies of the field
-  int cu;         // which of them holds the input
+  const void* ui;  // the copy of the field that is loaded
+  void* uo;        // the other copy, which takes the result
   int storage;
   Consts c;
   const StepParams* prm;
@@ -1517,7 +1515,7 @@ k_diffuse_tiles(const __grid_constant__ DiffuseArgs a) {
   for (int r = 0; r < R; r++)
 #pragma unroll
     for (int q = 0; q < 8; q++) u[r][q] = 0.0f;
-  on_cells(a.storage, [&](auto io) { patch_in<R>(io, u, a.cu ? a.U1 : a.U0, P, W, H, stage); });
+  on_cells(a.storage, [&](auto io) { patch_in<R>(io, u, a.ui, P, W, H, stage); });
   const DiffLane L = diff_lane(P, R, W, H);
   const float coeff = diffusion_coeff<float>(c, a.prm->dt);
   const unsigned epoch = a.n > a.D ? ld_acquire_gpu(a.sync.epochs + blockIdx.x) : 0u;
@@ -1541,12 +1539,10 @@ k_diffuse_tiles(const __grid_constant__ DiffuseArgs a) {
     done += sweeps;
   }
   if (number != epoch && threadIdx.x == 0) a.sync.epochs[blockIdx.x] = number;
-  const bool swap = ((a.n + a.K - 1) / a.K) & 1;
-  void* uo = (a.cu != 0) != swap ? a.U1 : a.U0;
   const Patch Q = patch_of(a.g, R, W, H);
   float* const out = ALIGNED ? nullptr : stage_of(tile_smem, a.g);
   on_cells(a.storage, [&](auto io) {
-    patch_out<R>(io, u, uo, Q, rows_in(Q.y0, R, Q.oy0, Q.oy1), W, H, out);
+    patch_out<R>(io, u, a.uo, Q, rows_in(Q.y0, R, Q.oy0, Q.oy1), W, H, out);
   });
   cluster_arrive();  // no CTA leaves while another may still send to it
   cluster_wait();

@@ -216,8 +216,8 @@ inline cudaError_t launch_tiles(void (*kernel)(const Args), const Args& a, const
 
 // The resident forms' tiles, all of one launch resident together, and the
 // sweeps between their exchanges (n when one tile is the whole grid). block_k
-// is not their depth: it says which copy the fields end in and, with 16-bit
-// storage, how often they are rounded. 0 when the grid does not fit.
+// is not their depth: it says how often 16-bit fields are rounded. 0 when the
+// grid does not fit.
 inline int resident_tile(const os_handle* h, bool projection, RegTile* g) {
   const bool pressure = h->cfg.enable_pressure != 0;
   const int K = h->block_k, n = std::max(h->c.n, 1);
@@ -257,7 +257,7 @@ inline int phase_tile(os_handle* h, bool projection, int K, bool resident, RegTi
 
 // The projection phase: one launch for all its passes (resident), or one per
 // pass of block_k sweeps. `cur_u` / `cur_v` say which copy holds the live
-// field (0: u, v; 1: ub, vb) and advance by the passes. `extrapolate`: the
+// field (0: u, v; 1: ub, vb); each launch moves it to the other. `extrapolate`: the
 // last pass applies the extrapolation that follows in a step. Returns the
 // launches, or -1.
 inline int enqueue_tiled_projection(os_handle* h, cudaStream_t st, int* cur_u, int* cur_v,
@@ -265,7 +265,7 @@ inline int enqueue_tiled_projection(os_handle* h, cudaStream_t st, int* cur_u, i
   const int K = h->block_k, n = h->c.n;
   const bool pressure = h->cfg.enable_pressure != 0;
   ProjectArgs a{};
-  a.U0 = h->u, a.U1 = h->ub, a.V0 = h->v, a.V1 = h->vb;
+  void *const U[2] = {h->u, h->ub}, *const V[2] = {h->v, h->vb};
   a.storage = h->storage;
   a.p = h->p;
   a.flags = h->flags;
@@ -278,7 +278,8 @@ inline int enqueue_tiled_projection(os_handle* h, cudaStream_t st, int* cur_u, i
   if (h->resident) {
     if (!(a.D = phase_tile(h, true, K, true, &a.g))) return -1;
     a.n = n;
-    a.cu = *cur_u, a.cv = *cur_v;
+    a.ui = U[*cur_u], a.uo = U[1 - *cur_u];
+    a.vi = V[*cur_v], a.vo = V[1 - *cur_v];
     a.zero_pressure = zero_first;
     a.extrapolate = extrapolate;
     if (passes > 0 &&
@@ -292,7 +293,9 @@ inline int enqueue_tiled_projection(os_handle* h, cudaStream_t st, int* cur_u, i
       return -1;
     for (int p = 0; p < passes; p++, launches++) {
       a.n = std::min(K, n - p * K);
-      a.cu = (*cur_u + p) & 1, a.cv = (*cur_v + p) & 1;
+      const int cu = (*cur_u + p) & 1, cv = (*cur_v + p) & 1;
+      a.ui = U[cu], a.uo = U[1 - cu];
+      a.vi = V[cv], a.vo = V[1 - cv];
       a.zero_pressure = zero_first && p == 0;
       a.extrapolate = extrapolate && p == passes - 1;
       if (launch_tiles(project_kernel_of(a.g.R, pressure, quads_aligned(h->W, a.g.halo)), a, a.g, false, h->pdl, st) !=
@@ -300,8 +303,8 @@ inline int enqueue_tiled_projection(os_handle* h, cudaStream_t st, int* cur_u, i
         return -1;
     }
   }
-  *cur_u = (*cur_u + passes) & 1;
-  *cur_v = (*cur_v + passes) & 1;
+  *cur_u = (*cur_u + launches) & 1;
+  *cur_v = (*cur_v + launches) & 1;
   return launches;
 }
 
@@ -310,7 +313,7 @@ inline int enqueue_tiled_projection(os_handle* h, cudaStream_t st, int* cur_u, i
 inline int enqueue_tiled_diffusion(os_handle* h, cudaStream_t st, int* cur_u) {
   const int K = h->resident_diff ? h->block_k : diffusion_depth(h), n = h->c.n;
   DiffuseArgs a{};
-  a.U0 = h->u, a.U1 = h->ub;
+  void* const U[2] = {h->u, h->ub};
   a.storage = h->storage;
   a.c = h->c;
   a.prm = h->d_params;
@@ -321,7 +324,7 @@ inline int enqueue_tiled_diffusion(os_handle* h, cudaStream_t st, int* cur_u) {
   if (h->resident_diff) {
     if (!(a.D = phase_tile(h, false, K, true, &a.g))) return -1;
     a.n = n;
-    a.cu = *cur_u;
+    a.ui = U[*cur_u], a.uo = U[1 - *cur_u];
     if (passes > 0 && launch_tiles(diffuse_kernel_of(a.g.R, quads_aligned(h->W, a.g.halo)), a, a.g, n > a.D, h->pdl, st) !=
                           cudaSuccess)
       return -1;
@@ -330,12 +333,13 @@ inline int enqueue_tiled_diffusion(os_handle* h, cudaStream_t st, int* cur_u) {
     if (!(a.D = phase_tile(h, false, K, false, &a.g))) return -1;
     for (int p = 0; p < passes; p++, launches++) {
       a.n = std::min(K, n - p * K);
-      a.cu = (*cur_u + p) & 1;
+      const int cu = (*cur_u + p) & 1;
+      a.ui = U[cu], a.uo = U[1 - cu];
       if (launch_tiles(diffuse_kernel_of(a.g.R, quads_aligned(h->W, a.g.halo)), a, a.g, false, h->pdl, st) != cudaSuccess)
         return -1;
     }
   }
-  *cur_u = (*cur_u + passes) & 1;
+  *cur_u = (*cur_u + launches) & 1;
   return launches;
 }
 

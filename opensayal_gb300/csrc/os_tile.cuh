@@ -727,6 +727,10 @@ __device__ __forceinline__ void exchange(float (&f)[R][8], float (&f2)[R][8], fl
   const int64_t plane = packet_plane(W, H);
   constexpr int kPer = kPacketsPerQuad<FIELDS>;
   uint4* packets = sync.packets + (number & 1) * kPer * plane;
+  // The band takes words that the last exchange's ring may still be read from:
+  // a warp can be as many sweeps ahead of another as there are strips between
+  // them, which may be more than lie between two exchanges.
+  __syncthreads();
   {
     const Patch P = patch_of(g, R, W, H);
     exchange_patch<FIELDS, true, R>(f, f2, f_top, exchange_view(base, P, g, FIELDS), P, g);

@@ -72,17 +72,24 @@ BatchTileKernel batch_project_kernel() { return known(fake_batch<0>, kBatchProje
 BatchTileKernel batch_diffuse_kernel() { return known(fake_batch<1>, kBatchDiffuse); }
 }  // namespace osg
 
+void describe_tile(const osg::RegTile& g, HostLaunch* l) {
+  l->tiles = g.tiles_x * g.tiles_y, l->tiles_y = g.tiles_y;
+  l->R = g.R, l->warps = g.warps, l->halo = g.halo;
+}
+
 // The arguments of a launch of these kernels.
 extern "C" void host_describe(const void* fn, void** args, HostLaunch* l) {
   for (const FakeKernel& k : fake_kernels())
     if (k.fn == fn) l->kind = k.kind;
   if (l->kind == kProject) {
     const auto& a = *static_cast<const osg::ProjectArgs*>(args[0]);
-    l->n = a.n, l->K = a.K, l->D = a.D, l->tiles = a.g.tiles_x * a.g.tiles_y;
+    l->n = a.n, l->K = a.K, l->D = a.D;
+    describe_tile(a.g, l);
     l->ui = a.ui, l->vi = a.vi, l->uo = a.uo, l->vo = a.vo;
   } else if (l->kind == kDiffuse) {
     const auto& a = *static_cast<const osg::DiffuseArgs*>(args[0]);
-    l->n = a.n, l->K = a.K, l->D = a.D, l->tiles = a.g.tiles_x * a.g.tiles_y;
+    l->n = a.n, l->K = a.K, l->D = a.D;
+    describe_tile(a.g, l);
     l->ui = a.ui, l->uo = a.uo;
   }
 }

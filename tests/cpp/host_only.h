@@ -9,7 +9,8 @@ extern "C" {
 enum HostKind { kOther, kProject, kDiffuse, kBatchProject, kBatchDiffuse };
 struct HostLaunch {
   int32_t kind, tiles, cluster, cooperative, pdl;
-  int32_t n, K, D;       // tile kernels of a single grid, as the copies below
+  int32_t n, K, D;       // tile kernels of a single grid, as what follows
+  int32_t R, warps, halo, tiles_y;
   uint64_t smem, limit;  // dynamic shared memory, and the limit set for the kernel
   const void *fn, *ui, *vi, *uo, *vo;
 };

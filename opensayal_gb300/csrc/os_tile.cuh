@@ -370,7 +370,10 @@ __device__ __forceinline__ void idle_messages(const Link<WORDS>& link, unsigned 
 // exchange between from every neighbouring tile, whose CTAs sent it after their
 // reads of this one: a CTA sends behind its own barrier, and the CTAs of a
 // tile whose rows lie within a halo of each other have since exchanged
-// messages in the sweeps between, as many strips far as a halo has rows.
+// messages in the sweeps between. Those reach a strip further each, and two
+// exchanges lie D sweeps apart: at least D messages of the diffusion, whose halo
+// of D cells is D / R strips high, and 2 D + 1 of the projection, whose halo has
+// 2 D cells (R is at least 2, one strip more for the row that a strip starts in).
 // ---------------------------------------------------------------------------
 constexpr int kSpinLimit = 1 << 20;  // polls per wait
 
@@ -1135,7 +1138,7 @@ __device__ __forceinline__ void sweep_loop(float (&u)[R][8], float (&v)[R][8], f
 }
 
 // Messages of a segment of sweeps.
-__device__ __forceinline__ unsigned project_messages(int sweeps) { return 2 * sweeps + 1; }
+__host__ __device__ inline unsigned project_messages(int sweeps) { return 2 * sweeps + 1; }
 
 // `sweeps` red/black sweeps of the region, messages m .. m + 2 sweeps. Every
 // cell of the region is updated: validity shrinks by one cell per half-sweep
@@ -1273,11 +1276,24 @@ __device__ __forceinline__ void pressure_out(const ProjSmem& sm, float* p, const
   patch_out<R>(F32Cells{}, f, p, P, rows_in(P.y0, R, P.oy0, P.oy1), W, H, stage);
 }
 
-// Sweeps from `done` to the next exchange or, with 16-bit storage, the next
-// rounding.
-__device__ __forceinline__ int tile_segment(int n, int K, int D, int done, int storage) {
-  const int left = min(D, n - done);
-  return storage == OS_STORAGE_F32 ? left : min(left, K - done % K);
+// The sweeps from `done` on that run without a break, and what comes before
+// them: with 16-bit storage the rounding after every K sweeps, and in a launch
+// that exchanges (n > D) the ring after every D. A rounding needs no exchange: a
+// tile rounds its copies of its neighbours' cells as they round theirs, and the
+// halo is as wide as D sweeps need. (With an exchange at each rounding, K = 4 and
+// D = 20 left 4 messages between two exchanges, and halos of 10 strips.)
+struct Segment {
+  int sweeps;
+  bool round, exchange;
+};
+__host__ __device__ inline Segment segment_at(int n, int K, int D, int done, int storage) {
+  const bool rounded = storage != OS_STORAGE_F32;
+  Segment s;
+  s.sweeps = n - done < D - done % D ? n - done : D - done % D;
+  if (rounded && K - done % K < s.sweeps) s.sweeps = K - done % K;
+  s.round = rounded && done > 0 && done % K == 0;
+  s.exchange = n > D && done > 0 && done % D == 0;
+  return s;
 }
 
 struct ProjectArgs {
@@ -1340,22 +1356,20 @@ k_project_tiles(const __grid_constant__ ProjectArgs a) {
   unsigned message = 0;
 #pragma unroll 1
   for (int done = 0; done < a.n;) {
-    if (done > 0) {
-      if (a.storage != OS_STORAGE_F32 && done % a.K == 0) {
-        round_patch<R>(u, a.storage);
-        round_patch<R>(v, a.storage);
-        round_row(vt, a.storage);
-      }
-      if (a.n > a.D) {
-        number++;
-        exchange<2, R>(u, v, vt, sm.exchange, a.sync, a.g, W, H, number);
-      }
+    const Segment s = segment_at(a.n, a.K, a.D, done, a.storage);
+    if (s.round) {
+      round_patch<R>(u, a.storage);
+      round_patch<R>(v, a.storage);
+      round_row(vt, a.storage);
     }
-    const int sweeps = tile_segment(a.n, a.K, a.D, done, a.storage);
+    if (s.exchange) {
+      number++;
+      exchange<2, R>(u, v, vt, sm.exchange, a.sync, a.g, W, H, number);
+    }
     tile_sweeps<PRESSURE, R>(u, v, vt, L, sm, link, a.sync, P.yl * 64 + P.lane, P.down, c, d_t,
-                             sweeps, message);
-    message += project_messages(sweeps);
-    done += sweeps;
+                             s.sweeps, message);
+    message += project_messages(s.sweeps);
+    done += s.sweeps;
   }
   if (number != epoch && threadIdx.x == 0) a.sync.epochs[blockIdx.x] = number;
   const Patch Q = patch_of(a.g, R, W, H);
@@ -1529,18 +1543,16 @@ k_diffuse_tiles(const __grid_constant__ DiffuseArgs a) {
   unsigned message = 0;
 #pragma unroll 1
   for (int done = 0; done < a.n;) {
-    if (done > 0) {
-      if (a.storage != OS_STORAGE_F32 && done % a.K == 0) round_patch<R>(u, a.storage);
-      if (a.n > a.D) {
-        number++;
-        exchange<1, R>(u, u, none, tile_smem + a.g.warps * inbox_bytes(8), a.sync, a.g, W, H,
-                       number);
-      }
+    const Segment s = segment_at(a.n, a.K, a.D, done, a.storage);
+    if (s.round) round_patch<R>(u, a.storage);
+    if (s.exchange) {
+      number++;
+      exchange<1, R>(u, u, none, tile_smem + a.g.warps * inbox_bytes(8), a.sync, a.g, W, H,
+                     number);
     }
-    const int sweeps = tile_segment(a.n, a.K, a.D, done, a.storage);
-    jacobi_sweeps<R>(u, L, link, a.sync, coeff, sweeps, message);
-    message += sweeps;
-    done += sweeps;
+    jacobi_sweeps<R>(u, L, link, a.sync, coeff, s.sweeps, message);
+    message += s.sweeps;
+    done += s.sweeps;
   }
   if (number != epoch && threadIdx.x == 0) a.sync.epochs[blockIdx.x] = number;
   const Patch Q = patch_of(a.g, R, W, H);

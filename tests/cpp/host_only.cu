@@ -93,3 +93,18 @@ extern "C" void host_describe(const void* fn, void** args, HostLaunch* l) {
     l->ui = a.ui, l->uo = a.uo;
   }
 }
+
+extern "C" int32_t host_segment(int32_t projection, int32_t n, int32_t K, int32_t D,
+                                int32_t storage, int32_t k, int32_t* messages, int32_t* round,
+                                int32_t* exchange) {
+  for (int done = 0; done < n; k--) {
+    const osg::Segment s = osg::segment_at(n, K, D, done, storage);
+    if (k == 0) {
+      *messages = projection ? osg::project_messages(s.sweeps) : s.sweeps;
+      *round = s.round, *exchange = s.exchange;
+      return s.sweeps;
+    }
+    done += s.sweeps;
+  }
+  return 0;
+}

@@ -22,6 +22,10 @@ struct HostState {
 };
 
 void host_describe(const void* fn, void** args, HostLaunch* l);
+// Segment k of a phase of n sweeps (segment_at): its sweeps and the messages that
+// they take, and whether a rounding and an exchange come first. 0: there is none.
+int32_t host_segment(int32_t projection, int32_t n, int32_t K, int32_t D, int32_t storage,
+                     int32_t k, int32_t* messages, int32_t* round, int32_t* exchange);
 // The launches since the last call, `cap` at most; returns their number.
 int32_t host_launches(HostLaunch* out, int32_t cap);
 extern HostState host_state;

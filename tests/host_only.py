@@ -66,6 +66,18 @@ def launches(lib, *kinds):
     return [x for x in buf[:n] if not kinds or x.kind in kinds]
 
 
+def segments(lib, x, storage):
+    """The segments of sweeps of tile launch x: (sweeps, messages, round, exchange)."""
+    out = []
+    while True:
+        more = [C.c_int32() for _ in range(3)]
+        sweeps = lib.host_segment(x.kind == PROJECT, x.n, x.K, x.D, storage, len(out),
+                                  *map(C.byref, more))
+        if not sweeps:
+            return out
+        out.append((sweeps, *(m.value for m in more)))
+
+
 class Handle:
     """A tunnel of the host-only library."""
 

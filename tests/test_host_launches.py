@@ -3,7 +3,7 @@ makes: no GPU needed."""
 import pytest
 
 from opensayal_gb300 import native
-from tests.host_only import DIFFUSE, PROJECT, Handle, launches, load, tunnel
+from tests.host_only import DIFFUSE, PROJECT, Handle, launches, load, segments, tunnel
 
 
 @pytest.fixture(scope="module")
@@ -36,3 +36,37 @@ def test_no_launch_stores_to_the_copy_it_loads(lib, w, h, k, resident, storage):
                 if x.kind == PROJECT:
                     assert x.vi == live and x.vo != x.vi, n
                     live = x.vo
+
+
+@pytest.mark.parametrize("w,h", [(333, 187), (571, 157), (640, 448), (800, 400), (1003, 771),
+                                 (1280, 720), (1920, 1080)])
+@pytest.mark.parametrize("k", [2, 4, 6, 8, 12])
+@pytest.mark.parametrize("storage", [native.STORAGE_F32, native.STORAGE_F16, native.STORAGE_BF16])
+def test_exchanges_lie_a_halo_of_messages_apart(lib, w, h, k, storage):
+    """Packets are written again two exchanges later, and a copy is safe then
+    because the messages between two exchanges go from strip to strip over a
+    whole halo; the halo lasts for the sweeps between them; 16-bit fields are
+    rounded after every K sweeps, whatever lies between exchanges."""
+    exchanged = 0
+    for n, pressure in [(9, 0), (21, 1), (50, 0), (100, 1)]:
+        cfg = tunnel(w, h, projection_n=n, projection_block=k, projection_resident=3,
+                     storage=storage, enable_pressure=pressure)
+        with Handle(lib, cfg) as f:
+            assert f.update() == native.OS_OK
+            for x in launches(lib, DIFFUSE, PROJECT):
+                reach = x.halo // x.R + 1
+                done = since = messages = exchanges = 0
+                for sweeps, sent, rounded, exchange in segments(lib, x, storage):
+                    wide = storage == native.STORAGE_F32
+                    assert bool(rounded) == (not wide and done > 0 and done % k == 0)
+                    if exchange:
+                        assert x.cooperative and messages >= reach
+                        since = messages = 0
+                        exchanges += 1
+                    done, since, messages = done + sweeps, since + sweeps, messages + sent
+                    if x.tiles > 1:
+                        assert since * (2 if x.kind == PROJECT else 1) <= x.halo
+                assert done == x.n
+                assert x.tiles == 1 or exchanges == (x.n + x.D - 1) // x.D - 1
+                exchanged += exchanges
+    assert exchanged

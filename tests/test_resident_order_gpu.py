@@ -1,0 +1,42 @@
+"""Resident phases where the order between their tiles is what counts: few sweeps
+(no exchange, an even number of passes), a sweep more than lie between two
+exchanges, and 16-bit storage whose roundings come more often than exchanges.
+The bits of the same depth pass by pass: no tolerance."""
+import numpy as np
+import pytest
+
+from opensayal_gb300 import native
+from tests.parity_cases import FIELDS, load_lib
+from tests.test_tiles_gpu import state_of, tunnel
+
+pytestmark = pytest.mark.gpu
+
+
+def assert_same(a, b, fields):
+    """Equal cell for cell: infinities and the largest numbers apart, NaN with
+    NaN, +0 with -0."""
+    for field in fields:
+        assert np.array_equal(a.download(field), b.download(field), equal_nan=True), field
+
+
+@pytest.mark.parametrize("w,h", [(333, 187), (571, 157), (800, 400), (1003, 300)])
+@pytest.mark.parametrize("k,n", [(2, 3), (2, 8), (4, 6), (4, 13), (4, 33), (6, 21), (8, 16),
+                                 (8, 21), (12, 25)])
+@pytest.mark.parametrize("storage", [native.STORAGE_F32, native.STORAGE_F16, native.STORAGE_BF16])
+def test_resident_equals_passes(gpu, w, h, k, n, storage):
+    base = tunnel(w, h, projection_n=n, storage=storage, projection_block=k,
+                  enable_pressure=(w + n) % 2)
+    state = state_of(base, w + k + n)
+    passes, resident = base.copy(), base.copy()
+    passes.projection_resident, resident.projection_resident = -1, 3
+    a, b = load_lib(passes, state), load_lib(resident, state)
+    assert b.fields().projection_resident == (3 if k % 4 == 0 else 1)
+    for phase in (native.PHASE_DIFFUSION, native.PHASE_PROJECTION):
+        a.run_phase(phase, None, 0.05)
+        b.run_phase(phase, None, 0.05)
+    for _ in range(2):
+        a.update(None, 0.02)
+        b.update(None, 0.02)
+    assert_same(a, b, FIELDS + (("pressure",) if base.enable_pressure else ()))
+    a.close()
+    b.close()

@@ -1366,7 +1366,11 @@ k_project_tiles(const __grid_constant__ ProjectArgs a) {
       number++;
       exchange<2, R>(u, v, vt, sm.exchange, a.sync, a.g, W, H, number);
     }
-    tile_sweeps<PRESSURE, R>(u, v, vt, L, sm, link, a.sync, P.yl * 64 + P.lane, P.down, c, d_t,
+    // (High strips have no registers to keep the patch in: 1920 x 1080 with the
+    // pressure takes 320 us so, and 340 us with it kept; 640 x 448, with strips of
+    // two rows, 1.4% longer with it worked out anew.)
+    const Patch S = R >= 6 ? patch_of(a.g, R, W, H) : P;
+    tile_sweeps<PRESSURE, R>(u, v, vt, L, sm, link, a.sync, S.yl * 64 + S.lane, S.down, c, d_t,
                              s.sweeps, message);
     message += project_messages(s.sweeps);
     done += s.sweeps;

@@ -263,6 +263,7 @@ inline int phase_tile(os_handle* h, bool projection, int K, bool resident, RegTi
 inline int enqueue_tiled_projection(os_handle* h, cudaStream_t st, int* cur_u, int* cur_v,
                                     bool zero_first, bool extrapolate) {
   const int K = h->block_k, n = h->c.n;
+  if (n < 1) return 0;  // no sweeps, no tile to choose
   const bool pressure = h->cfg.enable_pressure != 0;
   ProjectArgs a{};
   void *const U[2] = {h->u, h->ub}, *const V[2] = {h->v, h->vb};
@@ -282,11 +283,10 @@ inline int enqueue_tiled_projection(os_handle* h, cudaStream_t st, int* cur_u, i
     a.vi = V[*cur_v], a.vo = V[1 - *cur_v];
     a.zero_pressure = zero_first;
     a.extrapolate = extrapolate;
-    if (passes > 0 &&
-        launch_tiles(project_kernel_of(a.g.R, pressure, quads_aligned(h->W, a.g.halo)), a, a.g, n > a.D, h->pdl, st) !=
-            cudaSuccess)
+    if (launch_tiles(project_kernel_of(a.g.R, pressure, quads_aligned(h->W, a.g.halo)), a, a.g,
+                     n > a.D, h->pdl, st) != cudaSuccess)
       return -1;
-    launches = passes > 0;
+    launches = 1;
   } else {
     if (projection_smem(2 + 4 * K, pressure) + kStaticSmem > kMaxSmem ||
         !(a.D = phase_tile(h, true, K, false, &a.g)))
@@ -312,6 +312,7 @@ inline int enqueue_tiled_projection(os_handle* h, cudaStream_t st, int* cur_u, i
 // else diffusion_depth.
 inline int enqueue_tiled_diffusion(os_handle* h, cudaStream_t st, int* cur_u) {
   const int K = h->resident_diff ? h->block_k : diffusion_depth(h), n = h->c.n;
+  if (n < 1) return 0;
   DiffuseArgs a{};
   void* const U[2] = {h->u, h->ub};
   a.storage = h->storage;
@@ -325,10 +326,10 @@ inline int enqueue_tiled_diffusion(os_handle* h, cudaStream_t st, int* cur_u) {
     if (!(a.D = phase_tile(h, false, K, true, &a.g))) return -1;
     a.n = n;
     a.ui = U[*cur_u], a.uo = U[1 - *cur_u];
-    if (passes > 0 && launch_tiles(diffuse_kernel_of(a.g.R, quads_aligned(h->W, a.g.halo)), a, a.g, n > a.D, h->pdl, st) !=
-                          cudaSuccess)
+    if (launch_tiles(diffuse_kernel_of(a.g.R, quads_aligned(h->W, a.g.halo)), a, a.g, n > a.D,
+                     h->pdl, st) != cudaSuccess)
       return -1;
-    launches = passes > 0;
+    launches = 1;
   } else {
     if (!(a.D = phase_tile(h, false, K, false, &a.g))) return -1;
     for (int p = 0; p < passes; p++, launches++) {

@@ -70,3 +70,20 @@ def test_exchanges_lie_a_halo_of_messages_apart(lib, w, h, k, storage):
                 assert x.tiles == 1 or exchanges == (x.n + x.D - 1) // x.D - 1
                 exchanged += exchanges
     assert exchanged
+
+
+@pytest.mark.parametrize("k,resident", [(-1, -1), (0, 0), (0, -1), (0, 3), (1, -1), (8, -1), (8, 3),
+                                        (24, -1), (32, 3)])
+@pytest.mark.parametrize("viscosity", [0.0, 0.02])
+@pytest.mark.parametrize("pressure", [0, 1])
+def test_no_sweeps_are_no_launches(lib, k, resident, viscosity, pressure):
+    """projection_n = 0 is a valid step without diffusion and projection."""
+    cfg = tunnel(640, 448, projection_n=0, projection_block=k, projection_resident=resident,
+                 viscosity=viscosity, enable_pressure=pressure)
+    with Handle(lib, cfg) as f:
+        assert f.update() == native.OS_OK, lib.os_last_error()
+        done = launches(lib)
+        assert done and not [x for x in done if x.kind in (DIFFUSE, PROJECT)]
+        for phase in (native.PHASE_DIFFUSION, native.PHASE_PROJECTION):
+            assert lib.os_run_phase(f.h, phase, None, 0.05) == native.OS_OK
+        assert not launches(lib)

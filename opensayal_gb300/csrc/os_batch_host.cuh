@@ -91,9 +91,7 @@ int batch_tiles(int size, int pitch, int halo, int region) {
 
 // Clusters of the kernel that are resident together (several CTAs to an SM).
 int batch_clusters(BatchTileKernel kernel, const RegTile& g, cudaLaunchAttribute* attr) {
-  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g.smem) !=
-      cudaSuccess)
-    return 0;
+  if (allow_most(kernel) != cudaSuccess) return 0;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(g.cluster * 1024);
   cfg.blockDim = dim3(32 * g.warps);

@@ -16,7 +16,9 @@
 
 #include <algorithm>
 #include <mutex>
+#include <set>
 #include <type_traits>
+#include <utility>
 
 namespace osg {
 
@@ -295,6 +297,32 @@ inline void launch_pdl(bool pdl, void (*kernel)(KArgs...), dim3 grid, dim3 block
 constexpr size_t kMaxSmem = 227 * 1024;
 constexpr size_t kStaticSmem = 256;
 
+// Lets a kernel take as much dynamic shared memory as there is beside its own
+// static memory, and clusters beyond the portable size. These limits belong to
+// the kernel, not to a launch, and to the whole process: set to one grid's size
+// before its launch, they could be lowered between the two by another thread
+// with a smaller grid, and the launch was refused. So they are set once per
+// kernel and device, to the most, and stay.
+inline cudaError_t allow_most(const void* kernel) {
+  static std::mutex mu;
+  static std::set<std::pair<const void*, int>> done;
+  int device = 0;
+  cudaError_t e = cudaGetDevice(&device);
+  if (e != cudaSuccess) return e;
+  std::lock_guard<std::mutex> lock(mu);
+  if (done.count({kernel, device})) return cudaSuccess;
+  e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)(kMaxSmem - kStaticSmem));
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  if (e == cudaSuccess) done.insert({kernel, device});
+  return e;
+}
+template <class... KArgs>
+inline cudaError_t allow_most(void (*kernel)(KArgs...)) {
+  return allow_most(reinterpret_cast<const void*>(kernel));
+}
+
 // Owned tile height for a given halo: aim for one CTA per SM per wave
 // (152 SMs), keep TY even, and fit shared memory.
 inline TileGeom make_geom(int W, int H, int halo, int sms) {
@@ -400,8 +428,7 @@ inline int enqueue_tma_diffusion(os_handle* h, cudaStream_t st, int* cur_u) {
   float* U[2] = {static_cast<float*>(h->u), static_cast<float*>(h->ub)};
   const int tiles = g.tiles_x * g.tiles_y;
   const size_t smem = tma_diffusion_smem(g.RH);
-  cudaFuncSetAttribute(k_diffuse_blocked_tma, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)smem);
+  if (allow_most(k_diffuse_blocked_tma) != cudaSuccess) return -1;
   int launches = 0;
   for (int done = 0; done < h->c.n;) {
     const int sweeps = std::min(K, h->c.n - done);

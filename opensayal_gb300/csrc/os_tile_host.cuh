@@ -68,7 +68,7 @@ inline int ctas_per_sm(int R, int warps, bool projection, size_t smem) {
 }
 
 // Clusters of `cluster` CTAs that are resident together with `ctas` CTAs to an
-// SM.
+// SM. An answer is kept; a query that fails is made again the next time.
 inline int resident_clusters(int device, int cluster, int ctas) {
   static std::mutex mu;
   static std::map<std::tuple<int, int, int>, int> known;
@@ -79,12 +79,10 @@ inline int resident_clusters(int device, int cluster, int ctas) {
   const auto kernel = diffuse_kernel<2>(true);
   const size_t smem = (227 / ctas - 1) * 1024;  // as much as leaves room for no more CTAs
   int n = 0;
-  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) ==
-          cudaSuccess &&
-      cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) ==
-          cudaSuccess) {
+  cudaError_t e = allow_most(kernel);
+  if (e == cudaSuccess) {
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(cluster * 152);
+    cfg.gridDim = dim3(cluster * sm_count(device));
     cfg.blockDim = dim3(128);
     cfg.dynamicSmemBytes = smem;
     cudaLaunchAttribute attr[1];
@@ -93,9 +91,12 @@ inline int resident_clusters(int device, int cluster, int ctas) {
     attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) n = 0;
+    e = cudaOccupancyMaxActiveClusters(&n, kernel, &cfg);
   }
-  cudaGetLastError();
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
   known[key] = n;
   return n;
 }
@@ -185,10 +186,7 @@ inline double choose_tile(int W, int H, int D, bool projection, bool pressure, b
 template <class Args>
 inline cudaError_t launch_tiles(void (*kernel)(const Args), const Args& a, const RegTile& g,
                                 bool cooperative, bool pdl, cudaStream_t st) {
-  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)g.smem);
-  if (e == cudaSuccess && g.cluster > 8)
-    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  const cudaError_t e = allow_most(kernel);
   if (e != cudaSuccess) return e;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(g.tiles_x * g.tiles_y * g.cluster);

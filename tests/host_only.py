@@ -2,6 +2,7 @@
 and host_runtime.cpp): kernels do not run, launches are written down."""
 import ctypes as C
 import os
+import shutil
 import subprocess
 
 from opensayal_gb300 import native
@@ -37,11 +38,12 @@ def build():
     objects = [LIB.with_suffix(f".{k}.o") for k in range(2)]
     # The device code is not used: PTX, without the assembler's time.
     cmds = [[f"{cuda}/bin/nvcc", "-std=c++17", "-O1", "--use_fast_math", "-gencode",
-             "arch=compute_103a,code=compute_103a", "-Xcompiler", "-fPIC", "-diag-suppress", "177",
-             "-c", "-o", str(objects[0]), str(SOURCES[0])],
+             "arch=compute_103a,code=compute_103a", "-Xcompiler", "-fPIC,-fno-gnu-unique",
+             "-diag-suppress", "177", "-c", "-o", str(objects[0]), str(SOURCES[0])],
             ["g++", "-std=c++17", "-O1", "-fPIC", f"-I{cuda}/include", "-c", "-o",
              str(objects[1]), str(SOURCES[1])],
-            # The runtime calls bind to the ones here, whatever the process has loaded.
+            # The runtime calls bind to the ones here, whatever the process has loaded
+            # (and what inline functions keep is this library's own: no unique symbols).
             ["g++", "-shared", "-Wl,-Bsymbolic", "-Wl,-z,defs", "-o", str(LIB),
              *map(str, objects), "-lpthread"]]
     for cmd in cmds:
@@ -49,8 +51,12 @@ def build():
     return LIB
 
 
-def load():
-    lib = C.CDLL(str(build()))
+def load(copy_to=None):
+    """The library; a copy in a folder has a state of its own."""
+    path = build()
+    if copy_to is not None:
+        path = shutil.copy(path, copy_to)
+    lib = C.CDLL(str(path))
     for name, res, args in native.SIGNATURES:
         fn = getattr(lib, name)
         fn.argtypes, fn.restype = args, res

@@ -87,3 +87,31 @@ def test_no_sweeps_are_no_launches(lib, k, resident, viscosity, pressure):
         for phase in (native.PHASE_DIFFUSION, native.PHASE_PROJECTION):
             assert lib.os_run_phase(f.h, phase, None, 0.05) == native.OS_OK
         assert not launches(lib)
+
+
+def test_limits_of_kernels_are_never_lowered(lib):
+    """A kernel's shared-memory limit is the process's, not a launch's: a handle
+    that lowers it takes it from another thread's launch."""
+    sizes = [(256, 128), (1920, 1080), (333, 187), (4096, 4096), (640, 448), (800, 400)]
+    for resident in (-1, 3):
+        for pressure in (0, 1):
+            for w, h in sizes + sizes[::-1]:
+                cfg = tunnel(w, h, projection_n=20, projection_block=4,
+                             projection_resident=resident, enable_pressure=pressure)
+                with Handle(lib, cfg) as f:
+                    assert f.update() == native.OS_OK
+                    assert all(x.smem <= x.limit for x in launches(lib, DIFFUSE, PROJECT))
+    assert lib.state.limits_lowered == 0
+
+
+def test_a_failed_query_is_made_again(tmp_path):
+    """A passing error must not keep the process's later handles off the tiles."""
+    lib = load(copy_to=tmp_path)  # a library without answers kept from other tests
+    cfg = tunnel(640, 448, projection_n=20, projection_block=8, projection_resident=3)
+    lib.state.fail_attribute = 1 << 30
+    with Handle(lib, cfg) as f:
+        assert f.fields().projection_resident == 0
+    lib.state.fail_attribute = 0
+    with Handle(lib, cfg) as f:
+        assert f.fields().projection_resident == 3
+        assert f.update() == native.OS_OK

@@ -368,12 +368,13 @@ int os_render_traces(os_handle* h, const os_visual_config* v, float dt, int32_t*
                      int32_t* d_y, void* stream);
 
 /*
- * Failure detection of the resident projection's inter-tile waits, without a
- * fault: one CTA waits on a neighbour flag that nothing sets. Every such wait
- * is bounded; when it gives up it records the failure, and the host call that
- * synchronises reports OS_ERR_TIMEOUT. *status receives what that path
- * reports here (OS_ERR_TIMEOUT when the bound works). No reference
- * counterpart.
+ * Failure detection of the tile phases' waits, without a fault: one CTA waits
+ * for a neighbouring tile's packet that nothing sends, then one for the
+ * messages of a neighbouring strip that sends none. Every such wait is bounded
+ * (about a second); when one gives up it records the failure, the waits after
+ * it end with it, and the host call that synchronises reports OS_ERR_TIMEOUT.
+ * *status receives what that path reports here (OS_ERR_TIMEOUT when both bounds
+ * work). No reference counterpart.
  */
 int os_selftest_bounded_wait(int32_t device, int32_t* status);
 

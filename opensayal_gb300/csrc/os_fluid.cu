@@ -1291,12 +1291,22 @@ int os_selftest_bounded_wait(int32_t device, int32_t* status) {
     *host_err = 0;
     e = cudaHostGetDevicePointer((void**)&d_host_err, host_err, 0);
   }
-  if (e == cudaSuccess) {
-    k_wait_selftest<<<1, 32>>>(ResidentSync{nullptr, packets, dev_err, d_host_err});
-    e = cudaGetLastError();
+  // Packets, then messages (400, as many as 200 sweeps take): each must report.
+  const ResidentSync sync{nullptr, packets, dev_err, d_host_err};
+  bool reported = true;
+  for (int messages = 0; messages < 2 && e == cudaSuccess; messages++) {
+    *host_err = 0;
+    if ((e = cudaMemset(dev_err, 0, sizeof(int))) != cudaSuccess) break;
+    if (messages) {
+      e = launch_message_selftest(sync, 400);
+    } else {
+      k_wait_selftest<<<1, 32>>>(sync);
+      e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) e = cudaDeviceSynchronize();
+    reported = reported && *(volatile int*)host_err;
   }
-  if (e == cudaSuccess) e = cudaDeviceSynchronize();
-  if (e == cudaSuccess) *status = *(volatile int*)host_err ? OS_ERR_TIMEOUT : OS_OK;
+  if (e == cudaSuccess) *status = reported ? OS_ERR_TIMEOUT : OS_OK;
   if (packets) cudaFree(packets);
   if (dev_err) cudaFree(dev_err);
   if (host_err) cudaFreeHost(host_err);

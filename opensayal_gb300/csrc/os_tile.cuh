@@ -228,7 +228,7 @@ __device__ __forceinline__ uint32_t rows_in(int y0, int R, int lo, int hi) {
 // send to the strip that is not there.
 // ---------------------------------------------------------------------------
 constexpr int kInboxHead = 16;      // two mbarriers
-constexpr int kMessageSpin = 1 << 20;  // polls of a bounded wait
+constexpr uint32_t kMessageLimit = 1000000000u;  // of a bounded wait, in ns
 
 __host__ __device__ constexpr int inbox_bytes(int words) { return kInboxHead + 4 * words * 128; }
 
@@ -255,6 +255,7 @@ struct Link {
   uint32_t mine;                 // this warp's inbox (shared address)
   uint32_t up, down;             // the neighbours' inboxes (cluster shared addresses)
   uint32_t up_part, down_part;   // where this strip's part goes in them
+  bool lost;  // a wait gave up: the strip takes no further part (the same in the warp)
 };
 
 // Prepares the warp's inbox and finds the neighbours'; the caller passes a
@@ -266,6 +267,7 @@ __device__ __forceinline__ Link<WORDS> open_link(char* smem, const Patch& P, con
   const uint32_t base = shared_address(smem);
   const int rank = blockIdx.x % g.cluster;
   k.mine = base + P.warp * kBytes;
+  k.lost = false;
   const uint32_t self = cluster_address(k.mine, rank);
   k.up = P.up ? (P.warp + 1 < g.warps ? cluster_address(k.mine + kBytes, rank)
                                       : cluster_address(base, rank + 1))
@@ -295,31 +297,39 @@ __device__ __forceinline__ void post(uint32_t inbox, uint32_t part, unsigned m, 
       : "memory");
 }
 
-// Waits until both parts of message m are there. A wait that gives up records
-// the failure and carries on; the host reports it.
+// Waits until both parts of message m are there, for kMessageLimit or until
+// another wait has given up (looked at every 64 polls, each of which the hardware
+// may hold for a while). A wait that gives up records the failure, and the strip
+// sends and awaits nothing more: every later wait for one of its messages ends
+// soon, and no mbarrier that is behind is armed again. The host reports it.
 template <int WORDS>
-__device__ __forceinline__ void await_message(const Link<WORDS>& link, unsigned m,
+__device__ __forceinline__ void await_message(Link<WORDS>& link, unsigned m,
                                               const ResidentSync& sync) {
   const uint32_t bar = link.mine + 8 * (m & 1u);
   if ((threadIdx.x & 31) == 0)
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar),
                  "r"(2 * Link<WORDS>::kPart)
                  : "memory");
-  uint32_t done = 0;
+  uint32_t done = 0, since = 0;
 #pragma unroll 1
-  for (int it = 0; !done; it++) {
+  for (int it = 0;; it++) {
     asm volatile(
         "{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
         " selp.u32 %0, 1, 0, p;\n}"
         : "=r"(done)
         : "r"(bar), "r"((m >> 1) & 1u)
         : "memory");
-    if (it >= kMessageSpin) {
+    if (done) break;
+    if (it % 64 != 63) continue;
+    uint32_t now;
+    asm volatile("mov.u32 %0, %%globaltimer_lo;" : "=r"(now));
+    if (it == 63) since = now;
+    if (now - since > kMessageLimit || *(volatile int*)sync.dev_err) {
       record_failure(sync);
       break;
     }
   }
-  __syncwarp();  // lanes may have left the loop apart
+  link.lost = !__all_sync(kAllLanes, done);  // lanes may have left the loop apart
 }
 // Words 4 k .. of the part from below (0) or above (1) of message m.
 template <int WORDS>
@@ -338,10 +348,10 @@ __device__ __forceinline__ float4 read_message(const Link<WORDS>& link, int part
 // that the strips beside it wait for nothing, and its cells stay as they are
 // (zero, as a neighbour's face off the grid is).
 template <int WORDS>
-__device__ __forceinline__ void idle_messages(const Link<WORDS>& link, unsigned m, int count,
+__device__ __forceinline__ void idle_messages(Link<WORDS>& link, unsigned m, int count,
                                               const ResidentSync& sync) {
 #pragma unroll 1
-  for (const unsigned end = m + count; m != end; m++) {
+  for (const unsigned end = m + count; m != end && !link.lost; m++) {
 #pragma unroll
     for (int k = 0; k < WORDS / 4; k++) {
       post<WORDS>(link.down, link.down_part, m, k, make_float4(0.0f, 0.0f, 0.0f, 0.0f));
@@ -1093,7 +1103,7 @@ __device__ __forceinline__ void strip_send(const float (&v)[R][8], const float (
 
 template <int COLOUR, int R>
 __device__ __forceinline__ void strip_receive(float (&v)[R][8], float (&vt)[8],
-                                              const Link<4>& link, unsigned m, bool down,
+                                              Link<4>& link, unsigned m, bool down,
                                               const ResidentSync& sync) {
   constexpr int nb = 1 - COLOUR, nt = 1 - ((COLOUR + R - 1) & 1);
   await_message(link, m, sync);
@@ -1112,7 +1122,7 @@ __device__ __forceinline__ void strip_receive(float (&v)[R][8], float (&vt)[8],
 template <int COLOUR, bool PRESSURE, Rows ROWS, int R>
 __device__ __forceinline__ void half_sweep(float (&u)[R][8], float (&v)[R][8], float (&ur)[R],
                                            float (&vt)[8], const ProjLane& L, const ProjSmem& sm,
-                                           const Link<4>& link, const ResidentSync& sync,
+                                           Link<4>& link, const ResidentSync& sync,
                                            int cell0, bool down, unsigned m, const Consts& c,
                                            float d_t) {
 #pragma unroll
@@ -1127,11 +1137,11 @@ __device__ __forceinline__ void half_sweep(float (&u)[R][8], float (&v)[R][8], f
 template <bool PRESSURE, Rows ROWS, int R>
 __device__ __forceinline__ void sweep_loop(float (&u)[R][8], float (&v)[R][8], float (&ur)[R],
                                            float (&vt)[8], const ProjLane& L, const ProjSmem& sm,
-                                           const Link<4>& link, const ResidentSync& sync,
+                                           Link<4>& link, const ResidentSync& sync,
                                            int cell0, bool down, const Consts& c, float d_t,
                                            int sweeps, unsigned m) {
 #pragma unroll 1
-  for (int t = 0; t < sweeps; t++, m += 2) {
+  for (int t = 0; t < sweeps && !link.lost; t++, m += 2) {
     half_sweep<0, PRESSURE, ROWS, R>(u, v, ur, vt, L, sm, link, sync, cell0, down, m, c, d_t);
     half_sweep<1, PRESSURE, ROWS, R>(u, v, ur, vt, L, sm, link, sync, cell0, down, m + 1, c, d_t);
   }
@@ -1147,10 +1157,11 @@ __host__ __device__ inline unsigned project_messages(int sweeps) { return 2 * sw
 template <bool PRESSURE, int R>
 __device__ __forceinline__ void tile_sweeps(float (&u)[R][8], float (&v)[R][8], float (&vt)[8],
                                             const ProjLane& L, const ProjSmem& sm,
-                                            const Link<4>& link, const ResidentSync& sync,
+                                            Link<4>& link, const ResidentSync& sync,
                                             int cell0, bool down, const Consts& c, float d_t,
                                             int sweeps, unsigned m) {
   static_assert(R % 2 == 0, "strips start on even rows");
+  if (link.lost) return;
   if (L.idle) return idle_messages(link, m, project_messages(sweeps), sync);
   float ur[R];
 #pragma unroll
@@ -1166,7 +1177,7 @@ __device__ __forceinline__ void tile_sweeps(float (&u)[R][8], float (&v)[R][8], 
   else
     sweep_loop<PRESSURE, Rows::kPlain, R>(u, v, ur, vt, L, sm, link, sync, cell0, down, c, d_t,
                                           sweeps, m);
-  strip_receive<1, R>(v, vt, link, m + 2 * sweeps, down, sync);
+  if (!link.lost) strip_receive<1, R>(v, vt, link, m + 2 * sweeps, down, sync);
 }
 
 // apply_extrapolation_at (src/fluid.cu:720-733) on a patch, in
@@ -1326,7 +1337,7 @@ k_project_tiles(const __grid_constant__ ProjectArgs a) {
   const int W = c.W, H = c.H, rows = a.g.warps * R;
   const Patch P = patch_of(a.g, R, W, H);
   const ProjSmem sm = project_smem_of(tile_smem, rows, a.g.warps, PRESSURE);
-  const Link<4> link = open_link<4>(tile_smem, P, a.g);
+  Link<4> link = open_link<4>(tile_smem, P, a.g);
   cluster_arrive();
   float* const stage = ALIGNED ? nullptr : stage_of(tile_smem, a.g);
   ProjLane L;
@@ -1464,12 +1475,12 @@ __device__ __forceinline__ void row_receive(float (&f)[8], const Link<8>& link, 
 }
 
 template <int R, Kept KEPT>
-__device__ __forceinline__ void jacobi_loop(float (&u)[R][8], const Link<8>& link,
+__device__ __forceinline__ void jacobi_loop(float (&u)[R][8], Link<8>& link,
                                             const ResidentSync& sync, const DiffLane& L, float a,
                                             float den, float rden, bool rcp, int sweeps,
                                             unsigned m) {
 #pragma unroll 1
-  for (int t = 0; t < sweeps; t++, m++) {
+  for (int t = 0; t < sweeps && !link.lost; t++, m++) {
     rows_send<R>(u, link, m);
     // The inner rows first, while the neighbours' rows come in.
     float down[8], second[8], row[8];
@@ -1491,7 +1502,7 @@ __device__ __forceinline__ void jacobi_loop(float (&u)[R][8], const Link<8>& lin
 // the sweeps reach from the owned rows.
 template <int R>
 __device__ __forceinline__ void jacobi_sweeps(float (&u)[R][8], const DiffLane& L,
-                                              const Link<8>& link, const ResidentSync& sync,
+                                              Link<8>& link, const ResidentSync& sync,
                                               float a, int sweeps, unsigned m) {
   const float den = fma_rn(4.0f, a, 1.0f);
   const float rden = __fdividef(1.0f, den);
@@ -1528,7 +1539,7 @@ k_diffuse_tiles(const __grid_constant__ DiffuseArgs a) {
   const Consts& c = a.c;
   const int W = c.W, H = c.H;
   const Patch P = patch_of(a.g, R, W, H);
-  const Link<8> link = open_link<8>(tile_smem, P, a.g);
+  Link<8> link = open_link<8>(tile_smem, P, a.g);
   cluster_arrive();
   float* const stage = ALIGNED ? nullptr : stage_of(tile_smem, a.g);
   pdl_entry();

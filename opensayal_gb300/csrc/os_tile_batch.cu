@@ -5,12 +5,30 @@
 // Bound by the sweeps' instructions and by the faces' way from strip to strip;
 // the loads and stores of one tile run beside the sweeps of the other on the
 // SM. 21 tunnels of 128 to 1024 cells a side (6.85 M cells in all): a step
-// takes 2035 us, and took 2968 us with tiles held in shared memory; 6 tunnels
-// of mixed storage 2036 us, and 3378 us.
+// takes 2004 us, and took 2968 us with tiles held in shared memory; 6 tunnels
+// of mixed storage 1978 us, and 3378 us.
 #include "os_batch_plan.cuh"
 
 namespace osg {
 namespace {
+
+// A tile's faces out after a pass. Which tile and whose is read anew (kept across
+// the sweeps it costs registers that their faces need).
+template <int R>
+__device__ __forceinline__ void tile_done(float (&u)[R][8], float (&v)[R][8],
+                                          const TileRef* tiles, const ScenarioDesc* descs, int it,
+                                          int pass, const RegTile& g, char* smem) {
+  asm volatile("" : "+r"(it));
+  const TileRef t = tiles[it];
+  const ScenarioDesc& d = descs[t.slot];
+  const int W = d.c.W, H = d.c.H;
+  const int iu = (d.diff_passes + pass) & 1, iv = pass & 1;
+  const Patch P = patch_at(TilePlace{t.tx, t.ty, d.proj_tiles_x, d.proj_tiles_y}, g, R, W, H);
+  float* const stage = quads_aligned(W, g.halo) ? nullptr : stage_of(smem, g);
+  if (!P.idle)
+    faces_out<R>(u, v, iu ? d.u : d.ub, iv ? d.v : d.vb, d.storage, P, W, H, stage,
+                 pass + 1 == d.proj_passes);
+}
 
 // Two CTAs of six warps with 168 registers fill an SM's register file: three
 // warps to a scheduler hide the faces' way better than two of four warps with
@@ -21,7 +39,7 @@ k_batch_project_tiles(const PlanHeader* __restrict__ plan, const int* __restrict
   constexpr int R = kBatchProjectRows;
   extern __shared__ __align__(16) char tile_smem[];
   const ProjSmem sm = project_smem_of(tile_smem, g.warps * R, g.warps, false);
-  const Link<4> link = open_link<4>(tile_smem, patch_at(TilePlace{0, 0, 1, 1}, g, R, 1, 1), g);
+  Link<4> link = open_link<4>(tile_smem, patch_at(TilePlace{0, 0, 1, 1}, g, R, 1, 1), g);
   cluster_arrive();
   pdl_entry();
   const int items = plan->proj_items[pass];
@@ -30,7 +48,8 @@ k_batch_project_tiles(const PlanHeader* __restrict__ plan, const int* __restrict
   cluster_wait();
   unsigned message = 0;
 #pragma unroll 1
-  for (int it = blockIdx.x / g.cluster; it < items; it += gridDim.x / g.cluster) {
+  for (int it = blockIdx.x / g.cluster; it < items && !link.lost;
+       it += gridDim.x / g.cluster) {
     const TileRef t = tiles[it];
     if (remaining[t.slot] == 0) continue;  // the same for the whole cluster
     const ScenarioDesc& d = descs[t.slot];
@@ -65,11 +84,7 @@ k_batch_project_tiles(const PlanHeader* __restrict__ plan, const int* __restrict
     }
     tile_sweeps<false, R>(u, v, vt, L, sm, link, sync, cell0, down, c, 0.0f, sweeps, message);
     message += project_messages(sweeps);
-    const Patch P = patch_at(place, g, R, W, H);
-    float* const out = quads_aligned(W, g.halo) ? nullptr : stage_of(tile_smem, g);
-    if (!P.idle)
-      faces_out<R>(u, v, iu ? d.u : d.ub, iv ? d.v : d.vb, d.storage, P, W, H, out,
-                   pass + 1 == d.proj_passes);
+    tile_done<R>(u, v, tiles, descs, it, pass, g, tile_smem);
   }
   cluster_arrive();  // no CTA leaves while another may still send to it
   cluster_wait();
@@ -80,7 +95,7 @@ k_batch_diffuse_tiles(const PlanHeader* __restrict__ plan, const int* __restrict
                       int pass, int K, const RegTile g, const ResidentSync sync) {
   constexpr int R = kBatchDiffuseRows;
   extern __shared__ __align__(16) char tile_smem[];
-  const Link<8> link = open_link<8>(tile_smem, patch_at(TilePlace{0, 0, 1, 1}, g, R, 1, 1), g);
+  Link<8> link = open_link<8>(tile_smem, patch_at(TilePlace{0, 0, 1, 1}, g, R, 1, 1), g);
   cluster_arrive();
   pdl_entry();
   const int items = plan->diff_items[pass];
@@ -89,7 +104,8 @@ k_batch_diffuse_tiles(const PlanHeader* __restrict__ plan, const int* __restrict
   cluster_wait();
   unsigned message = 0;
 #pragma unroll 1
-  for (int it = blockIdx.x / g.cluster; it < items; it += gridDim.x / g.cluster) {
+  for (int it = blockIdx.x / g.cluster; it < items && !link.lost;
+       it += gridDim.x / g.cluster) {
     const TileRef t = tiles[it];
     if (remaining[t.slot] == 0) continue;  // the same for the whole cluster
     const ScenarioDesc& d = descs[t.slot];

@@ -350,7 +350,7 @@ inline size_t resident_packet_bytes(int W, int H, int per_quad) {
   return (size_t)2 * packet_plane(W, H) * per_quad * sizeof(uint4);
 }
 
-// Failure-detection self-test: a warp waits for a packet that nothing sends, so
+// Failure-detection self-tests. A warp waits for a packet that nothing sends, so
 // the wait must give up and report.
 __global__ void k_wait_selftest(ResidentSync sync) {
   float a = 0.0f, b = 0.0f, c = 0.0f;
@@ -360,6 +360,36 @@ __global__ void k_wait_selftest(ResidentSync sync) {
     again = !__all_sync(kAllLanes, ok) && poll_again(it, sync);
     again = __any_sync(kAllLanes, again);
   }
+}
+
+// The strip of the first of two CTAs takes part in `count` messages, and the
+// second's sends none: the first wait must give up, and the others end with it.
+__global__ void k_message_selftest(ResidentSync sync, int count) {
+  extern __shared__ __align__(16) char tile_smem[];
+  RegTile g{};
+  g.R = 2, g.warps = 1, g.cluster = 2, g.RH = 4;
+  Link<4> link = open_link<4>(tile_smem, patch_at(TilePlace{0, 0, 1, 1}, g, g.R, 1, 1), g);
+  cluster_arrive();
+  cluster_wait();
+  if (blockIdx.x == 0) idle_messages(link, 0, count, sync);
+  cluster_arrive();
+  cluster_wait();
+}
+
+inline cudaError_t launch_message_selftest(const ResidentSync& sync, int count) {
+  cudaError_t e = allow_most(k_message_selftest);
+  if (e != cudaSuccess) return e;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = 2;
+  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(2);
+  cfg.blockDim = dim3(32);
+  cfg.dynamicSmemBytes = inbox_bytes(4);
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, k_message_selftest, sync, count);
 }
 
 }  // namespace osg

@@ -190,6 +190,7 @@ struct os_handle {
   uint4* rpackets = nullptr;   // exchanged cells
   uint4* dpackets = nullptr;
   int* rerr = nullptr;
+  bool stepped = false;  // this handle's own steps or phases have been enqueued
   int* host_rerr = nullptr;
   int* d_host_rerr = nullptr;
   cudaGraphExec_t graph = nullptr;
@@ -512,6 +513,7 @@ int enqueue_step(os_handle* h, Enq& q) {
 }
 
 int dispatch_step(os_handle* h, Enq& q) {
+  h->stepped = true;
   switch (h->storage) {
     case OS_STORAGE_F32: return enqueue_step<float, float>(h, q);
     case OS_STORAGE_F16: return enqueue_step<__half, float>(h, q);
@@ -522,6 +524,7 @@ int dispatch_step(os_handle* h, Enq& q) {
 }
 
 int dispatch_phase(os_handle* h, int phase, Enq& q) {
+  h->stepped = true;
   switch (h->storage) {
     case OS_STORAGE_F32: return enqueue_phase<float, float>(h, phase, q);
     case OS_STORAGE_F16: return enqueue_phase<__half, float>(h, phase, q);
@@ -645,19 +648,30 @@ int enable_resident(os_handle* h, int mask) {
   return OS_OK;
 }
 
-// After the handle's stream has drained: a resident projection whose waits
-// gave up left its fields undefined and its flags out of step; report it and
-// reset the flags so the next launch starts clean.
+// After the handle's stream has drained: a launch in which a wait gave up left
+// its fields undefined and the exchange numbers out of step; report it and reset
+// them so that the next launch starts clean.
 int check_resident(os_handle* h) {
-  if (!h->host_rerr || *(volatile int*)h->host_rerr == 0) return OS_OK;
-  *(volatile int*)h->host_rerr = 0;
+  if (h->host_rerr) {
+    if (*(volatile int*)h->host_rerr == 0) return OS_OK;
+    *(volatile int*)h->host_rerr = 0;
+  } else {
+    // A scenario of a batch with a memory budget has no mapped word: where it
+    // was stepped by itself, the device's word is read.
+    if (!h->stepped) return OS_OK;
+    int gave_up = 0;
+    CUDA_OR_RETURN(cudaMemcpyAsync(&gave_up, h->rerr, sizeof gave_up, cudaMemcpyDeviceToHost,
+                                   h->stream));
+    CUDA_OR_RETURN(cudaStreamSynchronize(h->stream));
+    if (!gave_up) return OS_OK;
+  }
   if (h->resident_block)
     cudaMemsetAsync(h->resident_block, 0, h->resident_bytes, h->stream);
   cudaMemsetAsync(h->rerr, 0, sizeof(int), h->stream);
   cudaStreamSynchronize(h->stream);
   return set_err(OS_ERR_TIMEOUT,
-                 "a bounded device wait gave up (resident projection or diffusion "
-                 "neighbours, or a tensor copy); the fields are undefined");
+                 "a bounded device wait gave up (strips or tiles of the projection or the "
+                 "diffusion, or a tensor copy); the fields are undefined");
 }
 
 void free_handle(os_handle* h) {

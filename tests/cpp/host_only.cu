@@ -86,11 +86,13 @@ extern "C" void host_describe(const void* fn, void** args, HostLaunch* l) {
     l->n = a.n, l->K = a.K, l->D = a.D;
     describe_tile(a.g, l);
     l->ui = a.ui, l->vi = a.vi, l->uo = a.uo, l->vo = a.vo;
+    l->err = a.sync.dev_err;
   } else if (l->kind == kDiffuse) {
     const auto& a = *static_cast<const osg::DiffuseArgs*>(args[0]);
     l->n = a.n, l->K = a.K, l->D = a.D;
     describe_tile(a.g, l);
     l->ui = a.ui, l->uo = a.uo;
+    l->err = a.sync.dev_err;
   }
 }
 

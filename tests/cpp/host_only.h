@@ -13,6 +13,7 @@ struct HostLaunch {
   int32_t R, warps, halo, tiles_y;
   uint64_t smem, limit;  // dynamic shared memory, and the limit set for the kernel
   const void *fn, *ui, *vi, *uo, *vo;
+  int32_t* err;  // the error word of bounded waits
 };
 // What the runtime does, and what it saw.
 struct HostState {

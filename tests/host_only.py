@@ -20,7 +20,7 @@ class HostLaunch(C.Structure):
     _fields_ = [(k, C.c_int32) for k in ("kind", "tiles", "cluster", "cooperative", "pdl",
                                          "n", "K", "D", "R", "warps", "halo", "tiles_y")]
     _fields_ += [("smem", C.c_uint64), ("limit", C.c_uint64)]
-    _fields_ += [(k, C.c_void_p) for k in ("fn", "ui", "vi", "uo", "vo")]
+    _fields_ += [(k, C.c_void_p) for k in ("fn", "ui", "vi", "uo", "vo", "err")]
 
 
 class HostState(C.Structure):

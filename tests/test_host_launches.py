@@ -1,5 +1,7 @@
 """What the host decides for the tile phases, read from the launches that a step
 makes: no GPU needed."""
+import ctypes as C
+
 import pytest
 
 from opensayal_gb300 import native
@@ -115,3 +117,23 @@ def test_a_failed_query_is_made_again(tmp_path):
     with Handle(lib, cfg) as f:
         assert f.fields().projection_resident == 3
         assert f.update() == native.OS_OK
+
+
+def test_a_wait_that_gave_up_in_a_member_alone_is_reported(lib):
+    """Members of a batch with a memory budget have no mapped word of their own; a
+    step enqueued on one by itself still has to report a wait that gave up."""
+    batch, mid, h = C.c_void_p(), C.c_int64(), C.c_void_p()
+    assert lib.os_batch_create_dynamic(0, 4, 1 << 28, C.byref(batch)) == native.OS_OK
+    cfg = tunnel(333, 187, projection_n=9)
+    assert lib.os_batch_add(batch, C.byref(cfg), -1, C.byref(mid)) == native.OS_OK
+    assert lib.os_batch_scenario(batch, mid, C.byref(h)) == native.OS_OK
+    launches(lib)
+    assert lib.os_update(h, None, 0.05) == native.OS_OK
+    word = C.c_int32.from_address(launches(lib, PROJECT)[0].err)
+    for call in (lambda: lib.os_synchronize(h), lambda: lib.os_update(h, None, 0.05),
+                 lambda: lib.os_query(h, C.byref(C.c_int32()))):
+        word.value = 1
+        assert call() == native.OS_ERR_TIMEOUT
+        assert word.value == 0
+        assert call() == native.OS_OK
+    lib.os_batch_destroy(batch)

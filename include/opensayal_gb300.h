@@ -119,15 +119,22 @@ typedef struct os_config {
                                690-693): 0 (default) FP32 float-pair
                                arithmetic that rounds like the FP64
                                expression; 1 literal FP64; 2 plain FP32 */
-  int32_t projection_resident; /* phases run as one cooperative launch each,
-                               tiles kept in shared memory and exchanging
-                               halos between passes: a mask, 1 the
-                               projection, 2 the diffusion, 3 both, each
-                               where the grid fits one co-resident tile per
-                               SM (projection: projection_block even;
-                               diffusion: a multiple of 4); 0 = the autotuner
-                               decides (with projection_block 0; a fixed
-                               projection_block runs pass by pass); -1 = never */
+  int32_t projection_resident; /* phases run as one launch each, tiles kept
+                               in the registers of thread-block clusters
+                               from the first sweep to the last and
+                               exchanging halos through device memory (24
+                               bytes a cell for the projection, 16 for the
+                               diffusion): a mask, 1 the projection, 2 the
+                               diffusion, 3 both, each where all tiles fit
+                               the GPU together and there is memory for the
+                               halos (projection: projection_block even;
+                               diffusion: a multiple of 4), else pass by
+                               pass; 0 = the autotuner decides (with
+                               projection_block 0; a fixed projection_block
+                               runs pass by pass); -1 = never. How many
+                               sweeps lie between two exchanges is the
+                               library's choice; projection_block only says
+                               how often 16-bit fields are rounded */
   int32_t diffusion_block; /* Jacobi sweeps fused per diffusion pass when the
                                diffusion runs pass by pass (not resident):
                                0 = projection_block's depth, or with
@@ -486,7 +493,8 @@ int os_batch_poll(os_batch* b, int32_t wait, int64_t* ids, int32_t cap, int32_t*
 int os_batch_wait(os_batch* b, int64_t max_in_flight);
 /* A member's state (os_member_state) and steps still to run (-1: unlimited). */
 int os_batch_status(os_batch* b, int64_t id, int32_t* state, int64_t* steps_left);
-/* Device bytes held by the members, and the budget (0: none). */
+/* Device bytes held by the members (the exchange packets of members with
+ * projection_resident among them), and the budget (0: none). */
 int os_batch_memory(os_batch* b, uint64_t* used, uint64_t* budget);
 /* The handle of member `id`, owned by the batch (do not destroy it). */
 int os_batch_scenario(os_batch* b, int64_t id, os_handle** out);

@@ -621,7 +621,8 @@ struct TuneChoice {
 TuneChoice autotune_projection(const os_config& base);
 
 // Sets up the resident projection (mask bit 0) and diffusion (bit 1) that
-// the grid fits (flags, error words).
+// the grid fits (exchange numbers and packets; none where there is no memory for
+// them: the phases then run pass by pass).
 int enable_resident(os_handle* h, int mask) {
   if (h->block_k <= 0 || h->storage == OS_STORAGE_F64 || h->arena) return OS_OK;
   const int sms = sm_count(h->cfg.device);
@@ -632,12 +633,18 @@ int enable_resident(os_handle* h, int mask) {
   cudaGetLastError();
   if (!proj && !diff) return OS_OK;
   // One block: the exchange numbers, and the packets of the phases whose tiles
-  // exchange any.
+  // exchange any (24 bytes a cell for the projection, 16 for the diffusion).
   const size_t head = 2 * resident_epoch_bytes(sms);
   const size_t pb = proj && h->c.n > dp ? resident_packet_bytes(h->W, h->H, kPacketsPerQuad<2>) : 0;
   const size_t db = diff && h->c.n > dd ? resident_packet_bytes(h->W, h->H, kPacketsPerQuad<1>) : 0;
   h->resident_bytes = head + pb + db;
-  CUDA_OR_RETURN(cudaMalloc(&h->resident_block, h->resident_bytes));
+  if (cudaMalloc(&h->resident_block, h->resident_bytes) != cudaSuccess) {
+    cudaGetLastError();
+    h->resident_block = nullptr;
+    h->resident_bytes = 0;
+    return OS_OK;
+  }
+  h->device_bytes += h->resident_bytes;
   CUDA_OR_RETURN(cudaMemsetAsync(h->resident_block, 0, h->resident_bytes, h->stream));
   h->rflags = reinterpret_cast<unsigned*>(h->resident_block);
   h->dflags = h->rflags + resident_epoch_bytes(sms) / sizeof(unsigned);

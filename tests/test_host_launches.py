@@ -137,3 +137,31 @@ def test_a_wait_that_gave_up_in_a_member_alone_is_reported(lib):
         assert word.value == 0
         assert call() == native.OS_OK
     lib.os_batch_destroy(batch)
+
+
+def test_memory_of_the_exchange_is_counted_and_may_be_refused(lib):
+    """Tiles that exchange hold packets: 24 bytes a cell for the projection and 16
+    for the diffusion. They count as the handle's device memory, and without room
+    for them the phases run pass by pass."""
+    cfg = tunnel(800, 400, projection_n=50, projection_block=8, projection_resident=3)
+
+    def member_bytes(c):
+        batch, used, budget = C.c_void_p(), C.c_uint64(), C.c_uint64()
+        assert lib.os_batch_create(C.byref(c), 1, 8, C.byref(batch)) == native.OS_OK
+        assert lib.os_batch_memory(batch, C.byref(used), C.byref(budget)) == native.OS_OK
+        lib.os_batch_destroy(batch)
+        return used.value
+
+    passes = cfg.copy()
+    passes.projection_resident = -1
+    packets = (24 + 16) * 800 * 400
+    extra = member_bytes(cfg) - member_bytes(passes)
+    assert packets <= extra <= packets + 4096
+    lib.state.fail_malloc_from = packets
+    try:
+        with Handle(lib, cfg) as f:
+            assert f.fields().projection_resident == 0
+            assert f.update() == native.OS_OK
+            assert all(not x.cooperative for x in launches(lib, DIFFUSE, PROJECT))
+    finally:
+        lib.state.fail_malloc_from = 0

@@ -34,6 +34,7 @@ struct os_batch {
   int K = 8;
   int cluster = 4;  // CTAs per cluster of the tile kernels: the tiles' height
   int sms = 152;
+  bool pdl = programmatic_launch();
   cudaStream_t stream = nullptr;
   Arena* arena = nullptr;  // null: members allocate with cudaMalloc
   RegTile gd{}, gp{};
@@ -163,19 +164,19 @@ int build_batch_graph(os_batch* b, int dpasses, int ppasses) {
     cfg.dynamicSmemBytes = g.smem;
     cfg.stream = st;
     cfg.attrs = attr;
-    cfg.numAttrs = 2;
+    cfg.numAttrs = b->pdl ? 2 : 1;
     cudaLaunchKernelEx(&cfg, kernel, P, (const int*)R, pass, b->K, g,
                        ResidentSync{nullptr, nullptr, b->d_err, b->h_err});
     kernels++;
   };
-  launch_pdl(true, k_batch_forces, row_grid, 128, 0, st, P, (const int*)R);
+  launch_pdl(b->pdl, k_batch_forces, row_grid, 128, 0, st, P, (const int*)R);
   for (int p = 0; p < dpasses; p++) tile_pass(batch_diffuse_kernel(), b->gd, b->gd_clusters, p);
   for (int p = 0; p < ppasses; p++) tile_pass(batch_project_kernel(), b->gp, b->gp_clusters, p);
-  launch_pdl(true, k_batch_extrapolate, b->sms * 4, 1024, 0, st, P, (const int*)R);
-  launch_pdl(true, k_batch_advect_velocity, row_grid, 128, 0, st, P, (const int*)R);
-  launch_pdl(true, k_batch_advect_smoke, row_grid, 128, 0, st, P, (const int*)R);
-  launch_pdl(true, k_batch_finish_smoke, row_grid, 128, 0, st, P, (const int*)R);
-  launch_pdl(true, k_batch_tick, 1, 256, 0, st, P, R);
+  launch_pdl(b->pdl, k_batch_extrapolate, b->sms * 4, 1024, 0, st, P, (const int*)R);
+  launch_pdl(b->pdl, k_batch_advect_velocity, row_grid, 128, 0, st, P, (const int*)R);
+  launch_pdl(b->pdl, k_batch_advect_smoke, row_grid, 128, 0, st, P, (const int*)R);
+  launch_pdl(b->pdl, k_batch_finish_smoke, row_grid, 128, 0, st, P, (const int*)R);
+  launch_pdl(b->pdl, k_batch_tick, 1, 256, 0, st, P, R);
   kernels += 6;
   const cudaError_t le = cudaGetLastError();
   cudaGraph_t g = nullptr;

@@ -276,6 +276,13 @@ k_diffuse_blocked_tma(const __grid_constant__ CUtensorMap in_map, float* __restr
 // Host: tile geometry and pass enqueue.
 // ---------------------------------------------------------------------------
 
+// Whether step kernels are launched programmatically: OPENSAYAL_GB300_PDL=0 turns
+// it off for the handles and batches made from then on.
+inline bool programmatic_launch() {
+  const char* env = std::getenv("OPENSAYAL_GB300_PDL");
+  return !(env && env[0] == '0');
+}
+
 // Launch with programmatic stream serialisation when `pdl` (the kernels call
 // pdl_entry() first, so the dependency on the previous kernel is kept).
 template <class... KArgs, class... Args>

@@ -928,8 +928,7 @@ static int create_handle(const os_config* cfg, Arena* arena, os_handle** out) {
   if ((e = cudaGetLastError()) != cudaSuccess ||
       (e = cudaStreamSynchronize(h->stream)) != cudaSuccess)
     return fail(set_err(OS_ERR_CUDA, "init: %s", cudaGetErrorString(e)));
-  const char* pdl_env = std::getenv("OPENSAYAL_GB300_PDL");
-  h->pdl = !(pdl_env && pdl_env[0] == '0');
+  h->pdl = programmatic_launch();
   // Tensor-copy staging of the diffusion passes is opt-in: inside a step it
   // measured 2% slower than the vector loads (with programmatic launch both
   // overlap the previous kernel, the vector loads more so).

@@ -5,7 +5,8 @@ import ctypes as C
 import pytest
 
 from opensayal_gb300 import native
-from tests.host_only import DIFFUSE, PROJECT, Handle, launches, load, segments, tunnel
+from tests.host_only import (BATCH_DIFFUSE, BATCH_PROJECT, DIFFUSE, PROJECT, Handle, launches,
+                             load, segments, tunnel)
 
 
 @pytest.fixture(scope="module")
@@ -165,3 +166,23 @@ def test_memory_of_the_exchange_is_counted_and_may_be_refused(lib):
             assert all(not x.cooperative for x in launches(lib, DIFFUSE, PROJECT))
     finally:
         lib.state.fail_malloc_from = 0
+
+
+@pytest.mark.parametrize("pdl", [None, "0", "1"])
+def test_programmatic_launch_can_be_turned_off(lib, monkeypatch, pdl):
+    """OPENSAYAL_GB300_PDL=0 turns it off for a handle and for a batch."""
+    if pdl is None:
+        monkeypatch.delenv("OPENSAYAL_GB300_PDL", raising=False)
+    else:
+        monkeypatch.setenv("OPENSAYAL_GB300_PDL", pdl)
+    cfg = tunnel(333, 187, projection_n=9, projection_block=4, projection_resident=-1)
+    with Handle(lib, cfg) as f:
+        assert f.update() == native.OS_OK
+        assert {x.pdl for x in launches(lib)} == {int(pdl != "0")}
+    batch = C.c_void_p()
+    assert lib.os_batch_create(C.byref(cfg), 1, 4, C.byref(batch)) == native.OS_OK
+    made = launches(lib)  # the member's set-up, and the step that the graph captures
+    lib.os_batch_destroy(batch)
+    step = [x.pdl for x in made if x.kind in (BATCH_DIFFUSE, BATCH_PROJECT)]
+    assert step and set(step) == {int(pdl != "0")}
+    assert any(x.pdl for x in made) == (pdl != "0")

@@ -865,8 +865,8 @@ __device__ __forceinline__ float add_pressure(float p, float vd, const Consts& c
 // check_walls keeps away from here. (Selected or predicated away instead: 257 and
 // 246 us a step at 1920 x 1080 instead of 237.)
 // The division by the count is a product with its reciprocal, which has the
-// fast-math division's bits for every float input (checked for 4 and for 3 by
-// tests/cpp).
+// fast-math division's bits for every float input and every count (compared by
+// tests/cpp/count_division.cu).
 template <int A, bool PRESSURE, bool WALL>
 __device__ __forceinline__ void row_full(float (&u)[8], float& ur, float (&vb)[8], float (&vt)[8],
                                          const ProjLane& L, const Consts& c, float d_t,

@@ -33,6 +33,7 @@ struct os_batch {
   int device = 0;
   int K = 8;
   int cluster = 4;  // CTAs per cluster of the tile kernels: the tiles' height
+  bool cluster_by_size = true;  // the members' heights and number choose it (not timed)
   int sms = 152;
   bool pdl = programmatic_launch();
   cudaStream_t stream = nullptr;
@@ -219,10 +220,66 @@ ScenarioDesc describe(const os_batch* b, const os_handle* h) {
   return d;
 }
 
+// Tiles of `cluster` CTAs at depth K, as many as fit the GPU at once.
+int size_tiles(os_batch* b, int K, int cluster) {
+  b->K = K;
+  b->cluster = cluster;
+  b->gd = batch_geom(K, false, cluster);
+  b->gp = batch_geom(K, true, cluster);
+  cudaLaunchAttribute attr;
+  b->gd_clusters = batch_clusters(batch_diffuse_kernel(), b->gd, &attr);
+  b->gp_clusters = batch_clusters(batch_project_kernel(), b->gp, &attr);
+  if (b->gd_clusters < 1 || b->gp_clusters < 1)
+    return set_err(OS_ERR_CUDA, "batch set-up: %s", cudaGetErrorString(cudaGetLastError()));
+  return OS_OK;
+}
+
+// Rows of the projection's tiles with `cluster` CTAs.
+int batch_region_rows(int cluster) { return kBatchProjectRows * kBatchProjectWarps * cluster; }
+
+bool member_live(const os_batch* b, const os_batch::Member& m) {
+  return m.finish_at < 0 || m.finish_at > b->steps_enqueued;
+}
+int tallest_member(const os_batch* b) {
+  int h = 0;
+  for (auto& kv : b->members)
+    if (member_live(b, kv.second)) h = std::max(h, kv.second.h->H);
+  return h;
+}
+
+// Members that fit tiles of two CTAs take as many tiles of those as of four, with
+// half the strips: worth it when there are more tiles than clusters of four fit
+// the GPU at once (200 tunnels of 32 to 64 cells a side, depth 8: 561 us a step
+// against 770; 16 of them the same within 3%). A taller member takes the batch
+// back to four, whose tiles have the less halo for it; fewer members do not, as a
+// change rebuilds the graph.
+int fit_cluster(os_batch* b, cudaStream_t st) {
+  if (!b->cluster_by_size) return OS_OK;
+  const bool low = tallest_member(b) <= batch_region_rows(2);
+  int want = low ? b->cluster : 4;
+  if (low && b->cluster == 4) {
+    int64_t tiles = 0;
+    for (auto& kv : b->members)
+      if (member_live(b, kv.second))
+        tiles += batch_tiles(kv.second.h->W, b->gp.TX, b->gp.halo, kTileW);
+    if (tiles > b->gp_clusters) want = 2;
+  }
+  if (want == b->cluster) return OS_OK;
+  if (b->graph) {
+    CUDA_OR_RETURN(cudaStreamSynchronize(st));
+    CUDA_OR_RETURN(cudaStreamSynchronize(b->stream));
+    cudaGraphExecDestroy(b->graph);
+    b->graph = nullptr;
+  }
+  return size_tiles(b, b->K, want);
+}
+
 // Writes the plan for the current members (those with steps still to run
 // after the ones already enqueued) and enqueues its copy on `st`; members
 // joining now get their step counts set on the device right after the copy.
 int write_plan(os_batch* b, cudaStream_t st) {
+  int rc = fit_cluster(b, st);
+  if (rc) return rc;
   struct Entry {
     int64_t id;
     ScenarioDesc d;
@@ -320,8 +377,8 @@ int write_plan(os_batch* b, cudaStream_t st) {
       CUDA_OR_RETURN(cudaStreamSynchronize(b->stream));
     }
     // Room for n up to the largest seen, so later members rarely force this.
-    int rc = build_batch_graph(b, std::max(dpasses, b->graph_dpasses),
-                               std::max(ppasses, b->graph_ppasses));
+    rc = build_batch_graph(b, std::max(dpasses, b->graph_dpasses),
+                           std::max(ppasses, b->graph_ppasses));
     if (rc) return rc;
   }
 
@@ -433,20 +490,6 @@ int batch_progress(os_batch* b) {
   return OS_OK;
 }
 
-// Tiles of `cluster` CTAs at depth K, as many as fit the GPU at once.
-int size_tiles(os_batch* b, int K, int cluster) {
-  b->K = K;
-  b->cluster = cluster;
-  b->gd = batch_geom(K, false, cluster);
-  b->gp = batch_geom(K, true, cluster);
-  cudaLaunchAttribute attr;
-  b->gd_clusters = batch_clusters(batch_diffuse_kernel(), b->gd, &attr);
-  b->gp_clusters = batch_clusters(batch_project_kernel(), b->gp, &attr);
-  if (b->gd_clusters < 1 || b->gp_clusters < 1)
-    return set_err(OS_ERR_CUDA, "batch set-up: %s", cudaGetErrorString(cudaGetLastError()));
-  return OS_OK;
-}
-
 // Blocking depth and tile height for the whole batch; the plan and graph are
 // rewritten at the next step.
 int set_geometry(os_batch* b, int K, int cluster) {
@@ -477,9 +520,11 @@ int tune_batch(os_batch* b) {
   struct Cand {
     int K, cluster;
   };
+  b->cluster_by_size = false;
+  const bool low = tallest_member(b) <= batch_region_rows(2);
   std::vector<Cand> cands;
   for (int K : {4, 6, 8, 12})
-    for (int cluster : {4, 8}) cands.push_back({K, cluster});
+    for (int cluster : {low ? 2 : 4, low ? 4 : 8}) cands.push_back({K, cluster});
   int max_n = 0;
   for (auto& kv : b->members) max_n = std::max(max_n, kv.second.h->c.n);
   cudaEvent_t a = nullptr, z = nullptr;

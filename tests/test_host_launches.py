@@ -186,3 +186,28 @@ def test_programmatic_launch_can_be_turned_off(lib, monkeypatch, pdl):
     step = [x.pdl for x in made if x.kind in (BATCH_DIFFUSE, BATCH_PROJECT)]
     assert step and set(step) == {int(pdl != "0")}
     assert any(x.pdl for x in made) == (pdl != "0")
+
+
+def test_batch_tiles_follow_the_members(lib):
+    """Many members no taller than two CTAs' rows take clusters of two, few of them
+    and taller ones clusters of four; a member that comes later changes it."""
+    low, tall = tunnel(60, 50, projection_n=9), tunnel(60, 200, projection_n=9)
+
+    def clusters():
+        return {x.cluster for x in launches(lib, BATCH_DIFFUSE, BATCH_PROJECT)}
+
+    for cfgs, want in (([low] * 16, 4), ([low] * 200, 2), ([low] * 200 + [tall], 4)):
+        batch = C.c_void_p()
+        arr = (native.OsConfig * len(cfgs))(*cfgs)
+        assert lib.os_batch_create(arr, len(cfgs), 4, C.byref(batch)) == native.OS_OK
+        assert clusters() == {want}
+        lib.os_batch_destroy(batch)
+    batch, mid = C.c_void_p(), C.c_int64()
+    assert lib.os_batch_create_dynamic(0, 4, 0, C.byref(batch)) == native.OS_OK
+    for members, cfg, want in ((16, low, {4}), (184, low, {2}), (1, tall, {4}), (1, low, set())):
+        for _ in range(members):
+            assert lib.os_batch_add(batch, C.byref(cfg), -1, C.byref(mid)) == native.OS_OK
+        launches(lib)
+        assert lib.os_batch_step(batch, 1, None) == native.OS_OK
+        assert clusters() == want
+    lib.os_batch_destroy(batch)

@@ -61,37 +61,6 @@ __device__ __forceinline__ float4 vec4_to_f32(const __nv_bfloat16* p) {
   const float2 b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&r.y));
   return make_float4(a.x, a.y, b.x, b.y);
 }
-__device__ __forceinline__ void f32_to_vec4(float* p, float4 q) {
-  *reinterpret_cast<float4*>(p) = q;
-}
-__device__ __forceinline__ void f32_to_vec4(__half* p, float4 q) {
-  __half2 a = __floats2half2_rn(q.x, q.y), b = __floats2half2_rn(q.z, q.w);
-  uint2 r;
-  r.x = *reinterpret_cast<uint32_t*>(&a);
-  r.y = *reinterpret_cast<uint32_t*>(&b);
-  *reinterpret_cast<uint2*>(p) = r;
-}
-__device__ __forceinline__ void f32_to_vec4(__nv_bfloat16* p, float4 q) {
-  __nv_bfloat162 a = __floats2bfloat162_rn(q.x, q.y), b = __floats2bfloat162_rn(q.z, q.w);
-  uint2 r;
-  r.x = *reinterpret_cast<uint32_t*>(&a);
-  r.y = *reinterpret_cast<uint32_t*>(&b);
-  *reinterpret_cast<uint2*>(p) = r;
-}
-
-template <class S>
-__device__ __forceinline__ void store_quad(S* __restrict__ f, int W, int H, int i, int j,
-                                           bool vec, float4 q) {
-  const int64_t row = (int64_t)(H - 1 - j) * W;
-  if (vec && i + 3 < W) {
-    f32_to_vec4(f + row + i, q);
-    return;
-  }
-  if (i < W) st(f + row + i, q.x);
-  if (i + 1 < W) st(f + row + i + 1, q.y);
-  if (i + 2 < W) st(f + row + i + 2, q.z);
-  if (i + 3 < W) st(f + row + i + 3, q.w);
-}
 
 // One column's run of Jacobi updates, rows e0, e0 + rs, ... (n of them), from
 // A into B. The buffers never overlap, so the loads of later rows may be
@@ -155,9 +124,9 @@ __device__ __forceinline__ void diff_sweeps(float*& A, float*& B, int tx, int ty
 }
 
 // Owned cells of the region in A back to global (FLIP as in diff_sweeps).
-template <class S, bool FLIP = false>
+template <bool FLIP = false>
 __device__ __forceinline__ void diff_store_owned(const float* A, int tx, int ty,
-                                                 S* __restrict__ u_out, const Consts& c, int halo,
+                                                 float* __restrict__ u_out, const Consts& c, int halo,
                                                  int TX, int TY) {
   const int gx0 = tx * TX - halo, gy0 = ty * TY - halo;
   const int W = c.W, H = c.H;
@@ -169,12 +138,13 @@ __device__ __forceinline__ void diff_store_owned(const float* A, int tx, int ty,
     if (j >= H || i >= W) continue;
     const float* src = A + (FLIP ? RH - 1 - y : y) * kRegionW + x;
     if (vec && x >= halo && x + 3 < halo + TX) {
-      store_quad(u_out, W, H, i, j, true, *reinterpret_cast<const float4*>(src));
+      *reinterpret_cast<float4*>(u_out + cell_index(W, H, i, j)) =
+          *reinterpret_cast<const float4*>(src);
       continue;
     }
     for (int d = 0; d < 4; d++) {
       if (x + d < halo || x + d >= halo + TX || i + d >= W) continue;
-      st(u_out + cell_index(W, H, i + d, j), src[d]);
+      u_out[cell_index(W, H, i + d, j)] = src[d];
     }
   }
 }
@@ -269,7 +239,7 @@ k_diffuse_blocked_tma(const __grid_constant__ CUtensorMap in_map, float* __restr
     return;
   }
   diff_sweeps<true>(A, B, tx, ty, c, prm, sweeps, halo, TX, TY);
-  diff_store_owned<float, true>(A, tx, ty, u_out, c, halo, TX, TY);
+  diff_store_owned<true>(A, tx, ty, u_out, c, halo, TX, TY);
 }
 
 // ---------------------------------------------------------------------------

@@ -172,9 +172,6 @@ struct os_handle {
   char* pinned = nullptr;   // one pinned block: h_params, h_pkeys, host_rerr
   float* conv = nullptr;    // FP32 staging for non-FP32 storage transfers
   double* diag = nullptr;   // diagnostics partials and result (first use)
-  // The device error word and the mapped host word that a kernel sets when a
-  // bounded wait gives up (the host word: handles outside a batch), and the
-  // resident forms' exchange state.
   // Diffusion passes staged by the tensor memory accelerator: maps of u, ub.
   CUtensorMap diff_maps[2];
   bool tma_diffusion = false;
@@ -183,12 +180,14 @@ struct os_handle {
   TileChoice tile_choice[2];  // projection, diffusion
   int resident = 0;       // projection
   int resident_diff = 0;  // diffusion
-  char* resident_block = nullptr;  // the four arrays that follow
+  char* resident_block = nullptr;  // the resident forms' state: the four arrays that follow
   size_t resident_bytes = 0;
   unsigned* rflags = nullptr;  // exchange numbers per CTA: projection, diffusion
   unsigned* dflags = nullptr;
   uint4* rpackets = nullptr;   // exchanged cells
   uint4* dpackets = nullptr;
+  // The device's error word, and the mapped host word (handles that no budgeted
+  // batch owns), that a kernel sets when a bounded wait gives up.
   int* rerr = nullptr;
   bool stepped = false;  // this handle's own steps or phases have been enqueued
   int* host_rerr = nullptr;

@@ -345,8 +345,8 @@ __device__ __forceinline__ float4 read_message(const Link<WORDS>& link, int part
 }
 
 // The messages of a strip off the grid, m .. m + count - 1: it takes part so
-// that the strips beside it wait for nothing, and its cells stay as they are
-// (zero, as a neighbour's face off the grid is).
+// that the strips beside it do not wait. What it sends is read by no cell of the
+// grid.
 template <int WORDS>
 __device__ __forceinline__ void idle_messages(Link<WORDS>& link, unsigned m, int count,
                                               const ResidentSync& sync) {
@@ -471,10 +471,10 @@ __device__ __forceinline__ void turn_out(const float (&f)[8], float (&g)[8], flo
 }
 
 // The whole patch from a field (row j of the grid at (H - 1 - j) W). `stage`: see
-// above; null where quads are aligned: the loads then carry no condition (a kernel's code is fetched cold once per launch, so what it
-// does once has to be short), and a cell off the grid reads the nearest quad
-// or row of it: cells off the grid may hold any value, no cell of the grid
-// depends on them.
+// above; null where quads are aligned: the loads then carry no condition (a
+// kernel's code is fetched cold once per launch, so what it does once has to be
+// short), and a cell off the grid reads the nearest quad or row of it: cells off
+// the grid may hold any value, no cell of the grid depends on them.
 template <int R, class IO>
 __device__ __forceinline__ void patch_in(const IO& io, float (&f)[R][8], const void* field,
                                          const Patch& P, int W, int H, float* stage) {
@@ -978,8 +978,8 @@ __device__ __forceinline__ float4 reciprocal_counts(uint32_t w) {
 
 // The strip's flags: what row_full may take, and for a strip that it may not the
 // flag words and reciprocal counts into shared memory (each lane's own).
-// A lane wholly off the grid puts no condition: its cells are zeros whose
-// faces no cell of the grid reads.
+// A lane wholly off the grid puts no condition: whatever its cells hold, no cell
+// of the grid reads their faces.
 template <int R>
 __device__ __forceinline__ void flags_in(const uint8_t* __restrict__ flags, const Patch& P,
                                          const ProjSmem& sm, int W, int H, bool vec,

@@ -255,8 +255,8 @@ inline int phase_tile(os_handle* h, bool projection, int K, bool resident, RegTi
 
 // The projection phase: one launch for all its passes (resident), or one per
 // pass of block_k sweeps. `cur_u` / `cur_v` say which copy holds the live
-// field (0: u, v; 1: ub, vb); each launch moves it to the other. `extrapolate`: the
-// last pass applies the extrapolation that follows in a step. Returns the
+// field (0: u, v; 1: ub, vb); each launch moves it to the other. `extrapolate`:
+// the last pass applies the extrapolation that follows in a step. Returns the
 // launches, or -1.
 inline int enqueue_tiled_projection(os_handle* h, cudaStream_t st, int* cur_u, int* cur_v,
                                     bool zero_first, bool extrapolate) {
@@ -296,8 +296,8 @@ inline int enqueue_tiled_projection(os_handle* h, cudaStream_t st, int* cur_u, i
       a.vi = V[cv], a.vo = V[1 - cv];
       a.zero_pressure = zero_first && p == 0;
       a.extrapolate = extrapolate && p == passes - 1;
-      if (launch_tiles(project_kernel_of(a.g.R, pressure, quads_aligned(h->W, a.g.halo)), a, a.g, false, h->pdl, st) !=
-          cudaSuccess)
+      if (launch_tiles(project_kernel_of(a.g.R, pressure, quads_aligned(h->W, a.g.halo)), a, a.g,
+                       false, h->pdl, st) != cudaSuccess)
         return -1;
     }
   }
@@ -334,7 +334,8 @@ inline int enqueue_tiled_diffusion(os_handle* h, cudaStream_t st, int* cur_u) {
       a.n = std::min(K, n - p * K);
       const int cu = (*cur_u + p) & 1;
       a.ui = U[cu], a.uo = U[1 - cu];
-      if (launch_tiles(diffuse_kernel_of(a.g.R, quads_aligned(h->W, a.g.halo)), a, a.g, false, h->pdl, st) != cudaSuccess)
+      if (launch_tiles(diffuse_kernel_of(a.g.R, quads_aligned(h->W, a.g.halo)), a, a.g, false,
+                       h->pdl, st) != cudaSuccess)
         return -1;
     }
   }

@@ -40,3 +40,23 @@ def test_resident_equals_passes(gpu, w, h, k, n, storage):
     assert_same(a, b, FIELDS + (("pressure",) if base.enable_pressure else ()))
     a.close()
     b.close()
+
+
+@pytest.mark.parametrize("w,h", [(257, 63), (252, 511), (480, 129), (800, 400)])
+@pytest.mark.parametrize("k,n", [(4, 33), (8, 17)])
+@pytest.mark.parametrize("resident", [-1, 3])
+def test_wild_states_equal_plain(gpu, w, h, k, n, resident):
+    """Cells that are not finite: infinities stay apart from the largest numbers."""
+    base = tunnel(w, h, projection_n=n, enable_pressure=w % 2)
+    state = state_of(base, w + h + k, wild=True)
+    plain, tiles = base.copy(), base.copy()
+    plain.projection_block = -1
+    tiles.projection_block, tiles.projection_resident = k, resident
+    a, b = load_lib(plain, state), load_lib(tiles, state)
+    assert b.fields().projection_resident == max(resident, 0)
+    for phase in (native.PHASE_DIFFUSION, native.PHASE_PROJECTION):
+        a.run_phase(phase, None, 0.05)
+        b.run_phase(phase, None, 0.05)
+    assert_same(a, b, FIELDS + (("pressure",) if base.enable_pressure else ()))
+    a.close()
+    b.close()

@@ -6,6 +6,7 @@ import numpy as np
 import pytest
 
 from opensayal_gb300 import native
+from opensayal_gb300.batch import Batch
 from tests.parity_cases import FIELDS, load_lib
 from tests.test_tiles_gpu import state_of, tunnel
 
@@ -60,3 +61,30 @@ def test_wild_states_equal_plain(gpu, w, h, k, n, resident):
     assert_same(a, b, FIELDS + (("pressure",) if base.enable_pressure else ()))
     a.close()
     b.close()
+
+
+@pytest.mark.parametrize("k,n", [(4, 7), (8, 16), (8, 50)])
+def test_resident_beside_other_work_equals_alone(gpu, k, n):
+    """Other streams hold SMs meanwhile, so that a resident launch's tiles do not
+    all start together: a tunnel pass by pass and a batch."""
+    res = tunnel(800, 400, projection_n=n, projection_block=k, projection_resident=3)
+    other = tunnel(1003, 771, projection_n=20, projection_block=8, projection_resident=-1)
+    low = [tunnel(96 + 16 * i, 64 + 8 * i, projection_n=30) for i in range(6)]
+    state, other_state = state_of(res, 1), state_of(other, 2)
+    steps = 40
+    with load_lib(res, state) as a, load_lib(res, state) as b, load_lib(other, other_state) as o, \
+            Batch(low, block_k=8) as batch:
+        assert a.fields().projection_resident == 3
+        a.update_async(None, 0.02, steps)
+        a.synchronize()
+        for _ in range(steps // 8):
+            o.update_async(None, 0.02, 8)
+            batch.step(8)
+            b.update_async(None, 0.02, 8)
+        for x in (b, o, batch):
+            x.synchronize()
+        assert_same(a, b, FIELDS)
+        with load_lib(other, other_state) as alone:
+            alone.update_async(None, 0.02, steps)
+            alone.synchronize()
+            assert_same(o, alone, FIELDS)

@@ -1548,12 +1548,13 @@ float time_steps(os_handle* t, float dt, int warm, int reps) {
   return ms;
 }
 
-// Candidates: depths {4, 6, 8, 12, 16} pass by pass (2 for fewer sweeps than 4) and, unless
-// projection_resident is -1, the resident forms (projection and diffusion,
+// Candidates: depths {4, 6, 8, 12, 16} pass by pass (2 for fewer sweeps than 4) and,
+// unless projection_resident is -1, the resident forms (projection and diffusion,
 // alone or together) where the grid fits them, at one depth: a resident form
 // chooses its own sweeps between exchanges, and the depth only says how often
-// 16-bit fields are rounded. A positive projection_resident fixes the forms
-// and leaves only the depth to choose.
+// 16-bit fields are rounded: with those it is deeper, so that they are rounded no
+// more often than by the passes that would run instead. A positive
+// projection_resident fixes the forms and leaves only the depth to choose.
 TuneChoice autotune_projection(const os_config& base) {
   constexpr TuneChoice kDefault{4, 0, 0};
   const char* env = std::getenv("OPENSAYAL_GB300_AUTOTUNE");
@@ -1575,11 +1576,13 @@ TuneChoice autotune_projection(const os_config& base) {
       cands.push_back({K, 0, 0});
   }
   if (base.projection_resident == 0) {
-    const int K = base.projection_n >= 8 ? 8 : base.projection_n >= 4 ? 4 : 2;
+    const int n = base.projection_n;
+    const bool rounded = base.storage != OS_STORAGE_F32;
+    const int K = rounded && n >= 12 ? (n >= 16 ? 16 : 12) : n >= 8 ? 8 : n >= 4 ? 4 : 2;
     cands.push_back({K, 1, 0});
     if (K % 4 == 0 && base.viscosity != 0.0f) {
       cands.push_back({K, 2, 0});
-      cands.push_back({K, 3, 0});
+      cands.push_back({rounded && n >= 24 ? 24 : K, 3, 0});
     }
   }
   const float dt = base.d_t > 0.0f ? base.d_t : 0.05f;

@@ -380,8 +380,9 @@ int os_render_traces(os_handle* h, const os_visual_config* v, float dt, int32_t*
  * messages of a neighbouring strip that sends none. Every such wait is bounded
  * (about a second); when one gives up it records the failure, the waits after
  * it end with it, and the host call that synchronises reports OS_ERR_TIMEOUT.
- * *status receives what that path reports here (OS_ERR_TIMEOUT when both bounds
- * work). No reference counterpart.
+ * A third launch expects other thread-block clusters than it has: it must report
+ * in the same way instead of using them. *status receives what that path reports
+ * here (OS_ERR_TIMEOUT when all three work). No reference counterpart.
  */
 int os_selftest_bounded_wait(int32_t device, int32_t* status);
 

@@ -1310,14 +1310,15 @@ int os_selftest_bounded_wait(int32_t device, int32_t* status) {
     *host_err = 0;
     e = cudaHostGetDevicePointer((void**)&d_host_err, host_err, 0);
   }
-  // Packets, then messages (400, as many as 200 sweeps take): each must report.
+  // Packets, messages (400, as many as 200 sweeps take), and a launch in clusters of
+  // two that expects four: each must report.
   const ResidentSync sync{nullptr, packets, dev_err, d_host_err};
   bool reported = true;
-  for (int messages = 0; messages < 2 && e == cudaSuccess; messages++) {
+  for (int test = 0; test < 3 && e == cudaSuccess; test++) {
     *host_err = 0;
     if ((e = cudaMemset(dev_err, 0, sizeof(int))) != cudaSuccess) break;
-    if (messages) {
-      e = launch_message_selftest(sync, 400);
+    if (test) {
+      e = launch_message_selftest(sync, test == 1 ? 2 : 4, 400);
     } else {
       k_wait_selftest<<<1, 32>>>(sync);
       e = cudaGetLastError();

@@ -46,6 +46,7 @@ k_batch_project_tiles(const PlanHeader* __restrict__ plan, const int* __restrict
   const TileRef* tiles = plan_array<TileRef>(plan, plan->off_proj_tiles);
   const ScenarioDesc* descs = plan_array<ScenarioDesc>(plan, plan->off_desc);
   cluster_wait();
+  if (!clusters_of(g.cluster, sync)) return;
   unsigned message = 0;
 #pragma unroll 1
   for (int it = blockIdx.x / g.cluster; it < items && !link.lost;
@@ -103,6 +104,7 @@ k_batch_diffuse_tiles(const PlanHeader* __restrict__ plan, const int* __restrict
   const TileRef* tiles = plan_array<TileRef>(plan, plan->off_diff_tiles);
   const ScenarioDesc* descs = plan_array<ScenarioDesc>(plan, plan->off_desc);
   cluster_wait();
+  if (!clusters_of(g.cluster, sync)) return;
   unsigned message = 0;
 #pragma unroll 1
   for (int it = blockIdx.x / g.cluster; it < items && !link.lost;

@@ -365,19 +365,21 @@ __global__ void k_wait_selftest(ResidentSync sync) {
 
 // The strip of the first of two CTAs takes part in `count` messages, and the
 // second's sends none: the first wait must give up, and the others end with it.
-__global__ void k_message_selftest(ResidentSync sync, int count) {
+// With a `cluster` that is not the launch's, it must report that and end at once.
+__global__ void k_message_selftest(ResidentSync sync, int cluster, int count) {
   extern __shared__ __align__(16) char tile_smem[];
   RegTile g{};
   g.R = 2, g.warps = 1, g.cluster = 2, g.RH = 4;
   Link<4> link = open_link<4>(tile_smem, patch_at(TilePlace{0, 0, 1, 1}, g, g.R, 1, 1), g);
   cluster_arrive();
   cluster_wait();
+  if (!clusters_of(cluster, sync)) return;
   if (blockIdx.x == 0) idle_messages(link, 0, count, sync);
   cluster_arrive();
   cluster_wait();
 }
 
-inline cudaError_t launch_message_selftest(const ResidentSync& sync, int count) {
+inline cudaError_t launch_message_selftest(const ResidentSync& sync, int cluster, int count) {
   cudaError_t e = allow_most(k_message_selftest);
   if (e != cudaSuccess) return e;
   cudaLaunchAttribute attr;
@@ -390,7 +392,7 @@ inline cudaError_t launch_message_selftest(const ResidentSync& sync, int count) 
   cfg.dynamicSmemBytes = inbox_bytes(4);
   cfg.attrs = &attr;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, k_message_selftest, sync, count);
+  return cudaLaunchKernelEx(&cfg, k_message_selftest, sync, cluster, count);
 }
 
 }  // namespace osg

@@ -1,10 +1,12 @@
 """What the host decides for the tile phases, read from the launches that a step
 makes: no GPU needed."""
 import ctypes as C
+import re
 
 import pytest
 
 from opensayal_gb300 import native
+from tests.conftest import ROOT
 from tests.host_only import (BATCH_DIFFUSE, BATCH_PROJECT, DIFFUSE, PROJECT, Handle, launches,
                              load, segments, tunnel)
 
@@ -211,3 +213,17 @@ def test_batch_tiles_follow_the_members(lib):
         assert lib.os_batch_step(batch, 1, None) == native.OS_OK
         assert clusters() == want
     lib.os_batch_destroy(batch)
+
+
+def test_tile_kernels_check_their_clusters():
+    """Each kernel that sends messages between CTAs asks whether the launch has its
+    clusters before it sends the first."""
+    for name, kernels in (("os_tile.cuh", 2), ("os_tile_batch.cu", 2), ("os_tile_host.cuh", 1)):
+        text = (ROOT / "opensayal_gb300" / "csrc" / name).read_text()
+        opened = [m.start() for m in re.finditer(r"Link<\d> link = open_link<", text)]
+        assert len(opened) == kernels, name
+        for at in opened:
+            asked = re.compile(r"cluster_wait\(\);[^\n]*\n  if \(!clusters_of\([^)]*\)\) return;")
+            found = asked.search(text, at)
+            sent = re.compile(r"(tile_sweeps|jacobi_sweeps|idle_messages)(<[^>]*>)?\(").search(text, at)
+            assert found and sent and found.start() < sent.start(), name

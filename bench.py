@@ -369,14 +369,15 @@ def run_gb300(args, world, rank, local) -> dict | None:
     traffic, traffic_source, on_chip = None, "not captured for this configuration", None
     # launches of the projection kernel in one phase: one resident launch, or
     # one blocked launch per pass
-    k_proj = (1 if f.fields().projection_resident else
+    resident = bool(f.fields().projection_resident & 1)  # bit 1 is the diffusion's
+    k_proj = (1 if resident else
               -(-cfg.projection_n // max(1, f.fields().projection_block)))
     tfile = ROOT / "profiles" / "roofline_traffic.json"
     if tfile.exists():
         key = f"{args.workload}:block{f.fields().projection_block}" + (
-            ":resident" if f.fields().projection_resident else "")
+            ":resident" if resident else "")
         entry = json.loads(tfile.read_text()).get(key)
-        if entry:
+        if entry and entry["kernel"] == "k_project_tiles":  # not of a kernel that is gone
             traffic = entry["bytes_per_launch"] * k_proj
             traffic_source = entry["source"]
             if "smsp__issue_active" in entry:
@@ -405,14 +406,15 @@ def run_gb300(args, world, rank, local) -> dict | None:
                      "kernels_per_phase_timed": k_proj,
                      "launches_per_phase_with_copy_back": proj_kernels // 3,
                      "peak_source": pk["source"]},
-        # The projection's sweeps run in shared memory and its halo exchanges
-        # go through L2; DRAM sees the fields about once per phase. The level
-        # that binds is on-chip, so the same algorithmic rate is also given
-        # against a live L2-resident copy.
+        # The projection's sweeps run in registers and its halos (or its passes)
+        # go through L2; DRAM sees the fields about once per pass at most. What
+        # binds is on the SM, so the algorithmic rate says how many bytes a sweep by
+        # sweep schedule would have to move, not what HBM or L2 carry; it is also
+        # given against a live L2-resident copy.
         "roofline_l2": {"bound": "l2", "achieved": achieved, "peak": l2["gbs"], "unit": "GB/s",
                         "frac": achieved / l2["gbs"], "peak_source": "measured live: " + l2["how"],
                         "peak_buffer_mib": l2.get("buffer_mib"),
-                        # the binding pipes: instruction issue and shared memory
+                        # what the SM does meanwhile: instruction issue, L1 and shared memory
                         "on_chip": on_chip},
         "step_roofline": {"bytes_per_cell_step": step_bytes,
                           "achieved": step_bytes * value / world / 1e9, "unit": "GB/s",
@@ -952,7 +954,7 @@ def main():
                          "autotuned, the autotuner's)")
     ap.add_argument("--no-cpu-baseline", action="store_true")
     ap.add_argument("--resident", type=int, default=None, choices=[-1, 0, 1, 2, 3],
-                    help="phases as resident cooperative launches: mask 1 projection, "
+                    help="phases as one resident launch each: mask 1 projection, "
                          "2 diffusion, 3 both; -1 never; 0 autotuner decides")
     ap.add_argument("--mixed", action="store_true",
                     help="batched: BF16 storage for half of the scenarios")

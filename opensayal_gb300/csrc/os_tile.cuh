@@ -877,7 +877,7 @@ __device__ __forceinline__ float add_pressure(float p, float vd, const Consts& c
 // first or last column is not updated; the cell beside a solid one has three
 // neighbours). A = first active column. A face that stays takes +0 off or -0
 // on, without a branch, which leaves as it is every value but those that
-// check_walls keeps away from here. (Selected or predicated away instead: 257 and
+// zeros_change keeps away from here. (Selected or predicated away instead: 257 and
 // 246 us a step at 1920 x 1080 instead of 237.)
 // The division by the count is a product with its reciprocal, which has the
 // fast-math division's bits for every float input and every count (compared by
@@ -1063,27 +1063,28 @@ __device__ __forceinline__ void flags_in(const uint8_t* __restrict__ flags, cons
 
 // Faces that stay hold what they hold, but row_full adds zeros to those beside the
 // grid's left and right edges, which flushes a value below the smallest normal
-// number and makes one NaN of all. A strip with such a value there is taken by its
-// flags instead.
-__device__ __forceinline__ bool zero_changes(float x) {
-  const uint32_t b = __float_as_uint(x) & 0x7fffffffu;
-  return b - 1u < 0x7fffffu || b > 0x7f800000u;
-}
+// number and makes one NaN of all. Whether it would change one of this strip,
+// which then goes by its flags. (A kernel's code is fetched cold once per launch:
+// an addition and a logic operation a face, where a test of its exponent took 0.5
+// us of every launch at 256 x 128.)
 template <int R>
-__device__ __forceinline__ void check_walls(const float (&u)[R][8], const float (&v)[R][8],
-                                            const float (&vt)[8],
-                                            const uint8_t* __restrict__ flags, const Patch& P,
-                                            const ProjSmem& sm, int W, int H, ProjLane& L) {
-  if (!L.full || !L.wall) return;  // the same for the warp
-  bool left = zero_changes(vt[0]), right = zero_changes(vt[7]);
+__device__ __forceinline__ bool zeros_change(const float (&u)[R][8], const float (&v)[R][8],
+                                             const float (&vt)[8], const ProjLane& L) {
+  if (!L.full || !L.wall) return false;  // the same for the warp
+  float zero = -0.0f;
+  asm volatile("" : "+f"(zero));  // the compiler takes x + -0 for x
+  auto changed = [&](float x) { return __float_as_uint(x + zero) ^ __float_as_uint(x); };
+  uint32_t left = changed(vt[0]), right = changed(vt[7]);
 #pragma unroll
   for (int r = 0; r < R; r++) {
-    left = left || zero_changes(u[r][0]) || zero_changes(u[r][1]) || zero_changes(v[r][0]);
-    right = right || zero_changes(u[r][7]) || zero_changes(v[r][7]);
+    left |= changed(u[r][0]) | changed(u[r][1]) | changed(v[r][0]);
+    right |= changed(u[r][7]) | changed(v[r][7]);
   }
-  if (!__any_sync(kAllLanes, (L.wall_l && left) || (L.wall_r && right))) return;
-  L.full = false;
-  // The words that flags_in left out.
+  return __any_sync(kAllLanes, (L.wall_l && left) || (L.wall_r && right));
+}
+// The flag words and counts of a strip that flags_in took for full.
+static __device__ __noinline__ void flags_late(const uint8_t* flags, const Patch P,
+                                               const ProjSmem sm, int W, int H, int R) {
   const int gx = P.gx0 + P.x0;
 #pragma unroll 1
   for (int r = 0; r < R; r++) {
@@ -1416,7 +1417,10 @@ k_project_tiles(const __grid_constant__ ProjectArgs a) {
     patch_in<R>(io, v, a.vi, P, W, H, stage);
     if (P.up) row_in(io, vt, a.vi, P, P.y0 + R, W, H, stage);
   });
-  check_walls<R>(u, v, vt, a.flags, patch_of(a.g, R, W, H), sm, W, H, L);
+  if (zeros_change<R>(u, v, vt, L)) {
+    L.full = false;
+    flags_late(a.flags, patch_of(a.g, R, W, H), sm, W, H, R);
+  }
   const unsigned epoch = a.n > a.D ? ld_acquire_gpu(a.sync.epochs + blockIdx.x) : 0u;
   unsigned number = epoch;
   if (a.n > a.D) exchange_plan(sm.exchange, a.g, R, 2, W, H);

@@ -82,7 +82,10 @@ k_batch_project_tiles(const PlanHeader* __restrict__ plan, const int* __restrict
           patch_in<R>(io, v, vi, P, W, H, stage);
           if (P.up) row_in(io, vt, vi, P, P.y0 + R, W, H, stage);
         });
-      check_walls<R>(u, v, vt, d.flags, P, sm, W, H, L);
+      if (zeros_change<R>(u, v, vt, L)) {
+        L.full = false;
+        flags_late(d.flags, P, sm, W, H, R);
+      }
     }
     tile_sweeps<false, R>(u, v, vt, L, sm, link, sync, cell0, down, c, 0.0f, sweeps, message);
     message += project_messages(sweeps);
